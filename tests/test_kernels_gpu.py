@@ -180,6 +180,29 @@ def test_gemm_plain_ladder(shape, combo):
     close(run(a, w), a.double() @ w.double().t(), (1e-7 * math.sqrt(K) if tc == torch.float32 else 5e-3))
 
 
+@pytest.mark.parametrize("M", [1, 3, 4, 5, 8, 9, 16, 17, 64, 65, 130])
+@pytest.mark.parametrize("N,K", [(5, 4), (31, 128), (32, 132), (33, 100), (300, 1028), (4800, 256)])
+def test_gemm_plain_same_bits_in_every_kernel(M, N, K):
+    """32-bit rows of whole 16-byte vectors go to kernels of their own (up to 16 rows, and tiles); every output is the
+    same chain of multiply-adds over k there, so the bits are those of the general kernel, which takes a weight whose
+    rows are not 16-byte aligned.  NaN beside the operands must not reach a result."""
+    from odin_infer_b200.csrc import ops
+    torch.manual_seed(M * 1000 + N)
+    a = torch.full((M + 1, K + 8), float("nan"), device=DEV)
+    a[:M, :K] = torch.randn(M, K, device=DEV)
+    w = torch.full((N + 1, K + 4), float("nan"), device=DEV)
+    w[:N, :K] = torch.randn(N, K, device=DEV)
+    odd = torch.full((N + 1, K + 1), float("nan"), device=DEV)
+    odd[:N, :K] = w[:N, :K]
+    fast = torch.full((M + 1, N), 7.0, device=DEV)
+    general = torch.empty(M, N, device=DEV)
+    torch.cuda.synchronize()
+    ops.gemm_plain(a[:M, :K], w[:N, :K], fast[:M])
+    ops.gemm_plain(a[:M, :K], odd[:N, :K], general)
+    assert torch.equal(fast[:M], general)
+    assert (fast[M] == 7.0).all()
+
+
 def paged_cache(n_seqs, lengths, n_kv, hd, dtype, shuffle=True):
     """A cache whose pages are handed out in a scrambled order."""
     PAGE = 64

@@ -34,7 +34,7 @@ class Engine_Opts:
     that live sequences hold together, each rounded up to a page of 64; it sizes the
     cache (0: max_batch sequences of max_ctx).  dtype: "bfloat16" (the kernels and
     precisions of serving) or "float32" (everything in true 32-bit).  cuda_graphs: replay
-    captured graphs for one-token-per-sequence steps (bfloat16 only).  run_ahead: generation
+    captured graphs for one-token-per-sequence steps and short prompts.  run_ahead: generation
     launches a decode step before the host has read the tokens it continues from."""
     max_ctx: int = DEFAULT_MAX_CONTEXT
     max_tokens: int = 0
@@ -96,13 +96,18 @@ class Engine:
         nstate = self.cache.state_bytes_per_slot
         self.cache.state = torch.zeros(self.cache.max_slots, nstate, dtype=torch.uint8, device=self.rt.device)
         self.cache.zero_state = (lambda slot: self.cache.state[slot].zero_()) if nstate else None
-        # decode steps replay CUDA graphs in the serving precision; the 32-bit path stays eager
+        # decode steps and short prompts replay CUDA graphs: `graphs` those of the serving precision, `graphs_32bit` the
+        # 32-bit path's (fewer prompts, logits of the caller's own)
         self.last_step_h2d_bytes = 0
-        self.graphs = None
-        if opts.cuda_graphs and self.rt.dtype == torch.bfloat16:
+        self.graphs = self.graphs_32bit = None
+        if opts.cuda_graphs:
             if self.model.graph_safe:
-                self.graphs = DecodeGraphs(self.rt, self.model, self.cache)
-            elif opts.verbose:
+                g = DecodeGraphs(self.rt, self.model, self.cache)
+                if self.rt.dtype == torch.bfloat16:
+                    self.graphs = g
+                else:
+                    self.graphs_32bit = g
+            elif opts.verbose and self.rt.dtype == torch.bfloat16:
                 print("odin_infer_b200: steps run eagerly, not as CUDA graphs: these parts do not declare graph_safe: "
                       + ", ".join(self.model.parts_not_graph_safe()), file=sys.stderr, flush=True)
         self.notes = self.model.notes(self.rt)
@@ -182,9 +187,10 @@ class Engine:
                 starts.append(self.cache.extend(e.slot, len(e.tokens)))
                 grown.append(e)
             logits = NotImplemented
-            if self.graphs is not None and self.graphs.takes(entries):
-                logits = self.graphs.run(entries, starts, device_tokens)
-                self.last_step_h2d_bytes = self.graphs.last_h2d_bytes
+            graphs = self.graphs or self.graphs_32bit
+            if graphs is not None and graphs.takes(entries):
+                logits = graphs.run(entries, starts, device_tokens)
+                self.last_step_h2d_bytes = graphs.last_h2d_bytes
             if logits is NotImplemented:
                 batch = StepBatch(self.cache, entries, starts, self.rt.device)
                 if device_tokens is not None:
@@ -230,8 +236,9 @@ class Engine:
         for g in self.cache.groups.values():
             g.k = g.v = None
         self.cache.state = None
-        if self.graphs is not None:
-            self.graphs.clear()
+        for g in (self.graphs, self.graphs_32bit):
+            if g is not None:
+                g.clear()
         self.model = None
         torch.cuda.empty_cache()
 

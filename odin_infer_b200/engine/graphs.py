@@ -24,8 +24,13 @@ BUCKETS = (1, 2, 4, 8, 12, 16, 24, 32, 48, 64, 96, 128, 192, 256)
 # time each: 8 ms for what the device does in 3): steps of a few sequences with up to 1,024 tokens in
 # all are captured as well, per bucket of their token count and of their number of sequences, padded
 # with rows of sequence -1 and with empty sequences.
-PROMPT_BUCKETS = (32, 64, 128, 192, 256, 384, 512, 768, 1024)
+PROMPT_BUCKETS = (16, 32, 64, 128, 192, 256, 384, 512, 768, 1024)
 PROMPT_SEQ_BUCKETS = (1, 2, 4, 8, 16)
+
+# In 32-bit only up to 256 tokens, and at most one wanted place per sequence: beyond that a step of a model that is not
+# tiny keeps the device busy for longer than its launches take (the 1.7B size: 64 rows 9 ms beside 5.8 ms of launches),
+# while the padding rows cost their share of it; up to there the buckets are multiples of the products' 64-row tiles.
+PROMPT_ROWS_32BIT = 256
 
 
 def bucket_for(n: int) -> int | None:
@@ -45,6 +50,9 @@ class DecodeGraphs:
         """Is this a step that `run` may replay a graph for?"""
         if all(len(e.tokens) == 1 for e in entries):
             return True
+        if self.rt.dtype == torch.float32 and (sum(len(e.tokens) for e in entries) > PROMPT_ROWS_32BIT
+                                               or sum(len(e.want) for e in entries) > len(entries)):
+            return False
         return (len(entries) <= PROMPT_SEQ_BUCKETS[-1] and sum(len(e.tokens) for e in entries) <= PROMPT_BUCKETS[-1]
                 and any(e.want for e in entries))
 
@@ -63,7 +71,12 @@ class DecodeGraphs:
         graph.replay()
         ops.add_launches(n_kernels)
         self.last_h2d_bytes = batch.h2d_bytes
-        return logits
+        return self._handed_out(logits)
+
+    def _handed_out(self, logits: torch.Tensor) -> torch.Tensor:
+        """What a replay's caller gets: the graph's own buffer, which the next replay writes again; in 32-bit, whose logits
+        are compared and kept, a copy."""
+        return logits.clone() if self.rt.dtype == torch.float32 else logits
 
     def _first_run(self, key, batch: StepBatch, device_tokens=None) -> torch.Tensor | None:
         """The step itself, eagerly (first-use set-up of the kernels - function attributes, tensor
@@ -112,7 +125,7 @@ class DecodeGraphs:
         if not rows:
             return None
         if rows == list(range(len(rows))):
-            return logits[:len(rows)]
+            return logits[:len(rows)] if hit is None else self._handed_out(logits[:len(rows)])
         return logits[torch.tensor(rows, device=logits.device)]
 
     def clear(self) -> None:

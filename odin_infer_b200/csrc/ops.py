@@ -1183,9 +1183,11 @@ def head_prep(qkv: torch.Tensor, n_q: int, n_kv: int, head_dim: int, q_norm: tor
 def attention_plain(q: torch.Tensor, out: torch.Tensor, n_q: int, n_kv: int, head_dim: int,
                     k_cache: torch.Tensor, v_cache: torch.Tensor, tok_pos: torch.Tensor, tok_seq: torch.Tensor,
                     block_table: torch.Tensor, window: int = 0, chunk: int = 0, scale: float = 0.0,
-                    softcap: float = 0.0, v_head_dim: int | None = None, sink: torch.Tensor | None = None) -> None:
+                    softcap: float = 0.0, v_head_dim: int | None = None, sink: torch.Tensor | None = None,
+                    single: bool = False) -> None:
     """Causal attention of each token over its sequence's cache; q may be a strided view.
     sink: float32 [n_q]; exp(sink[h]) joins the softmax's denominator of head h (no key, no value).
+    single: every sequence brings one token (the kernel for decoding in 32-bit; the same bits either way).
 
     window > 0: only the last `window` keys; chunk > 0: only the keys of the query's own chunk of
     `chunk` positions; scale > 0 replaces 1 / sqrt(head_dim); softcap > 0: scores pass through
@@ -1200,7 +1202,7 @@ def attention_plain(q: torch.Tensor, out: torch.Tensor, n_q: int, n_kv: int, hea
         _ptr(q), c_longlong(q.stride(0)), _ptr(out), c_longlong(out.stride(0)), c_int(dtype_code(q.dtype)),
         c_int(T), c_int(n_q), c_int(n_kv), c_int(head_dim), c_int(vd), _ptr(k_cache), _ptr(v_cache), c_int(PAGE),
         _ptr(tok_pos), _ptr(tok_seq), _ptr(block_table), c_int(block_table.stride(0)), c_int(window), c_int(chunk),
-        c_float(scale), c_float(softcap), _ptr(_sink(sink, n_q)), _stream()), "attention_plain")
+        c_float(scale), c_float(softcap), _ptr(_sink(sink, n_q)), c_int(1 if single else 0), _stream()), "attention_plain")
 
 
 def _sink(sink: torch.Tensor | None, n_q: int) -> torch.Tensor | None:

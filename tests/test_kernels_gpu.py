@@ -289,6 +289,46 @@ def test_head_prep_and_attention_plain(geom, dtype):
         close(got, ref, 3e-6 if dtype == torch.float32 else 1e-2)
 
 
+@pytest.mark.parametrize("geom", [(2, 1, 16), (5, 1, 48), (6, 2, 64), (8, 1, 64), (4, 2, 128), (3, 3, 128), (8, 1, 128)])
+@pytest.mark.parametrize("options", [{}, {"softcap": 5.0, "scale": 0.3, "sink": True}, {"window": 40}, {"chunk": 48}])
+def test_attention_32bit_same_bits_in_every_kernel(geom, options):
+    """32-bit attention has kernels of its own for one token per sequence and for prompts; a row's bits are those of the
+    general kernel, which takes queries whose rows are not 16-byte aligned.  Sequences of 1 to 300 tokens side by side
+    (a tile holds the end of one and the start of the next), pieces that start late, padding rows, a page that is gone,
+    NaN in unwritten slots, and an infinite value that only later rows may see."""
+    from odin_infer_b200.csrc import ops
+    n_q, n_kv, hd = geom
+    torch.manual_seed(n_q * 100 + hd)
+    lengths = [1, 33, 64, 65, 300, 130]
+    k, v, bt = paged_cache(len(lengths), lengths, n_kv, hd, torch.float32)
+    for s, n in enumerate(lengths):
+        for p in range(n):
+            k[bt[s, p // 64], :, p % 64] = torch.randn(n_kv, hd, device=DEV)
+            v[bt[s, p // 64], :, p % 64] = torch.randn(n_kv, hd, device=DEV)
+    v[bt[4, 280 // 64], :, 280 % 64] = float("inf")
+    bt[5, 0] = -1   # released: nobody sees its keys
+    opt = dict(options)
+    if opt.pop("sink", False):
+        opt["sink"] = torch.randn(n_q, device=DEV)
+    starts = [0, 0, 10, 0, 77, 66]
+    prompt = [(s, p) for s, n in enumerate(lengths) for p in range(starts[s], n)]
+    single = [(s, n - 1) for s, n in enumerate(lengths)]
+    for rows, one in ((prompt, False), (single, True)):
+        rows = rows[:3] + [(-1, 0)] + rows[3:] + [(-1, 0)]
+        tok_seq = torch.tensor([s for s, _ in rows], dtype=torch.int32, device=DEV)
+        tok_pos = torch.tensor([p for _, p in rows], dtype=torch.int32, device=DEV)
+        q = torch.randn(len(rows), n_q * hd + 1, device=DEV)
+        aligned = q[:, :n_q * hd].contiguous()
+        general = torch.full((len(rows), n_q * hd), 7.0, device=DEV)
+        fast = general.clone()
+        args = (n_q, n_kv, hd, k, v, tok_pos, tok_seq, bt)
+        ops.attention_plain(q[:, :n_q * hd], general, *args, **opt)
+        ops.attention_plain(aligned, fast, *args, single=one, **opt)
+        assert torch.equal(fast.isnan(), general.isnan())
+        assert torch.equal(fast.nan_to_num(nan=1.0), general.nan_to_num(nan=1.0))
+        assert general[:3].isfinite().all()
+
+
 @pytest.mark.parametrize("geom", [(8, 2, 128), (6, 3, 64)])
 @pytest.mark.parametrize("parts", [0, 2])
 def test_head_prep_many_tokens_equals_few_at_a_time(geom, parts):

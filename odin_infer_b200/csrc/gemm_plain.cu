@@ -200,7 +200,8 @@ __global__ void __launch_bounds__(ROWS_THREADS) gemm_f32_rows_kernel(const float
 // What bounds it: the multiply-adds (M N K of them, 128 per cycle and SM: 71 TFLOP/s measured) and beside them the
 // shared loads and the register banks.  922 x 12288 x 2048: 1,061 us, 43.7 TFLOP/s (1,915 us before).  Tiles of 128 x 128
 // with 8 x 8 outputs a thread run at 41.3 there and at 45.5 on 922 x 24576 x 4096 (these: 44.2), but leave the SMs idle
-// on anything smaller: 500 x 2048 x 2048 takes them 191 us, these 113.
+// on anything smaller: 500 x 2048 x 2048 takes them 191 us, these 113.  Two multiply-adds an instruction (fma.rn.f32x2) on
+// tiles of 64 x 128 with both operands transposed on their way to shared memory, 4 bytes a copy: 1,117 us at best.
 constexpr int TILE_BK = 32;
 
 constexpr int RM = 4, RN = 4, TX = 8, TILE_STAGES = 4;

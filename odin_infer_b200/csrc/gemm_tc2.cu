@@ -5,11 +5,11 @@
 // cluster share one 256 x 256 output tile: each brings its own 128 token rows (A) and its own
 // half of the 256 weight rows (B), 32 KB per block and CTA, and the MMA of the pair reads both
 // halves of B from the two CTAs' shared memories.  A third less traffic per product, and a
-// ring of six stages instead of four.
+// ring of five or six stages instead of four.
 //
 // Roles in each CTA (192 threads): warp 0 issues its TMA loads; warp 1 allocates tensor
 // memory, and in the leading CTA (rank 0 of the pair) issues the MMAs for both; warps 2..5
-// read the CTA's half of the accumulator back (its 128 rows) and store it.
+// read the CTA's half of the accumulator back (its 128 rows) and store it (see TMA_C).
 // Barriers (same offsets in both CTAs):
 //   full[s]      in the leader: both CTAs' loads of stage s have landed (the peer's copies
 //                complete their bytes on the leader's barrier);
@@ -40,8 +40,12 @@ constexpr int ACC_BUFS = 2;
 constexpr int STAGE_A = BM * BK * 2;        // 16 KB
 constexpr int STAGE_B = (BN / 2) * BK * 2;  // 16 KB: this CTA's half of the weight rows
 constexpr int STAGE = STAGE_A + STAGE_B;
-constexpr int STAGES = 6;
-constexpr int SMEM = STAGES * STAGE + 1024 /*alignment*/ + 256 /*barriers*/;
+// With the output passing through shared memory (TMA_C) the ring has five stages and each of the four epilogue warps four
+// boxes of 32 rows x 128 bytes; six stages else.
+constexpr int stages_of(bool tma_c) { return tma_c ? 5 : 6; }
+constexpr int BOX = 32 * 128;
+constexpr int BOXES = 4;  // per epilogue warp
+constexpr int smem_of(bool tma_c) { return stages_of(tma_c) * STAGE + (tma_c ? 4 * BOXES * BOX : 0) + 1024 /*alignment*/ + 512 /*barriers*/; }
 constexpr int TMEM_COLS = ACC_BUFS * BN;    // 512
 
 struct Params2 {
@@ -58,6 +62,7 @@ struct Params2 {
     // parts, part s written to the slice s of the output, split_stride elements apart, as C[token][weight row].
     int n_split, kb_per_split;
     long long split_stride;
+    int band = 8;          // row tiles of a band (see tile_of, launch2)
     int out_act = 0;       // not DUAL, bfloat16 out: 1 = C is max(z, 0)^2 of the product
     int gate_act = 0;      // DUAL: what the gate goes through, 0 SiLU, 1 tanh-GELU
 };
@@ -152,34 +157,80 @@ __device__ __forceinline__ void store32<bf16>(bf16* dst, const uint32_t* r, int 
     }
 }
 
-// Which tile is the w-th?  Tiles are walked in bands of GROUP_M row tiles: within a band the row tile
+// Which tile is the w-th?  Tiles are walked in bands of `band_rows` row tiles: within a band the row tile
 // runs fastest, then the column tile, so that the clusters at work at one time share a few row tiles'
 // tokens and a few column tiles' weights, and a band's tokens stay in L2 while all weights pass by.
 // (Row tile fastest over ALL rows, as a first version had it, reads every token once per column tile:
 // with 75 k tokens the activations no longer fit L2 and the product ran at the speed of DRAM.)
-constexpr int GROUP_M = 8;
-__device__ __forceinline__ void tile_of(long long w, int tiles_m, int tiles_n, int& tm, int& tn) {
-    const long long band_tiles = (long long)GROUP_M * tiles_n;
+__device__ __forceinline__ void tile_of(long long w, int tiles_m, int tiles_n, int band_rows, int& tm, int& tn) {
+    const long long band_tiles = (long long)band_rows * tiles_n;
     const int band = (int)(w / band_tiles);
     const int in_band = (int)(w - band * band_tiles);
-    const int rows = min(GROUP_M, tiles_m - band * GROUP_M);
-    tm = band * GROUP_M + in_band % rows;
+    const int rows = min(band_rows, tiles_m - band * band_rows);
+    tm = band * band_rows + in_band % rows;
     tn = in_band / rows;
 }
 
-template <typename TO, bool DUAL, bool WIDE = false>
+// A box of the output (32 rows x 128 bytes, 128-byte swizzle) from shared memory to the matrix.
+__device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, int c0, int c1, const void* smem_src) {
+    asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group [%0, {%1, %2}], [%3];" ::"l"(map), "r"(c0), "r"(c1),
+                 "r"(tc::smem_u32(smem_src))
+                 : "memory");
+    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+}
+// All but the newest N of this thread's stores have been read out of shared memory.
+template <int N>
+__device__ __forceinline__ void tma_store_wait_read() { asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(N) : "memory"); }
+// All of this thread's stores are done.
+__device__ __forceinline__ void tma_store_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
+
+// The activation of DUAL: r becomes act(gate) * up, 32 columns.
+__device__ __forceinline__ void gate_up32(uint32_t (&r)[32], const uint32_t (&u)[32], int gate_act) {
+    if (gate_act == 0) {
+        // h = gate * sigmoid(gate) * up (infer/forward.odin:128-133)
+#pragma unroll
+        for (int q = 0; q < 32; ++q) {
+            float g = __uint_as_float(r[q]);
+            g = __fdividef(g, 1.0f + __expf(-g));  // one ex2 and one rcp: the epilogue's arithmetic is not free beside the MMAs
+            r[q] = __float_as_uint(g * __uint_as_float(u[q]));
+        }
+    } else {
+        // tanh-GELU: g (1 + tanh(y)) / 2 = g sigmoid(2 y), y = sqrt(2 / pi) (g + 0.044715 g^3)
+#pragma unroll
+        for (int q = 0; q < 32; ++q) {
+            float g = __uint_as_float(r[q]);
+            const float y2 = 1.5957691216057308f * g * fmaf(0.044715f * g, g, 1.0f);
+            g = __fdividef(g, 1.0f + __expf(-y2));
+            r[q] = __float_as_uint(g * __uint_as_float(u[q]));
+        }
+    }
+}
+
+// TMA_C: the output is read (accumulate) and written in boxes through shared memory (map_c).  A thread of the epilogue
+// holds a row, so that stores straight from its registers write 16 bytes of 32 rows at a time, half a sector each, and
+// adding to C waits for such loads 32 columns at a time; boxes are whole 128-byte lines, and the next ones' old values are
+// on their way while one is worked on.  The same bits.  What it measured, under the power cap (cuBLAS without the add or
+// the SwiGLU beside it): 12001 x 4096 x 4096 added to C 407 -> 347 us (300), 12001 x 4096 x 12288 1,036 -> 976 (887),
+// 12001 x 6144 x 4096 in bfloat16 494 -> 460 (449), 12001 x 24576 x 4096 with the SwiGLU 1,834 -> 1,742 (1,749), 66048 x
+// 4096 x 2048 in bfloat16 953 -> 846 (826).  What bounds it: the power cap; adding to C moves 8 bytes an element more.
+template <typename TO, bool DUAL, bool WIDE, bool TMA_C>
 __global__ void __launch_bounds__(192, 1)
-gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w, const Params2 p) {
+gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,
+                const __grid_constant__ CUtensorMap map_c, const Params2 p) {
+    static_assert(!(WIDE && TMA_C), "the transposed output is stored by threads");
+    constexpr int STAGES = stages_of(TMA_C);
     constexpr int ACC_N = DUAL ? BN / 2 : BN;  // columns of one product of the pair (DUAL: gate and up, 128 each)
     extern __shared__ uint8_t smem_raw[];
     // the same offsets in both CTAs: the dynamic shared memory starts at the same place in each
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + STAGES * STAGE);
+    uint8_t* boxes = smem + STAGES * STAGE;  // TMA_C: [epilogue warp][BOXES][BOX]
+    uint64_t* bars = reinterpret_cast<uint64_t*>(boxes + (TMA_C ? 4 * BOXES * BOX : 0));
     uint64_t* full = bars;
     uint64_t* empty = bars + STAGES;
     uint64_t* acc_full = bars + 2 * STAGES;
     uint64_t* acc_empty = acc_full + ACC_BUFS;
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + ACC_BUFS);
+    uint64_t* box_full = acc_empty + ACC_BUFS;  // TMA_C: [epilogue warp][BOXES] the old values have landed
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(box_full + 4 * BOXES);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -196,10 +247,13 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
             tc::mbar_init(&acc_full[a], 1);
             tc::mbar_init(&acc_empty[a], 8);  // four epilogue warps in each of the two CTAs
         }
+        if (TMA_C)
+            for (int b = 0; b < 4 * BOXES; ++b) tc::mbar_init(&box_full[b], 1);
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         tc::prefetch_tensormap(&map_a);
         tc::prefetch_tensormap(&map_w);
+        if (TMA_C) tc::prefetch_tensormap(&map_c);
     }
     if (warp == 1) tmem_alloc_pair(tmem_slot, TMEM_COLS);
     tc::fence_before_sync();
@@ -227,7 +281,7 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
                     tn = (int)(w % p.tiles_n); tm = (int)(rest / p.n_split);
                     kb0 = (int)(rest % p.n_split) * p.kb_per_split; kb1 = min(p.kb_total, kb0 + p.kb_per_split);
                 } else {
-                    tile_of(w, p.tiles_m, p.tiles_n, tm, tn);
+                    tile_of(w, p.tiles_m, p.tiles_n, p.band, tm, tn);
                 }
                 const int row_a = tm * 2 * BM + (int)rank * BM;
                 for (int kb = kb0; kb < kb1; ++kb) {
@@ -289,6 +343,135 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
         }
     } else {
         // ------------------------------------------------------------ epilogue (both CTAs)
+      if constexpr (TMA_C) {
+        const int quarter = warp & 3, ew = warp - 2;
+        constexpr int BOX_N = 128 / (int)sizeof(TO);   // columns of a box
+        constexpr int NBOX = ACC_N / BOX_N;
+        constexpr bool F32 = std::is_same<TO, float>::value;
+        const bool add = F32 && !DUAL && p.accumulate;
+        uint8_t* my_box = boxes + ew * BOXES * BOX;
+        uint64_t* my_full = box_full + ew * BOXES;
+        pdl_wait();
+        const uint32_t acc_empty_leader0 = map_to_rank(&acc_empty[0], 0);
+        // this warp's boxes in the order in which it comes to them: tile by tile, those that hold any of C.  `ahead` walks
+        // up to BOXES - 1 boxes before the one at work (lane 0, adding to C): its old values are asked for.
+        struct Walk { long long w; int b; int row, col; } ahead{cluster_id, -1, 0, 0};
+        auto step = [&](Walk& k) -> bool {
+            for (;;) {
+                if (++k.b == NBOX) { k.b = 0; k.w += n_clusters; }
+                if (k.w >= n_tiles) { k.b = NBOX - 1; return false; }
+                int tm, tn;
+                tile_of(k.w, p.tiles_m, p.tiles_n, p.band, tm, tn);
+                k.row = tm * 2 * BM + (int)rank * BM + quarter * 32;
+                k.col = tn * ACC_N + k.b * BOX_N;
+                if (k.row < p.M && k.col < p.N) return true;
+            }
+        };
+        uint32_t asked = 0;
+        auto ask = [&]() {
+            if (!step(ahead)) return;
+            const uint32_t s = asked % BOXES;
+            tc::mbar_expect_tx(&my_full[s], BOX);
+            tc::tma_load_2d(my_box + s * BOX, &map_c, ahead.col, ahead.row, &my_full[s]);
+            ++asked;
+        };
+        if (add && lane == 0)
+            for (int k = 0; k < BOXES - 1; ++k) ask();
+        uint32_t local = 0, n = 0;   // tiles and boxes done
+        bool ok = true;
+        for (long long w = cluster_id; w < n_tiles && ok; w += n_clusters, ++local) {
+            int tm, tn;
+            tile_of(w, p.tiles_m, p.tiles_n, p.band, tm, tn);
+            const uint32_t acc = local % ACC_BUFS, acc_phase = (local / ACC_BUFS) & 1;
+            ok = __all_sync(0xffffffffu, tc::mbar_wait(&acc_full[acc], acc_phase, abort_flag));
+            if (!ok) { if (lane == 0 && quarter == 2) report2(p.error, 4, (int)w, -1, (int)acc); break; }
+            tc::fence_after_sync();
+            const int row = tm * 2 * BM + (int)rank * BM + quarter * 32;
+            const uint32_t tacc = tmem_base + ((uint32_t)(quarter * 32) << 16) + acc * BN;
+#pragma unroll 1
+            for (int b = 0; b < NBOX; ++b) {
+                const int col = tn * ACC_N + b * BOX_N;
+                if (row >= p.M || col >= p.N) continue;
+                const uint32_t s = n % BOXES;
+                uint8_t* line = my_box + s * BOX + lane * 128;   // this thread's row of the box; piece q is stored at q ^ (row & 7)
+                if (add) {
+                    ok = __all_sync(0xffffffffu, tc::mbar_wait(&my_full[s], (n / BOXES) & 1, abort_flag));
+                    if (!ok) { if (lane == 0) report2(p.error, 5, (int)w, b, (int)s); break; }
+                } else {
+                    if (lane == 0) tma_store_wait_read<BOXES - 1>();   // the box's last store has left it
+                    __syncwarp();
+                }
+#pragma unroll
+                for (int half = 0; half < BOX_N / 32; ++half) {
+                    const int c0 = b * BOX_N + half * 32;
+                    uint32_t r[32];
+                    // DUAL: output column c0 + q has its gate in accumulator column c0 + q (+ 64 for the peer's
+                    // rows, c0 >= 64) and its up 64 columns further
+                    const uint32_t taddr = tacc + c0 + ((DUAL && c0 >= BN / 4) ? BN / 4 : 0);
+                    tc::tmem_ld32(taddr, r);
+                    if constexpr (DUAL) {
+                        uint32_t u[32];
+                        tc::tmem_ld32(taddr + BN / 4, u);
+                        tc::tmem_ld_wait();
+                        gate_up32(r, u, p.gate_act);
+                    } else {
+                        tc::tmem_ld_wait();
+                        if (!F32 && p.out_act) {
+#pragma unroll
+                            for (int q = 0; q < 32; ++q) {
+                                const float z = fmaxf(__uint_as_float(r[q]), 0.f);
+                                r[q] = __float_as_uint(z * z);
+                            }
+                        }
+                    }
+                    if constexpr (F32) {
+#pragma unroll
+                        for (int q = 0; q < 8; ++q) {
+                            float4* at = reinterpret_cast<float4*>(line + ((q ^ (lane & 7)) << 4));
+                            float4 v = make_float4(__uint_as_float(r[4 * q]), __uint_as_float(r[4 * q + 1]), __uint_as_float(r[4 * q + 2]),
+                                                   __uint_as_float(r[4 * q + 3]));
+                            if (add) {
+                                const float4 old = *at;
+                                v.x = old.x + v.x; v.y = old.y + v.y; v.z = old.z + v.z; v.w = old.w + v.w;
+                            }
+                            *at = v;
+                        }
+                    } else {
+#pragma unroll
+                        for (int q = 0; q < 4; ++q) {
+                            uint32_t h[4];
+#pragma unroll
+                            for (int j = 0; j < 4; ++j) {
+                                const __nv_bfloat162 v = __floats2bfloat162_rn(__uint_as_float(r[8 * q + 2 * j]), __uint_as_float(r[8 * q + 2 * j + 1]));
+                                h[j] = *reinterpret_cast<const uint32_t*>(&v);
+                            }
+                            *reinterpret_cast<uint4*>(line + (((half * 4 + q) ^ (lane & 7)) << 4)) = make_uint4(h[0], h[1], h[2], h[3]);
+                        }
+                    }
+                }
+                tc::fence_proxy_async();
+                __syncwarp();
+                if (lane == 0) {
+                    tma_store_2d(&map_c, col, row, my_box + s * BOX);
+                    if (add) {
+                        tma_store_wait_read<1>();   // the box before this one has left: its place takes the old values of the box BOXES - 1 on
+                        ask();
+                    }
+                }
+                ++n;
+            }
+            if (!ok) break;
+            tc::fence_before_sync();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_cluster(acc_empty_leader0 + acc * 8);
+        }
+        if (lane == 0) {
+            for (; n < asked; ++n)   // aborted: let the copies already in flight land before the CTA's memory is released
+                for (uint32_t i = 0; i < 4096; ++i)
+                    if (tc::mbar_try_wait(&my_full[n % BOXES], (n / BOXES) & 1)) break;
+            tma_store_wait_all();
+        }
+      } else {
         const int quarter = warp & 3;  // the TMEM lanes this warp may read: [32*quarter, +32)
         pdl_wait();
         uint32_t local = 0;
@@ -297,7 +480,7 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
         for (long long w = cluster_id; w < n_tiles && ok; w += n_clusters, ++local) {
             int tm, tn;
             if (WIDE) { tn = (int)(w % p.tiles_n); tm = (int)((w / p.tiles_n) / p.n_split); }
-            else tile_of(w, p.tiles_m, p.tiles_n, tm, tn);
+            else tile_of(w, p.tiles_m, p.tiles_n, p.band, tm, tn);
             const uint32_t acc = local % ACC_BUFS, acc_phase = (local / ACC_BUFS) & 1;
             if (!tc::mbar_wait(&acc_full[acc], acc_phase, abort_flag)) { if (lane == 0 && quarter == 2) report2(p.error, 4, (int)w, -1, (int)acc); ok = false; break; }
             tc::fence_after_sync();
@@ -332,23 +515,7 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
                     tc::tmem_ld32(taddr, r);
                     tc::tmem_ld32(taddr + BN / 4, u);
                     tc::tmem_ld_wait();
-                    if (p.gate_act == 0) {
-#pragma unroll
-                        for (int q = 0; q < 32; ++q) {
-                            float g = __uint_as_float(r[q]);
-                            g = __fdividef(g, 1.0f + __expf(-g));  // one ex2 and one rcp: the epilogue's arithmetic is not free beside the MMAs
-                            r[q] = __float_as_uint(g * __uint_as_float(u[q]));
-                        }
-                    } else {
-                        // tanh-GELU: g (1 + tanh(y)) / 2 = g sigmoid(2 y), y = sqrt(2 / pi) (g + 0.044715 g^3)
-#pragma unroll
-                        for (int q = 0; q < 32; ++q) {
-                            float g = __uint_as_float(r[q]);
-                            const float y2 = 1.5957691216057308f * g * fmaf(0.044715f * g, g, 1.0f);
-                            g = __fdividef(g, 1.0f + __expf(-y2));
-                            r[q] = __float_as_uint(g * __uint_as_float(u[q]));
-                        }
-                    }
+                    gate_up32(r, u, p.gate_act);
                 } else {
                     tc::tmem_ld32(taddr, r);
                     tc::tmem_ld_wait();
@@ -386,6 +553,7 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
             __syncwarp();
             if (lane == 0) mbar_arrive_cluster(acc_empty_leader0 + acc * 8);
         }
+      }
     }
 
     tc::fence_before_sync();
@@ -431,6 +599,21 @@ int make_map2(CUtensorMap* out, const void* ptr, long long rows, long long K, lo
     return r == CUDA_SUCCESS ? 0 : ODIN_ERR_BAD_ARG;
 }
 
+// The output [rows, N] with row stride ld, in boxes of 32 rows x 128 bytes.  False where TMA cannot write it: rows that do
+// not start on 16 bytes, or do not end on them (a store cut off at the edge of the matrix is cut at whole 16 bytes).
+bool make_map_c(CUtensorMap* out, void* ptr, int c_dtype, long long rows, long long N, long long ld) {
+    const int size = c_dtype == ODIN_F32 ? 4 : 2;
+    EncodeTiledFn fn = encode_fn2();
+    if (fn == nullptr || (((uintptr_t)ptr) & 15) || (ld * size) % 16 || (N * size) % 16) return false;
+    cuuint64_t dims[2] = {(cuuint64_t)N, (cuuint64_t)rows};
+    cuuint64_t strides[1] = {(cuuint64_t)(ld * size)};
+    cuuint32_t box[2] = {(cuuint32_t)(128 / size), 32};
+    cuuint32_t estr[2] = {1, 1};
+    return fn(out, size == 4 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, ptr, dims, strides, box, estr,
+              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 int* error_flag2() {
     static int* flag = nullptr;
     static std::once_flag once;
@@ -441,9 +624,10 @@ int* error_flag2() {
     return flag;
 }
 
-template <typename TO, bool DUAL, bool WIDE = false>
-int launch2(const CUtensorMap& ma, const CUtensorMap& mw, const Params2& p, cudaStream_t s) {
-    auto kern = gemm_tc2_kernel<TO, DUAL, WIDE>;
+template <typename TO, bool DUAL, bool WIDE, bool TMA_C>
+int launch2_as(const CUtensorMap& ma, const CUtensorMap& mw, const CUtensorMap& mc, const Params2& p, cudaStream_t s) {
+    constexpr int SMEM = smem_of(TMA_C);
+    auto kern = gemm_tc2_kernel<TO, DUAL, WIDE, TMA_C>;
     static int max_clusters = -1;
     if (max_clusters < 0) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
@@ -478,9 +662,21 @@ int launch2(const CUtensorMap& ma, const CUtensorMap& mw, const Params2& p, cuda
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = odin_pdl_enabled() ? 2 : 1;
-    cudaLaunchKernelEx(&cfg, kern, ma, mw, p);
+    cudaLaunchKernelEx(&cfg, kern, ma, mw, mc, p);
     ODIN_LAUNCH_CHECK();
     return 0;
+}
+
+template <typename TO, bool DUAL>
+int launch2(const CUtensorMap& ma, const CUtensorMap& mw, Params2 p, cudaStream_t s) {
+    CUtensorMap mc;
+    // Row tiles of a band: enough that the weights pass by seldom, few enough that the band's tokens stay in L2 beside
+    // them.  12001 x 24576 x 4096 with the SwiGLU: 1,861, 1,774 and 1,742 us with 4, 8 and 16; 12001 x 4096 x 12288 added
+    // to C: 981, 976, 997; 66048 x 2048 x 6144: 1,350, 1,364, 1,410.
+    p.band = p.K <= 4096 ? 16 : 8;
+    if (make_map_c(&mc, p.out, std::is_same<TO, float>::value ? ODIN_F32 : ODIN_BF16, p.M, p.N, p.ldc))
+        return launch2_as<TO, DUAL, false, true>(ma, mw, mc, p, s);
+    return launch2_as<TO, DUAL, false, false>(ma, mw, ma, p, s);
 }
 
 }  // namespace
@@ -582,8 +778,8 @@ extern "C" int odin_gemm_tc2_wide(const void* A, const void* W, void* C, int c_d
     if ((rc = make_map2(&ma, W, N, K, ldw, BM))) return rc;
     if ((rc = make_map2(&mw, A, M, K, lda, BN / 2))) return rc;
     cudaStream_t s = (cudaStream_t)stream;
-    if (c_dtype == ODIN_BF16) return launch2<bf16, false, true>(ma, mw, p, s);
-    if (c_dtype == ODIN_F32) return launch2<float, false, true>(ma, mw, p, s);
+    if (c_dtype == ODIN_BF16) return launch2_as<bf16, false, true, false>(ma, mw, ma, p, s);
+    if (c_dtype == ODIN_F32) return launch2_as<float, false, true, false>(ma, mw, ma, p, s);
     return ODIN_ERR_UNSUPPORTED;
 }
 

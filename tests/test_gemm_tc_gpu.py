@@ -330,6 +330,37 @@ extern "C" int bad_product_launch(const void* A, const void* W, float* C, int M,
 """
 
 
+@pytest.mark.parametrize("M,N,K", [(257, 132, 64), (300, 300, 200), (511, 264, 4160), (769, 513, 128), (4500, 1104, 72)])
+@pytest.mark.parametrize("kind", ["bf16", "f32", "add", "relu2"])
+def test_pair_kernel_output_boxes_same_bits(M, N, K, kind):
+    """The pair kernel's output goes through shared memory in boxes where TMA reaches its rows, and from registers where a
+    row does not start and end on 16 bytes: the same bits, nothing written beside the matrix, at edges of tiles, boxes and bands
+    (more than 16 row tiles: two bands)."""
+    from odin_infer_b200.csrc import ops
+    torch.manual_seed(M + N)
+    a = torch.randn(M, K, device=DEV).bfloat16()
+    w = torch.randn(N, K, device=DEV).bfloat16()
+    dtype = torch.bfloat16 if kind in ("bf16", "relu2") else torch.float32
+    wide = (N + 7) // 8 * 8 + 8
+    old = torch.randn(M + 1, N, device=DEV).to(dtype)
+    outs = []
+    for stride in (wide, wide + 1):
+        buf = torch.full((M + 1, stride), 7.0, device=DEV, dtype=dtype)
+        buf[:, :N] = old
+        torch.cuda.synchronize()
+        ops.gemm_tc2(a, w, buf[:M, :N], accumulate=kind == "add", **({"relu2": True} if kind == "relu2" else {}))
+        torch.cuda.synchronize()
+        assert (buf[:, N:] == 7.0).all() and torch.equal(buf[M, :N], old[M])
+        outs.append(buf[:M, :N].clone())
+    assert torch.equal(outs[0], outs[1])
+    ref = a.double() @ w.double().t()
+    ref = ref + old[:M].double() if kind == "add" else ref.clamp(min=0) ** 2 if kind == "relu2" else ref
+    # 32-bit sums of K products of unit normals: a few times sqrt(K) 2^-24 sqrt(K); bfloat16 rounds once, relative 2^-8
+    tol = 4e-7 * K if dtype == torch.float32 else 2 ** -8 * ref.abs().max().item()
+    assert (outs[0].double() - ref).abs().max().item() <= tol
+    ops.gemm_tc_check()
+
+
 def test_ladder_catches_a_known_bad_product(tmp_path):
     """The regression guard of the ladder itself: a product that skips every second block of K must
     fail at the first rung (all ones gives K/2), and with the names of the later rungs too."""

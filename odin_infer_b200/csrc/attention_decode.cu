@@ -238,8 +238,11 @@ attn_decode_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     pdl_trigger();
+    int t = (int)blockIdx.z;
+    if (p.by_length > 0)
+        t = attn_decode::token_by_length(p, t, (int)threadIdx.x, reinterpret_cast<int*>(smem + DecodeTcSmem<HD, SLOTS>::PAGES_AT));
     attn_decode::attn_decode_tc_body<HD, SLOTS, PREP, 0>(map_k, map_v, p, smem, (int)threadIdx.x, (int)blockIdx.x,
-                                                         (int)blockIdx.y, (int)blockIdx.z, [] { pdl_wait(); });
+                                                         (int)blockIdx.y, t, [] { pdl_wait(); });
 }
 
 // out[t][h][:] = sum_s w_s acc_s / sum_s w_s l_s, w_s = 2^(m_s - max m)
@@ -407,6 +410,8 @@ int launch_decode_tc(const bf16* q, size_t q_stride, bf16* out, size_t out_strid
     static int deep_upto = -1;
     if (deep_upto < 0) { const char* e = getenv("ODIN_DECODE_DEEP_UPTO"); deep_upto = e ? atoi(e) : 32; }
     const bool deep = ctas <= deep_upto;
+    // more CTAs than are resident together (two an SM): the longest sequences first
+    p.by_length = (ctas > 2LL * sms && B > 1 && B <= attn_decode::BY_LENGTH_MAX) ? B : 0;
 #define GO(PREP)                                                                  \
     (deep ? launch_decode_tc_slots<HD, 6, PREP>(mk, mv, p, grid, s)               \
           : launch_decode_tc_slots<HD, 3, PREP>(mk, mv, p, grid, s))

@@ -375,6 +375,38 @@ def test_experts_of_few_rows(T, E, per, d, ff, kind, gated, weigh_input):
     assert torch.equal(y1[:, 0], y[:, t])
 
 
+@pytest.mark.parametrize("n_seqs", [39, 64, 128, 130])
+@pytest.mark.parametrize("window", [0, 100])
+def test_decode_attention_of_many_unequal_sequences(n_seqs, window):
+    """More (sequence, kv head) items than fit the GPU at once start with the longest sequences: every sequence's result is
+    what it is alone, padding rows are left alone."""
+    from odin_infer_b200.csrc import ops
+    n_q, n_kv, hd = 16, 8, 128
+    torch.manual_seed(n_seqs)
+    lengths = [int(v) for v in torch.randint(1, 700, (n_seqs,))]
+    k, v, bt = paged_cache(n_seqs, lengths, n_kv, hd, torch.bfloat16)
+    for s, n in enumerate(lengths):
+        for p in range((n + 63) // 64):
+            m = min(64, n - p * 64)
+            k[bt[s, p], :, :m] = torch.randn(n_kv, m, hd, device=DEV).bfloat16()
+            v[bt[s, p], :, :m] = torch.randn(n_kv, m, hd, device=DEV).bfloat16()
+    q = torch.randn(n_seqs, n_q * hd, device=DEV).bfloat16()
+    tok_pos = torch.tensor([n - 1 for n in lengths], dtype=torch.int32, device=DEV)
+    tok_seq = torch.arange(n_seqs, dtype=torch.int32, device=DEV)
+    tok_seq[5] = -1
+    scratch = torch.empty(ops.attention_decode_scratch(n_seqs, n_q, hd, 1), device=DEV)
+    out = torch.full((n_seqs, n_q * hd), 7.0, device=DEV, dtype=torch.bfloat16)
+    torch.cuda.synchronize()
+    ops.attention_decode(q, out, n_q, n_kv, hd, k, v, tok_pos, tok_seq, bt, window, scratch, 1)
+    one = torch.empty(1, n_q * hd, device=DEV, dtype=torch.bfloat16)
+    for s in list(range(0, n_seqs, 7)) + [n_seqs - 1]:
+        ops.attention_decode(q[s:s + 1], one, n_q, n_kv, hd, k, v, tok_pos[s:s + 1], torch.zeros(1, dtype=torch.int32, device=DEV),
+                             bt[s:s + 1], window, scratch, 1)
+        assert torch.equal(one[0], out[s])
+    assert (out[5] == 7.0).all()
+    ops.attention_decode_check()
+
+
 @pytest.mark.parametrize("geom", [(8, 2, 128), (6, 3, 64)])
 @pytest.mark.parametrize("parts", [0, 2])
 def test_head_prep_many_tokens_equals_few_at_a_time(geom, parts):

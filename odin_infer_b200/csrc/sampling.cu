@@ -88,33 +88,39 @@ __device__ __forceinline__ float masked_sum(const float* row, int V, float inv_t
     return block_sum(s, red);
 }
 
-// P block-wide sums side by side, each in the order of block_sum: two barriers for all of them instead of two for each (a
-// row of 384 draws in 58 us with one sum after the other, most of it barriers).  red: [P][32].
+// P block-wide sums side by side, each in the order of block_sum.  What bounds a pass over a short row is not the row but
+// the shuffles of its sums, two rounds of P x 5 in all 32 warps when every warp adds up for itself: here the warps beyond
+// the row (their sums are zero) take no part in the first round, and one warp per sum does the second.  Draws from rows of
+// 384: 57.5 us a launch with one block sum after the other, 52.8 so.
+// red: [P][32], tot: [P].
 template <int P>
-__device__ __forceinline__ void block_sums(float (&v)[P], float (*red)[32]) {
+__device__ __forceinline__ void block_sums(float (&v)[P], int V, float (*red)[32], float* tot) {
+    static_assert(P <= 32, "a warp per sum");
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (warp * 32 < V) {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
+        for (int o = 16; o > 0; o >>= 1)
 #pragma unroll
-        for (int q = 0; q < P; ++q) v[q] += __shfl_xor_sync(0xffffffffu, v[q], o);
-    __syncthreads();
+            for (int q = 0; q < P; ++q) v[q] += __shfl_xor_sync(0xffffffffu, v[q], o);
+    }
 #pragma unroll
     for (int q = 0; q < P; ++q)
         if (lane == q) red[q][warp] = v[q];
     __syncthreads();
+    if (warp < P) {
+        const float t = warp_sum(red[warp][lane]);  // SB = 1024 threads = 32 warps
+        if (lane == 0) tot[warp] = t;
+    }
+    __syncthreads();
 #pragma unroll
-    for (int q = 0; q < P; ++q) v[q] = red[q][lane];  // SB = 1024 threads = 32 warps
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-        for (int q = 0; q < P; ++q) v[q] += __shfl_xor_sync(0xffffffffu, v[q], o);
+    for (int q = 0; q < P; ++q) v[q] = tot[q];
 }
 
 // The largest t in [lo, hi] (bit patterns of positive floats, which order like the floats) with
 // S(t) = sum of e_i >= t  >  target, given S(lo) > target.  S falls as t grows.  Eight probes per
 // pass over the row, so 2^30 candidates take ten passes instead of thirty.
 __device__ unsigned search_threshold(const float* row, int V, float inv_t, float m, float target, unsigned lo,
-                                     unsigned hi, float (*red)[32]) {
+                                     unsigned hi, float (*red)[32], float* tot) {
     constexpr int P = 8;
     while (lo < hi) {
         const unsigned span = hi - lo;  // probes lo < p_0 < ... <= hi
@@ -131,7 +137,7 @@ __device__ unsigned search_threshold(const float* row, int V, float inv_t, float
             for (int q = 0; q < P; ++q)
                 if (e >= __uint_as_float(probe[q])) acc[q] += e;
         }
-        block_sums<P>(acc, red);
+        block_sums<P>(acc, V, red, tot);
         int best = -1;
 #pragma unroll
         for (int q = 0; q < P; ++q)
@@ -157,7 +163,7 @@ __global__ void __launch_bounds__(SB) sample_kernel(const float* __restrict__ lo
                                                     float temperature, float top_p,
                                                     const float* __restrict__ coins, int* __restrict__ out) {
     __shared__ float red[32];
-    __shared__ float reds[8][32];
+    __shared__ float reds[8][32], tots[8];
     __shared__ __align__(16) float chunk_sum[SB];
     __shared__ int chosen;
     pdl_trigger();
@@ -181,7 +187,7 @@ __global__ void __launch_bounds__(SB) sample_kernel(const float* __restrict__ lo
         float cumulative = s_cut;  // the candidates together do not exceed topp: all of them stay
         if (s_cut > target) {
             // v: the value of the candidate at which the cumulative sum first exceeds topp
-            lo = search_threshold(row, V, inv_t, mx, target, lo, __float_as_uint(1.0f), reds);
+            lo = search_threshold(row, V, inv_t, mx, target, lo, __float_as_uint(1.0f), reds, tots);
             const float v = __uint_as_float(lo);
             const float above = masked_sum(row, V, inv_t, mx, __uint_as_float(lo + 1), red);
             const float ties = floorf((target - above) / v) + 1.0f;  // how many of value v it takes
@@ -192,7 +198,7 @@ __global__ void __launch_bounds__(SB) sample_kernel(const float* __restrict__ lo
         float u = __uint_as_float(lo);
         int nth = 0x7fffffff;  // which of the tokens of value u, in index order (beyond their number: the last)
         if (masked_sum(row, V, inv_t, mx, u, red) > r) {
-            ub = search_threshold(row, V, inv_t, mx, r, lo, __float_as_uint(1.0f), reds);
+            ub = search_threshold(row, V, inv_t, mx, r, lo, __float_as_uint(1.0f), reds, tots);
             u = __uint_as_float(ub);
             const float above = masked_sum(row, V, inv_t, mx, __uint_as_float(ub + 1), red);
             nth = (int)fminf(floorf(fmaxf(r - above, 0.f) / u), 2.0e9f);

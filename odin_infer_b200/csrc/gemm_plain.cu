@@ -192,24 +192,23 @@ __global__ void __launch_bounds__(ROWS_THREADS) gemm_f32_rows_kernel(const float
 }
 
 // ---- many rows of A --------------------------------------------------------
-// Tiles of 64 x 32, 128 threads, 4 x 4 outputs each (rows ty + 16 i, columns tx + 8 j); K in steps of 32 through a ring
-// filled with 16-byte asynchronous copies, pieces stored at piece ^ (row & 7).  A thread reads four k of each of its rows
-// and columns at a time.  A warp is 8 x 4 threads, laid out so that neighbouring lanes read the same row of A, and lanes
-// two apart the same column: such a load takes the shared memory 2.2 cycles, one whose pairs of neighbours differ 4.0
-// (measured).
+// TY x TX threads, RM x RN outputs each (rows ty + TY i, columns tx + TX j); K in steps of 32 through a ring filled with
+// 16-byte asynchronous copies, pieces stored at piece ^ (row & 7).  A thread reads four k of each of its rows and columns
+// at a time.  A warp is 8 x 4 threads, laid out so that neighbouring lanes read the same row of A, and lanes two apart the
+// same column: such a load takes the shared memory 2.2 cycles, one whose pairs of neighbours differ 4.0 (measured).
 // What bounds it: the multiply-adds (M N K of them, 128 per cycle and SM: 71 TFLOP/s measured) and beside them the
-// shared loads and the register banks.  922 x 12288 x 2048: 1,061 us, 43.7 TFLOP/s (1,915 us before).  Tiles of 128 x 128
-// with 8 x 8 outputs a thread run at 41.3 there and at 45.5 on 922 x 24576 x 4096 (these: 44.2), but leave the SMs idle
-// on anything smaller: 500 x 2048 x 2048 takes them 191 us, these 113.  Two multiply-adds an instruction (fma.rn.f32x2) on
-// tiles of 64 x 128 with both operands transposed on their way to shared memory, 4 bytes a copy: 1,117 us at best.
+// shared loads and the register banks.  Two sizes (see launch_tiles): 64 x 128 with 8 x 8 outputs a thread, two blocks an
+// SM, has half the shared loads per multiply-add; 64 x 32 with 4 x 4 occupies the SMs with a quarter of the tiles' work.
+// 922 x 12288 x 2048: 947 us (48.9 TFLOP/s) and 1,064, 1,915 before; 922 x 2048 x 6144: 569 and 574, 1,403 before; 500 x
+// 2048 x 2048: 185 and 113.  Two multiply-adds an instruction (fma.rn.f32x2) on tiles of 64 x 128 with both operands
+// transposed on their way to shared memory, 4 bytes a copy: 1,117 us on the first; tiles of 128 x 128: 1,124.
 constexpr int TILE_BK = 32;
 
-constexpr int RM = 4, RN = 4, TX = 8, TILE_STAGES = 4;
-constexpr int TILE_THREADS = 16 * TX, TMR = 16 * RM, TNR = TX * RN;  // 128 threads, 64 x 32 outputs
-
-__global__ void __launch_bounds__(TILE_THREADS, 4) gemm_f32_tile_kernel(const float* A, const float* __restrict__ W, float* C,
+template <int RM, int RN, int TX, int TY, int TILE_STAGES, int BLOCKS>
+__global__ void __launch_bounds__(TX * TY, BLOCKS) gemm_f32_tile_kernel(const float* A, const float* __restrict__ W, float* C,
                                                                        int M, int N, int K, size_t lda, size_t ldw, size_t ldc) {
-    constexpr int THREADS = TILE_THREADS;
+    constexpr int THREADS = TX * TY, TMR = TY * RM, TNR = TX * RN;
+    static_assert(TX % 8 == 0 && TY % 8 == 0, "a thread's rows and columns share (row & 7)");
     constexpr int STAGE = (TMR + TNR) * TILE_BK;
     constexpr int AHEAD = TILE_STAGES - 1;
     extern __shared__ __align__(128) float sm[];
@@ -265,11 +264,10 @@ __global__ void __launch_bounds__(TILE_THREADS, 4) gemm_f32_tile_kernel(const fl
 #pragma unroll
         for (int q = 0; q < TILE_BK / 4; ++q) {
             float4 w[RN], a[RM];
-            // a thread's rows are 16 and its columns TX apart, multiples of 8: (row & 7) is the same for all of them
 #pragma unroll
             for (int j = 0; j < RN; ++j) w[j] = *reinterpret_cast<const float4*>(ws + j * TX * TILE_BK + ((q ^ (tx & 7)) << 2));
 #pragma unroll
-            for (int i = 0; i < RM; ++i) a[i] = *reinterpret_cast<const float4*>(as + i * 16 * TILE_BK + ((q ^ (ty & 7)) << 2));
+            for (int i = 0; i < RM; ++i) a[i] = *reinterpret_cast<const float4*>(as + i * TY * TILE_BK + ((q ^ (ty & 7)) << 2));
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
 #pragma unroll
@@ -285,7 +283,7 @@ __global__ void __launch_bounds__(TILE_THREADS, 4) gemm_f32_tile_kernel(const fl
     cp_wait<0>();
 #pragma unroll
     for (int i = 0; i < RM; ++i) {
-        const int m = m0 + ty + 16 * i;
+        const int m = m0 + ty + TY * i;
         if (m >= M) continue;
 #pragma unroll
         for (int j = 0; j < RN; ++j) {
@@ -324,13 +322,24 @@ int launch_rows(const float* A, const float* W, float* C, int M, int N, int K, s
     return launch_rows_ring<MT, 3>(A, W, C, M, N, K, lda, ldw, ldc, s);
 }
 
+template <int RM, int RN, int TX, int TY, int STAGES, int BLOCKS>
 int launch_tile(const float* A, const float* W, float* C, int M, int N, int K, size_t lda, size_t ldw, size_t ldc, cudaStream_t s) {
-    constexpr int smem = TILE_STAGES * (TMR + TNR) * TILE_BK * 4;
-    const cudaError_t e = cudaFuncSetAttribute(gemm_f32_tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    constexpr int TMR = TY * RM, TNR = TX * RN, smem = STAGES * (TMR + TNR) * TILE_BK * 4;
+    auto k = gemm_f32_tile_kernel<RM, RN, TX, TY, STAGES, BLOCKS>;
+    const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return (int)e;
-    odin_launch(gemm_f32_tile_kernel, dim3((N + TNR - 1) / TNR, (M + TMR - 1) / TMR), dim3(TILE_THREADS), (size_t)smem, s, A, W, C,
-                M, N, K, lda, ldw, ldc);
+    odin_launch(k, dim3((N + TNR - 1) / TNR, (M + TMR - 1) / TMR), dim3(TX * TY), (size_t)smem, s, A, W, C, M, N, K, lda, ldw, ldc);
     return 0;
+}
+
+// Large tiles where their whole rounds (two blocks an SM: 189 us a round at K = 2048) take less than the small tiles'
+// rounds (four an SM, 106 us; a last round of fewer blocks takes accordingly less).
+int launch_tiles(const float* A, const float* W, float* C, int M, int N, int K, size_t lda, size_t ldw, size_t ldc, cudaStream_t s) {
+    const int sms = sm_count();
+    const long long rows = (M + 63) / 64, large = rows * ((N + 127) / 128), small = rows * ((N + 31) / 32);
+    const double rounds_large = (double)((large + 2 * sms - 1) / (2 * sms)), rounds_small = (double)small / (4.0 * sms);
+    if (189.0 * rounds_large < 106.0 * rounds_small) return launch_tile<8, 8, 16, 8, 3, 2>(A, W, C, M, N, K, lda, ldw, ldc, s);
+    return launch_tile<4, 4, 8, 16, 4, 4>(A, W, C, M, N, K, lda, ldw, ldc, s);
 }
 
 bool aligned16(const void* p) { return ((uintptr_t)p & 15) == 0; }
@@ -355,7 +364,7 @@ extern "C" int odin_gemm_plain(const void* A, int a_dtype, const void* W, int w_
         if (M <= 4) rc = launch_rows<1>(a, w, c, M, N, K, lda, ldw, ldc, s);
         else if (M <= 8) rc = launch_rows<2>(a, w, c, M, N, K, lda, ldw, ldc, s);
         else if (M <= ROWS_MAX) rc = launch_rows<4>(a, w, c, M, N, K, lda, ldw, ldc, s);
-        else rc = launch_tile(a, w, c, M, N, K, lda, ldw, ldc, s);
+        else rc = launch_tiles(a, w, c, M, N, K, lda, ldw, ldc, s);
         if (rc != 0) return rc;
         ODIN_LAUNCH_CHECK();
         return 0;

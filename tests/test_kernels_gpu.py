@@ -180,8 +180,8 @@ def test_gemm_plain_ladder(shape, combo):
     close(run(a, w), a.double() @ w.double().t(), (1e-7 * math.sqrt(K) if tc == torch.float32 else 5e-3))
 
 
-@pytest.mark.parametrize("M", [1, 3, 4, 5, 8, 9, 16, 17, 64, 65, 130])
-@pytest.mark.parametrize("N,K", [(5, 4), (31, 128), (32, 132), (33, 100), (300, 1028), (4800, 256)])
+@pytest.mark.parametrize("M", [1, 3, 4, 5, 8, 9, 16, 17, 64, 65, 130, 1000])
+@pytest.mark.parametrize("N,K", [(5, 4), (31, 128), (32, 132), (33, 100), (300, 1028), (4800, 256), (12001, 36)])
 def test_gemm_plain_same_bits_in_every_kernel(M, N, K):
     """32-bit rows of whole 16-byte vectors go to kernels of their own (up to 16 rows, and tiles); every output is the
     same chain of multiply-adds over k there, so the bits are those of the general kernel, which takes a weight whose

@@ -54,9 +54,9 @@ MOE_GROUPED_FROM_ROWS = int(os.environ.get("ODIN_MOE_GROUPED_FROM", "32"))
 
 # Up to this many rows (token, choice) per expert the experts' products take an expert's rows together straight from the
 # choices (see Runtime.experts).  Measured against the grouped products, both products of 32 experts of 2048 x 768 / 64 of
-# 4096 x 1024: 1 row per expert 51 against 80 us, 215 against 311; 3 rows 74 against 111, 366 against 393; 4.5 rows and up
-# 95 against 112, 463 against 386.
-MOE_FEW_ROWS_PER_EXPERT = int(os.environ.get("ODIN_MOE_FEW_UPTO", "4"))
+# 4096 x 1024: 1 row per expert 45 against 79 us, 178 against 239; 3 rows 67 against 111, 337 against 394; 4.5 rows 382
+# against 392; 6 rows 85 against 112, 412 against 395.
+MOE_FEW_ROWS_PER_EXPERT = int(os.environ.get("ODIN_MOE_FEW_UPTO", "5"))
 
 # from this many tokens on a product per head runs on the tensor cores
 HEADS_TC_FROM = 128

@@ -1000,7 +1000,8 @@ def rope_heads(src: torch.Tensor, src_head_stride: int, dst: torch.Tensor, dst_h
 
 
 def gemm_plain(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> None:
-    """out[M, N] = a[M, K] @ w[N, K]^T on the CUDA cores with 32-bit accumulation."""
+    """out[M, N] = a[M, K] @ w[N, K]^T on the CUDA cores with 32-bit accumulation.  w is a weight: like the tensor-core
+    products, the kernel for few rows may read it before the kernel launched before it has ended."""
     M, K = a.shape
     N = w.shape[0]
     assert w.shape[1] == K and out.shape == (M, N)

@@ -44,6 +44,9 @@ class DecodeGraphs:
     def __init__(self, rt, model, cache):
         self.rt, self.model, self.cache = rt, model, cache
         self._graphs: dict[tuple, tuple] = {}
+        # In 32-bit, whose logits are copied out right behind a replay, the graphs share their scratch memory: they replay one
+        # after the other on one stream, and nothing of a replay but its logits is read after it.
+        self._pool = torch.cuda.graph_pool_handle() if rt.dtype == torch.float32 else None
         self.last_h2d_bytes = 0
 
     def takes(self, entries: list[StepEntry]) -> bool:
@@ -88,7 +91,7 @@ class DecodeGraphs:
         torch.cuda.current_stream().synchronize()
         graph = torch.cuda.CUDAGraph()
         n0 = ops.launch_count()
-        with torch.cuda.graph(graph):
+        with torch.cuda.graph(graph, pool=self._pool):
             captured = self.rt.run(self.model, batch)
         n_kernels = ops.launch_count() - n0
         ops.add_launches(-n_kernels)          # recorded, not launched

@@ -34,7 +34,7 @@ GROUPS = {
     "state_space": ["state_space.cu"],
     "gated_unit": ["gated_unit.cu"],
     "streams": ["streams.cu"],
-    "moe": ["moe.cu", "moe_few.cu"],
+    "moe": ["moe.cu"],
     "moe_tc": ["moe_tc.cu"],
     "latent": ["latent.cu"],
     "gemm_plain": ["gemm_plain.cu"],

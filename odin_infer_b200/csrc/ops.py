@@ -469,38 +469,6 @@ def moe_down(a: torch.Tensor, w: torch.Tensor, ids: torch.Tensor, wts: torch.Ten
         c_int(per), c_int(ff), c_int(d), _ptr(out), _stream()), "moe_down")
 
 
-def moe_few_supported(h: torch.Tensor, w_gate_up: torch.Tensor, w_down: torch.Tensor) -> bool:
-    """Shapes and types that `moe_few_up` and `moe_few_down` take (bfloat16, rows of whole 16 bytes, whose inputs fit an SM)."""
-    return (h.shape[0] <= 512 and max(w_gate_up.shape[2], w_down.shape[2]) <= 5120 and w_gate_up.data_ptr() % 16 == 0
-            and w_down.data_ptr() % 16 == 0 and moe_grouped_supported(h, w_gate_up, w_down))
-
-
-def moe_few_up(h: torch.Tensor, w: torch.Tensor, ids: torch.Tensor, kind: str, out: torch.Tensor, gated: bool = True,
-               in_wts: torch.Tensor | None = None) -> None:
-    """`moe_gate_up` for bfloat16 with all rows of an expert together (tensor cores, the weights read once per 16 of them);
-    in_wts is multiplied in 32-bit and rounded once.  Rows of choices without an expert are left as they are."""
-    T, d = h.shape
-    per, ff = ids.shape[1], out.shape[1]
-    assert h.dtype == w.dtype == out.dtype == torch.bfloat16 and h.stride(1) == 1 and w.is_contiguous() and out.is_contiguous()
-    assert tuple(w.shape[1:]) == ((2 if gated else 1) * ff, d) and out.shape[0] == T * per
-    assert ids.dtype == torch.int32 and ids.is_contiguous() and ids.shape[0] == T
-    _check(_fn("moe", "odin_moe_few_up")(
-        _ptr(h), c_longlong(h.stride(0)), _ptr(w), _ptr(ids), _wts(in_wts, ids), c_int(T), c_int(per), c_int(w.shape[0]), c_int(ff),
-        c_int(d), c_int(ACTIVATIONS[kind]), c_int(1 if gated else 0), _ptr(out), _stream()), "moe_few_up")
-
-
-def moe_few_down(a: torch.Tensor, w: torch.Tensor, ids: torch.Tensor, wts: torch.Tensor | None, out: torch.Tensor) -> None:
-    """`moe_down` for bfloat16 with all rows of an expert together."""
-    T, per = ids.shape
-    ff, d = a.shape[1], w.shape[1]
-    assert a.dtype == w.dtype == torch.bfloat16 and a.is_contiguous() and a.shape[0] == T * per and w.is_contiguous() and w.shape[2] == ff
-    assert out.dtype == torch.float32 and out.is_contiguous() and tuple(out.shape) == (per, T, d)
-    assert ids.dtype == torch.int32 and ids.is_contiguous()
-    _check(_fn("moe", "odin_moe_few_down")(
-        _ptr(a), _ptr(w), _ptr(ids), _wts(wts, ids), c_int(T), c_int(per), c_int(w.shape[0]), c_int(ff), c_int(d), _ptr(out),
-        _stream()), "moe_few_down")
-
-
 def moe_places(rows: int, n_experts: int) -> int:
     """Places that `rows` rows take at most once every expert's rows are padded to whole tiles of 128."""
     return (rows + n_experts * 127 + 127) // 128 * 128

@@ -52,12 +52,6 @@ WIDE_CHUNKS_MAX_TOKENS = int(os.environ.get("ODIN_WIDE_CHUNKS_MAX_TOKENS", "1024
 # shorter than the row kernels', although it launches three kernels more; at 192 rows half as long)
 MOE_GROUPED_FROM_ROWS = int(os.environ.get("ODIN_MOE_GROUPED_FROM", "32"))
 
-# Up to this many rows (token, choice) per expert the experts' products take an expert's rows together straight from the
-# choices (see Runtime.experts).  Measured against the grouped products, both products of 32 experts of 2048 x 768 / 64 of
-# 4096 x 1024: 1 row per expert 45 against 79 us, 178 against 239; 3 rows 67 against 111, 337 against 394; 4.5 rows 382
-# against 392; 6 rows 85 against 112, 412 against 395.
-MOE_FEW_ROWS_PER_EXPERT = int(os.environ.get("ODIN_MOE_FEW_UPTO", "5"))
-
 # from this many tokens on a product per head runs on the tensor cores
 HEADS_TC_FROM = 128
 
@@ -265,15 +259,6 @@ class Runtime:
         T, per = ids.shape
         in_wts, out_wts = (wts, None) if weigh_input else (None, wts)
         inner, width = w_down.shape[2], w_down.shape[1]
-        # A decode step's rows: an expert's rows together, two kernels (with weighted inputs from where they are rounded to
-        # bfloat16 anyway).
-        if (T * per <= MOE_FEW_ROWS_PER_EXPERT * w_down.shape[0] and ops.moe_few_supported(h, w_gate_up, w_down)
-                and (in_wts is None or T * per >= MOE_GROUPED_FROM_ROWS)):
-            a = self.empty(T * per, inner)
-            ops.moe_few_up(h, w_gate_up, ids, activation, a, gated=gated, in_wts=in_wts)
-            y = self.empty(per, T, width, dtype=torch.float32)
-            ops.moe_few_down(a, w_down, ids, out_wts, y)
-            return y
         if T * per >= MOE_GROUPED_FROM_ROWS and ops.moe_grouped_supported(h, w_gate_up, w_down) and width % 4 == 0:
             # many rows: sorted by expert and multiplied tile by tile on the tensor cores (a row's weights are read
             # once per tile of 128 rows instead of once per row)

@@ -329,52 +329,6 @@ def test_attention_32bit_same_bits_in_every_kernel(geom, options):
         assert general[:3].isfinite().all()
 
 
-@pytest.mark.parametrize("T", [1, 3, 8, 9, 17, 40])
-@pytest.mark.parametrize("E,per,d,ff", [(3, 2, 8, 8), (5, 3, 72, 40), (32, 4, 264, 136), (1, 1, 1032, 520)])
-@pytest.mark.parametrize("kind,gated,weigh_input", [("silu", True, False), ("gelu_tanh", True, True), ("relu2", False, False)])
-def test_experts_of_few_rows(T, E, per, d, ff, kind, gated, weigh_input):
-    """A few rows per expert, straight from the choices: choices without an expert, an expert named twice by a token, more
-    rows of an expert than a pass takes (one expert, 40 tokens), K and widths that are no whole steps or groups.  Against
-    the same in float64; a row alone has the same bits."""
-    from odin_infer_b200.csrc import ops
-    torch.manual_seed(T * 100 + d)
-    h = torch.randn(T, d, device=DEV).bfloat16()
-    w1 = (torch.randn(E, (2 if gated else 1) * ff, d, device=DEV) / math.sqrt(d)).bfloat16()
-    w2 = (torch.randn(E, d, ff, device=DEV) / math.sqrt(ff)).bfloat16()
-    ids = torch.randint(-1, E, (T, per), device=DEV, dtype=torch.int32)
-    wts = torch.rand(T, per, device=DEV)
-
-    def run(h, ids, wts):
-        a = torch.full((ids.numel(), ff), float("nan"), device=DEV, dtype=torch.bfloat16)
-        y = torch.full((per, ids.shape[0], d), float("nan"), device=DEV)
-        torch.cuda.synchronize()
-        ops.moe_few_up(h, w1, ids, kind, a, gated=gated, in_wts=wts if weigh_input else None)
-        ops.moe_few_down(a, w2, ids, None if weigh_input else wts, y)
-        return a, y
-    a, y = run(h, ids, wts)
-    assert y.isfinite().all()
-    for t in range(T):
-        for k in range(per):
-            e = int(ids[t, k])
-            if e < 0:
-                assert (y[k, t] == 0).all()
-                continue
-            x = (h[t].float() * wts[t, k]).bfloat16().double() if weigh_input else h[t].double()
-            z = w1[e].double() @ x
-            g = z[:ff]
-            act = {"silu": lambda v: v * torch.sigmoid(v), "relu2": lambda v: v.clamp(min=0) ** 2,
-                   "gelu_tanh": lambda v: 0.5 * v * (1 + torch.tanh(math.sqrt(2 / math.pi) * (v + 0.044715 * v ** 3)))}[kind](g)
-            act = act * z[ff:] if gated else act
-            got = a[t * per + k].double()
-            # one rounding to bfloat16 of a 32-bit sum: 2^-8 of the value, and the sum's own rounding
-            assert (got - act).abs().max().item() <= 2 ** -8 * act.abs().max().item() + 1e-5
-            ref = (w2[e].double() @ got) * (1.0 if weigh_input else wts[t, k].double())
-            assert (y[k, t].double() - ref).abs().max().item() <= 1e-5 * max(1.0, ref.abs().max().item())
-    t = T // 2
-    a1, y1 = run(h[t:t + 1], ids[t:t + 1].contiguous(), wts[t:t + 1].contiguous())
-    assert torch.equal(y1[:, 0], y[:, t])
-
-
 @pytest.mark.parametrize("n_seqs", [39, 64, 128, 130])
 @pytest.mark.parametrize("window", [0, 100])
 def test_decode_attention_of_many_unequal_sequences(n_seqs, window):

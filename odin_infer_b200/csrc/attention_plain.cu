@@ -205,8 +205,8 @@ __device__ __forceinline__ float chunk_softmax(float dot, bool key, float scale,
 // softmax of the two chunks of 32, a thread per (element, head) adds the values up.
 // What bounds it: the chain of a block (hd multiply-adds of a dot product, two softmaxes one after the other, 64
 // multiply-adds of a sum, four barriers: 3.3 us for 64 keys of 128, 1.8 of 16), not the keys' traffic.  16 query heads on 8
-// kv heads of 128: sequences of 400, 287, 174 and 61 keys 24.8 us, 2,000 keys 106 us; a decode step of four such
-// sequences on the 1.7B size spent 7.2 ms of its 8 steps here, where attention_plain_kernel took a third of 158 ms.
+// kv heads of 128: sequences of 400, 287, 174 and 61 keys 24.8 us, 2,000 keys 106 us; 8 decode steps of four such
+// sequences on the 1.7B size spend 5.6 ms here.
 constexpr int SG_THREADS = 256;
 constexpr int SG_KEYS = 64;
 constexpr int SG_MAX_HD = 128;

@@ -28,8 +28,9 @@ PROMPT_BUCKETS = (16, 32, 64, 128, 192, 256, 384, 512, 768, 1024)
 PROMPT_SEQ_BUCKETS = (1, 2, 4, 8, 16)
 
 # In 32-bit only up to 256 tokens, and at most one wanted place per sequence: beyond that a step of a model that is not
-# tiny keeps the device busy for longer than its launches take (the 1.7B size: 64 rows 9 ms beside 5.8 ms of launches),
-# while the padding rows cost their share of it; up to there the buckets are multiples of the products' 64-row tiles.
+# tiny keeps the device busy for longer than its launches take (the 1.7B size: the products of 64 rows alone 9.3 ms beside
+# 5.8 ms of launches), while the padding rows cost their share of it; up to there the buckets from 64 on are multiples of the
+# products' 64-row tiles.
 PROMPT_ROWS_32BIT = 256
 
 

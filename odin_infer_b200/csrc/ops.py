@@ -505,12 +505,14 @@ def moe_gather(h: torch.Tensor, row_of_place: torch.Tensor, per: int, out: torch
 
 
 def moe_grouped(a: torch.Tensor, w: torch.Tensor, tile_expert: torch.Tensor, out: torch.Tensor, kind: str | None = None,
-                gated: bool = True) -> None:
+                gated: bool = True, row_of_place: torch.Tensor | None = None) -> None:
     """Every tile of 128 sorted rows of a [places, K] times the matrix of the tile's own expert (tcgen05).
     kind None: w [experts, N, K], out float32 [places, N] = a W[e]^T.  kind silu / gelu_tanh: w [experts, 2 N, K]
     (gate rows first), out bfloat16 [places, N] = act(a Wg[e]^T) * (a Wu[e]^T).  kind with gated=False (also relu2):
-    w [experts, N, K], out bfloat16 [places, N] = act(a W[e]^T), the activation applied as the sums are read back."""
+    w [experts, N, K], out bfloat16 [places, N] = act(a W[e]^T), the activation applied as the sums are read back.
+    row_of_place: the plan's; padding places of a tile with up to 16 rows may then be left as they are."""
     places, K = a.shape
+    assert row_of_place is None or (row_of_place.dtype == torch.int32 and row_of_place.numel() == places)
     n_e, rpe = w.shape[0], w.shape[1]
     N = out.shape[1]
     dual = kind is not None and gated
@@ -520,7 +522,7 @@ def moe_grouped(a: torch.Tensor, w: torch.Tensor, tile_expert: torch.Tensor, out
         assert tile_expert.numel() * 128 == places and rpe == N
         _check(_fn("moe_tc", "odin_moe_grouped")(
             _ptr(a), c_longlong(a.stride(0)), _ptr(w), c_longlong(K), c_int(n_e), c_int(rpe), c_int(places), c_int(N), c_int(K),
-            c_int(0), c_int(ACTIVATIONS[kind]), _ptr(tile_expert), _ptr(out), c_longlong(out.stride(0)), _stream()),
+            c_int(0), c_int(ACTIVATIONS[kind]), _ptr(tile_expert), _ptr(row_of_place), _ptr(out), c_longlong(out.stride(0)), _stream()),
             "moe_grouped")
         return
     assert a.dtype == w.dtype == torch.bfloat16 and a.is_contiguous() and w.is_contiguous() and w.shape[2] == K
@@ -528,7 +530,7 @@ def moe_grouped(a: torch.Tensor, w: torch.Tensor, tile_expert: torch.Tensor, out
     assert tile_expert.numel() * 128 == places and rpe == (2 * N if dual else N)
     _check(_fn("moe_tc", "odin_moe_grouped")(
         _ptr(a), c_longlong(a.stride(0)), _ptr(w), c_longlong(K), c_int(n_e), c_int(rpe), c_int(places), c_int(N), c_int(K),
-        c_int(1 if dual else 0), c_int(ACTIVATIONS[kind] if dual else 0), _ptr(tile_expert), _ptr(out),
+        c_int(1 if dual else 0), c_int(ACTIVATIONS[kind] if dual else 0), _ptr(tile_expert), _ptr(row_of_place), _ptr(out),
         c_longlong(out.stride(0)), _stream()), "moe_grouped")
 
 

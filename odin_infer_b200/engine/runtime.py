@@ -271,9 +271,9 @@ class Runtime:
             hs = self.empty(places, h.shape[1])
             ops.moe_gather(h, row_of_place, per, hs, in_wts)
             a = self.empty(places, inner)
-            ops.moe_grouped(hs, w_gate_up, tile_expert, a, activation, gated=gated)   # the activation rides in the epilogue
+            ops.moe_grouped(hs, w_gate_up, tile_expert, a, activation, gated=gated, row_of_place=row_of_place)   # the activation rides in the epilogue
             c = self.empty(places, width, dtype=torch.float32)
-            ops.moe_grouped(a, w_down, tile_expert, c)
+            ops.moe_grouped(a, w_down, tile_expert, c, row_of_place=row_of_place)
             y = self.empty(T, width, dtype=torch.float32)
             ops.moe_combine(c, place_of_row, out_wts, y)
             return y

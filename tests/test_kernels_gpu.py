@@ -329,6 +329,38 @@ def test_attention_32bit_same_bits_in_every_kernel(geom, options):
         assert general[:3].isfinite().all()
 
 
+@pytest.mark.parametrize("counts", [[1, 16, 17], [0, 15, 128, 129], [144, 145, 3]])
+@pytest.mark.parametrize("dual", [True, False])
+def test_grouped_products_of_tiles_with_few_rows(counts, dual):
+    """A tile of sorted rows with up to 16 of them is copied and stored by its first 16 places alone: every row's result is
+    what it is with the whole tile (around 16 rows in a tile, first tiles full and last ones not), whatever the padding
+    rows of the input hold."""
+    from odin_infer_b200.csrc import ops
+    torch.manual_seed(sum(counts))
+    E, K, N = len(counts), 136, 200
+    ids = torch.tensor([e for e, n in enumerate(counts) for _ in range(n)], dtype=torch.int32, device=DEV)[:, None].contiguous()
+    rows = ids.numel()
+    places = ops.moe_places(rows, E)
+    place_of_row = torch.empty(rows, dtype=torch.int32, device=DEV)
+    row_of_place = torch.empty(places, dtype=torch.int32, device=DEV)
+    tile_expert = torch.empty(places // 128, dtype=torch.int32, device=DEV)
+    ops.moe_plan(ids, E, place_of_row, row_of_place, tile_expert)
+    a = torch.full((places, K), float("nan"), device=DEV).bfloat16()
+    a[place_of_row.long()] = torch.randn(rows, K, device=DEV).bfloat16()
+    w = torch.randn(E, 2 * N if dual else N, K, device=DEV).bfloat16()
+    outs = []
+    for given in (None, row_of_place):
+        out = torch.full((places, N), 7.0, device=DEV, dtype=torch.bfloat16 if dual else torch.float32)
+        torch.cuda.synchronize()
+        ops.moe_grouped(a, w, tile_expert, out, "silu" if dual else None, row_of_place=given)
+        outs.append(out[place_of_row.long()])
+    assert outs[0].isfinite().all() and torch.equal(outs[0], outs[1])
+    if not dual:
+        ref = torch.einsum("rk,rnk->rn", a[place_of_row.long()].double(), w.double()[ids[:, 0].long()])
+        assert (outs[1].double() - ref).abs().max().item() <= 4e-7 * K   # a 32-bit sum of K products of unit normals
+    ops.moe_tc_check()
+
+
 @pytest.mark.parametrize("n_seqs", [39, 64, 128, 130])
 @pytest.mark.parametrize("window", [0, 100])
 def test_decode_attention_of_many_unequal_sequences(n_seqs, window):

@@ -65,10 +65,16 @@ class DecodeGraphs:
         n = sum(len(e.tokens) for e in entries)
         rows = next(b for b in PROMPT_BUCKETS if n <= b)
         seqs = next(b for b in PROMPT_SEQ_BUCKETS if len(entries) <= b)
-        key = ("prompt", rows, seqs, sum(len(e.want) for e in entries))
+        # In 32-bit a step keeps the forms that its own lengths choose, whatever the bucket and whoever shares it, so that its
+        # bits are those of the eager step; in bfloat16 the bucket's rows choose.
+        exact = self.rt.dtype == torch.float32
+        longest = max(len(e.tokens) for e in entries)
+        form = sum(longest >= n for n in self.model.forms_from) if exact else 0
+        key = ("prompt", rows, seqs, sum(len(e.want) for e in entries), form)
         hit = self._graphs.get(key)
         if hit is None:
-            batch = StepBatch(self.cache, entries, starts, self.rt.device, pad_rows_to=rows, pad_seqs_to=seqs)
+            batch = StepBatch(self.cache, entries, starts, self.rt.device, pad_rows_to=rows, pad_seqs_to=seqs,
+                              exact_forms=exact)
             return self._first_run(key, batch)
         graph, batch, logits, n_kernels = hit
         batch.fill(entries, starts)

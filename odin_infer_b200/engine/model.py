@@ -51,6 +51,11 @@ class DecoderModel:
         """May a step of this model be captured in a CUDA graph and replayed (see Part.graph_safe)?"""
         return all(p.graph_safe for p in self._all_parts())
 
+    @property
+    def forms_from(self) -> tuple[int, ...]:
+        """Every part's lines between its forms (see Part.forms_from), ascending."""
+        return tuple(sorted({n for p in self._all_parts() for n in p.forms_from}))
+
     def parts_not_graph_safe(self) -> list[str]:
         out = []
         for p in self._all_parts():

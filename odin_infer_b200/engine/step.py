@@ -42,20 +42,24 @@ class StepBatch:
     (first token row; n_seqs + 1 entries), seq_len_after[b] (its length once this step
     is done), and one block table row per cache group.  logit_rows: the token rows
     whose logits are wanted.  Host copies for parts that size their launches:
-    n_seqs, n_tokens, slots, lengths_after, seq_start_host, all_single, max_new.  carried: device
-    tensors by name that a layer hands to later layers of the same step.
+    n_seqs, n_tokens, slots, lengths_after, seq_start_host, all_single, max_new, longest_new.
+    max_new bounds what a sequence brings in any step of these buffers (it sizes launches);
+    longest_new is what a part chooses its form by (see Part.forms_from): the most tokens that a sequence
+    of this step brings, or, without exact_forms, max_new.  carried: device tensors by name that a
+    layer hands to later layers of the same step.
     """
 
     carried: dict
 
     def __init__(self, cache, entries: list[StepEntry], start_positions: list[int], device,
-                 pad_rows_to: int = 0, pad_seqs_to: int = 0, all_rows_wanted: bool = False):
+                 pad_rows_to: int = 0, pad_seqs_to: int = 0, all_rows_wanted: bool = False, exact_forms: bool = False):
         self.cache = cache
         self.device = device
         self.carried = {}
         self.n_seq_cap = max(len(entries), pad_seqs_to)
         self.n_row_cap = max(sum(len(e.tokens) for e in entries), pad_rows_to)
         self.all_rows_wanted = all_rows_wanted
+        self.exact_forms = exact_forms
         self._for_graph = pad_rows_to > 0 or pad_seqs_to > 0  # fixed buffers of a captured step
         wanted = sum(len(e.want) for e in entries)
         self.n_logit_cap = self.n_row_cap if all_rows_wanted else wanted
@@ -153,10 +157,12 @@ class StepBatch:
         la[:self.n_seqs] = self.lengths_after
         self.all_single = all(len(e.tokens) == 1 for e in entries)
         self.all_start = all(p0 == 0 for p0 in start_positions)
-        self.max_new = max((len(e.tokens) for e in entries), default=0)
+        self.max_new = self.longest_new = max((len(e.tokens) for e in entries), default=0)
         if self._for_graph and not self.all_single:
             # rows padded for a captured prompt step: the kernels' shapes must hold for any count of tokens up to the rows
             self.max_new = self.n_row_cap
+            if not self.exact_forms:
+                self.longest_new = self.max_new
         self.max_len_after = max(self.lengths_after, default=0)
         for key, g in self.cache.groups.items():
             bt = self._h(("bt", key))

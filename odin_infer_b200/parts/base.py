@@ -86,6 +86,10 @@ class Part:
     # May this part's forward be captured in a CUDA graph and replayed (see the module's text)?
     graph_safe = False
 
+    # The numbers of new tokens from which forward takes another form, one whose sums run in another order (compared with
+    # `step.longest_new`, never with `step.max_new`): a 32-bit graph replays only steps on the same side of all of them.
+    forms_from: tuple[int, ...] = ()
+
     def kernel_groups(self) -> set[str]:
         """Kernel libraries this part launches (compiled before the first step)."""
         return set()

@@ -78,6 +78,10 @@ class PreNormBlock(Block):
     def graph_safe(self):
         return all(p.graph_safe for p in self._parts())
 
+    @property
+    def forms_from(self):
+        return tuple(n for p in self._parts() for n in p.forms_from)
+
     @staticmethod
     def _norm(norm, rt, x, pending, **more):
         delta, bias = split_update(pending)

@@ -24,13 +24,13 @@ DELTA_CHUNKS_FROM = 2 * ops.DELTA_CHUNK
 
 
 def _block_len(step) -> int:
-    return RECURRENCE_BLOCK if step.max_new >= BLOCKS_FROM else 0
+    return RECURRENCE_BLOCK if step.longest_new >= BLOCKS_FROM else 0
 
 
 def _fixed_decay(step, q, k, v, decay, out, state, n_heads: int, dk: int, dv: int, silu: bool = False) -> None:
     """The recurrence with one constant decay per head: long prompts as products of tiles over blocks of tokens, shorter steps
     and every decode step token by token."""
-    if step.max_new >= BLOCKS_FROM:
+    if step.longest_new >= BLOCKS_FROM:
         ops.decay_blocks(q, k, v, decay, out, state, step.seq_start, step.seq_slots, step.n_seq_cap, n_heads, dk, dv,
                          step.max_new, silu)
     else:
@@ -60,6 +60,7 @@ class TokenShiftWKV(Mixer):
     """
 
     graph_safe = True
+    forms_from = (BLOCKS_FROM,)
     takes_residual = True
     STREAMS = ("r", "k", "v", "g", "w")
 
@@ -133,6 +134,7 @@ class Retention(Mixer):
     rotation, scaling, decay and state are 32-bit.  names: "q", "k", "v", "g", "o"."""
 
     graph_safe = True
+    forms_from = (BLOCKS_FROM,)
     rope_layouts = ("halves", "pairs")
 
     def __init__(self, width: int, n_heads: int, head_dim: int, v_head_dim: int, decay, names: dict,
@@ -199,6 +201,7 @@ class Lightning(Mixer):
     decay and state are 32-bit.  names: "q", "k", "v", "g", "norm", "o"."""
 
     graph_safe = True
+    forms_from = (BLOCKS_FROM,)
 
     def __init__(self, width: int, n_heads: int, head_dim: int, v_head_dim: int, decay, names: dict, eps: float = 1e-5):
         decay = [float(d) for d in decay]
@@ -254,6 +257,7 @@ class GatedLinearRecurrence(Mixer):
     """
 
     graph_safe = True
+    forms_from = (BLOCKS_FROM,)
     takes_residual = True
 
     def __init__(self, width: int, n_heads: int, head_dim: int, v_head_dim: int, names: dict, eps: float = 1e-5):
@@ -312,6 +316,7 @@ class GatedLinearAttention(Mixer):
     given).  names: "q", "k", "v", "g", "o", "norm", "a1", "a2", "a2_bias"."""
 
     graph_safe = True
+    forms_from = (BLOCKS_FROM,)
 
     def __init__(self, width: int, n_heads: int, head_dim: int, v_head_dim: int, tau: float, names: dict, eps: float = 1e-5,
                  decay_rank: int = 0):
@@ -380,6 +385,7 @@ class GatedDeltaRule(Mixer):
     names: "q", "k", "v", "g", "b", "a", "o", "q_conv", "k_conv", "v_conv", "A_log", "dt_bias", "norm"."""
 
     graph_safe = True
+    forms_from = (DELTA_CHUNKS_FROM,)
 
     def __init__(self, width: int, n_heads: int, n_groups: int, head_dim: int, v_head_dim: int, taps: int, names: dict,
                  eps: float = 1e-5, unit_eps: float = 1e-6):
@@ -433,7 +439,7 @@ class GatedDeltaRule(Mixer):
         ops.delta_rule(qkv[:, :qk], qkv[:, qk:2 * qk], qkv[:, 2 * qk:], a, b, self.A_log, self.dt_bias, o, S, step.seq_start,
                        step.seq_slots, step.n_seq_cap, H, self.D, self.V, heads_per_group=H // self.G,
                        q_scale=float(self.D) ** -0.5, unit_eps=self.unit_eps,
-                       chunked=step.max_new >= DELTA_CHUNKS_FROM, max_new=step.max_new)
+                       chunked=step.longest_new >= DELTA_CHUNKS_FROM, max_new=step.max_new)
         y = rt.empty(T, vv)
         ops.head_unit_scale(o, self.norm_w, False, g, self.eps, y, H, self.V)
         return rt.linear(y, self.w_o, out_dtype=torch.float32, may_split=True)

@@ -11,7 +11,7 @@ import torch
 
 from ..csrc import ops
 from .base import Biased, Combined, Mixer, ParamSpec, PartSpec, build_part, register_part
-from .recurrent import _block_len, _f32_view
+from .recurrent import BLOCKS_FROM, _block_len, _f32_view
 
 
 def _as_f32(*tensors):
@@ -29,6 +29,7 @@ class SelectiveScan(Mixer):
     then y * silu(z) through W_o.  names: "in", "conv", "conv_bias", "x", "dt", "dt_bias", "A_log", "D", "o"."""
 
     graph_safe = True
+    forms_from = (BLOCKS_FROM,)
 
     def __init__(self, width: int, inner: int, state: int, dt_rank: int, taps: int, names: dict):
         if min(width, inner, state, dt_rank, taps) < 1:
@@ -89,6 +90,7 @@ class StateSpaceDual(Mixer):
     names: "in", "conv", "conv_bias", "dt_bias", "A_log", "D", "norm", "o"."""
 
     graph_safe = True
+    forms_from = (BLOCKS_FROM,)
 
     def __init__(self, width: int, n_heads: int, head_dim: int, state: int, groups: int, norm_groups: int, taps: int,
                  names: dict, eps: float = 1e-5):
@@ -262,6 +264,10 @@ class SideBySide(Mixer):
     @property
     def graph_safe(self):
         return all(m.graph_safe for m in self._both())
+
+    @property
+    def forms_from(self):
+        return tuple(n for m in self._both() for n in m.forms_from)
 
     def params(self):
         out = [p for m in self._both() for p in m.params()]

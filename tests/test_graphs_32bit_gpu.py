@@ -1,0 +1,63 @@
+"""32-bit steps replayed as CUDA graphs: the same bits as the steps run eagerly, whatever shares the step, for every architecture;
+what a step hands out stays as it is; which steps are captured, and when."""
+import pytest
+import torch
+
+from odin_infer_b200 import Engine, Engine_Opts, StepEntry
+from odin_infer_b200.config import config_from_dict
+from tests import test_bafilorn_gpu, test_fugavik_gpu, test_meropel_gpu, test_nikonex_gpu, test_nufupel_gpu, test_tovalix_gpu, tiny
+from tests.tiny import random_tokens
+
+pytestmark = pytest.mark.gpu
+
+MODELS = {"qwen3": tiny.TINY_D, "tovalix": test_tovalix_gpu.MIXED, "nufupel": test_nufupel_gpu.MIXED, "nikonex": test_nikonex_gpu.MIXED,
+          "meropel": test_meropel_gpu.MIXED, "fugavik": test_fugavik_gpu.MIXED, "bafilorn": test_bafilorn_gpu.MIXED}
+
+
+def engine_of(name, graphs=True, max_batch=4, max_ctx=512):
+    return Engine.random(config_from_dict(MODELS[name]), 5, Engine_Opts(max_ctx=max_ctx, max_batch=max_batch, dtype="float32",
+                                                                        verbose=False, cuda_graphs=graphs))
+
+
+def prompts_of(engine, lens, seed):
+    return [random_tokens(n, engine.vocab_size, seed + i) for i, n in enumerate(lens)]
+
+
+def request(engine, prompts, steps=2):
+    """The prompts in one step, the last place of each wanted, then `steps` steps of one token; the logits of every step,
+    as the engine handed them out."""
+    slots = [engine.take_slot() for _ in prompts]
+    got = [engine.step([StepEntry(s, p, [len(p) - 1]) for s, p in zip(slots, prompts)])]
+    for i in range(steps):
+        got.append(engine.step([StepEntry(s, [7 + i], [0]) for s in slots]))
+    for s in slots:
+        engine.give_back_slot(s)
+    return got
+
+
+# Beside the lengths at which a recurrence changes its form (128 and 256 tokens) stand lengths whose buckets reach that line and
+# they do not, alone and because of what shares the step.
+@pytest.mark.parametrize("name", list(MODELS))
+def test_replayed_steps_are_the_eager_steps_bit_for_bit(name):
+    on, off = engine_of(name, True), engine_of(name, False)
+    for lens in ((200,), (130, 100), (40, 40), (20,), (3, 9, 2), (65,), (127, 2), (128,), (255,), (256,), (100, 27, 128)):
+        prompts = prompts_of(on, lens, 100)
+        want = request(off, prompts)
+        for turn in range(3):       # eagerly, captured, replayed
+            for i, (a, b) in enumerate(zip(request(on, prompts), want)):
+                assert torch.equal(a, b), (name, lens, turn, i, float((a - b).abs().max() / b.abs().max()))
+    on.destroy(), off.destroy()
+
+
+@pytest.mark.parametrize("name", list(MODELS))
+def test_a_request_has_the_same_bits_alone_and_beside_others(name):
+    """The lengths of a step lie on one side of the lines between a recurrence's forms, which the longest of them chooses."""
+    engine = engine_of(name)
+    for lens in ((120, 100) if name == "fugavik" else (130, 100), (40, 40), (20, 9), (90, 100, 30)):
+        prompts = prompts_of(engine, lens, 200)
+        alone = [request(engine, [p]) for p in prompts]
+        for turn in range(3):
+            for i, got in enumerate(request(engine, prompts)):
+                for j in range(len(prompts)):
+                    assert torch.equal(got[j:j + 1], alone[j][i]), (name, lens, turn, i, j)
+    engine.destroy()

@@ -46,6 +46,32 @@ def test_start_step_tables():
         StepBatch(m, [StepEntry(slots[0], [1], [1])], [3], "cpu")
 
 
+def test_the_form_of_a_padded_step_is_its_own_lengths_where_asked():
+    m = manager()
+    slots = [m.take_slot() for _ in range(3)]
+    def entries(lens):   # noqa: E306
+        return [StepEntry(s, [1] * n, [n - 1]) for s, n in zip(slots, lens)]
+    plain = StepBatch(m, entries([40, 40]), [0, 0], "cpu")
+    assert plain.max_new == plain.longest_new == 40
+    by_rows = StepBatch(m, entries([40, 40]), [0, 0], "cpu", pad_rows_to=128, pad_seqs_to=2)
+    assert by_rows.max_new == by_rows.longest_new == 128
+    exact = StepBatch(m, entries([40, 40]), [0, 0], "cpu", pad_rows_to=128, pad_seqs_to=2, exact_forms=True)
+    assert (exact.max_new, exact.longest_new) == (128, 40)
+    exact.fill(entries([3, 125]), [0, 0])
+    assert (exact.max_new, exact.longest_new) == (128, 125)
+
+
+def test_models_name_the_lines_between_their_forms():
+    from odin_infer_b200.config import config_from_dict, lookup_architecture
+    from odin_infer_b200.engine.model import DecoderModel
+    from tests import test_bafilorn_gpu, test_fugavik_gpu, test_meropel_gpu, test_nikonex_gpu, test_nufupel_gpu, test_tovalix_gpu, tiny
+    for raw, want in ((tiny.TINY_D, ()), (test_nufupel_gpu.MIXED, ()), (test_fugavik_gpu.MIXED, (128,)),
+                      (test_tovalix_gpu.MIXED, (256,)), (test_nikonex_gpu.MIXED, (256,)), (test_meropel_gpu.MIXED, (256,)),
+                      (test_bafilorn_gpu.MIXED, (256,))):
+        cfg = config_from_dict(raw)
+        assert DecoderModel(lookup_architecture(cfg.architecture).build_spec(cfg)).forms_from == want, cfg.architecture
+
+
 @pytest.mark.parametrize("window", [0, 128])
 def test_decode_steps_in_place_equal_tables_written_anew(window):
     m = manager(window)

@@ -165,8 +165,9 @@ struct F32Attn {
     const float *k, *v;   // one layer of the cache
     const int *tok_pos, *tok_seq, *block_table;
     const float* sink;
+    const int* seq_start;  // first token of every sequence and one past the last, or null
     size_t q_stride, out_stride;
-    int T, Hq, Hkv, hd, page_size, bt_stride, window, chunk;
+    int T, Hq, Hkv, hd, page_size, bt_stride, window, chunk, n_seqs;
     float scale, softcap;
 };
 
@@ -365,15 +366,18 @@ __global__ void __launch_bounds__(SG_THREADS) attention_f32_single_kernel(const 
 
 // ---- prompts ---------------------------------------------------------------
 // A block per (64 / G consecutive tokens, kv head): its 64 rows are (token, query head of the kv head), which share
-// every chunk of 32 keys and values (two chunks in shared memory, the next one's copies in flight).  Tokens of several
-// sequences in one tile are worked on one sequence after the other.  Per chunk: the 64 x 32 dot products, 4 x 2 a
+// every chunk of 32 keys and values (two chunks in shared memory, the next one's copies in flight).  With seq_start a
+// tile holds tokens of one sequence.  Where many bring a token or two behind long contexts, the sequences of a tile of
+// consecutive tokens would be worked on one after the other: 31 sequences with one token and 2,000 keys beside a prompt
+// of 2 take 0.66 ms so, 13.4 before and 1.4 in attention_plain_kernel; 16 sequences of 3 tokens with 300 keys 109 us,
+// 768 and 121.  Without seq_start tiles are of consecutive tokens.  Per chunk: the 64 x 32 dot products, 4 x 2 a
 // thread; the softmax, a warp per 8 rows, lane = key; the 64 x HD sums, 4 x HD / 16 a thread.  Rows of 16-byte pieces
 // are stored at piece ^ (row & 7), and a warp is 8 x 4 threads laid out as in the tiles of gemm_plain.cu.
 // No window and no chunk mask: every row's chunks then start at key 0, which is what lets rows share them and keeps the
 // bits those of attention_plain_kernel.
 // What bounds it: shared loads and multiply-adds, and on short prompts the tile that sees most keys.  16 query heads on 8
-// kv heads of 128: one prompt of 2,000 tokens 667 us (862 with the tiles in order of their tokens), four of 61 to 400
-// tokens 129 us.
+// kv heads of 128: one prompt of 2,000 tokens 690 us (862 with the tiles in order of their tokens), four of 61 to 400
+// tokens 135 us.  Prompts of up to 20 tokens take 2 us longer than in attention_plain_kernel (19 and 17).
 constexpr int TL_THREADS = 256;
 constexpr int TL_ROWS = 64;
 constexpr int TL_KEYS = 32;
@@ -406,6 +410,47 @@ __device__ __forceinline__ void add_values(const float* p, const float* v, const
     }
 }
 
+// The tokens [tok0, end) of the item-th tile: sequences from the last to the first, each in tiles of tt tokens from its
+// first token on, its last tile first.  tok0 >= end beyond the last item.
+__device__ __forceinline__ void tile_tokens(int item, int tt, const int* __restrict__ seq_start, int n_seqs, int tid, int& tok0, int& end) {
+    __shared__ int warp_sums[TL_THREADS / 32];
+    __shared__ int found[2];
+    const int lane = tid & 31, warp = tid >> 5;
+    if (tid == 0) found[0] = found[1] = 0;
+    for (int b0 = 0; b0 < n_seqs; b0 += TL_THREADS) {   // thread: a sequence
+        const int b = n_seqs - 1 - (b0 + tid);
+        int first = 0, last = 0;
+        if (b >= 0) {
+            first = seq_start[b];
+            last = seq_start[b + 1];
+        }
+        const int tiles = (last - first + tt - 1) / tt;
+        int sum = tiles;   // of this sequence and those before it in the walk
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int x = __shfl_up_sync(0xffffffffu, sum, o);
+            if (lane >= o) sum += x;
+        }
+        if (lane == 31) warp_sums[warp] = sum;
+        __syncthreads();
+        int total = 0;
+        for (int w = 0; w < TL_THREADS / 32; ++w) {
+            if (w < warp) sum += warp_sums[w];
+            total += warp_sums[w];
+        }
+        const int mine = item - (sum - tiles);   // which of this sequence's tiles, from its last
+        if (mine >= 0 && mine < tiles) {
+            found[0] = first + (tiles - 1 - mine) * tt;
+            found[1] = min(last, found[0] + tt);
+        }
+        __syncthreads();   // found; the warps' sums are written again
+        if (item < total) break;
+        item -= total;
+    }
+    tok0 = found[0];
+    end = found[1];
+}
+
 template <int HD>
 __global__ void __launch_bounds__(TL_THREADS, 2) attention_f32_tile_kernel(const F32Attn a) {
     constexpr int PIECES = HD / 4, DT = HD / 64;  // DT: groups of four elements that a thread sums
@@ -425,18 +470,26 @@ __global__ void __launch_bounds__(TL_THREADS, 2) attention_f32_tile_kernel(const
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int tx = (lane & 1) + 2 * (lane >> 4) + 4 * (warp & 3), ty = ((lane >> 1) & 7) + 8 * (warp >> 2);
     // the last tiles, whose tokens see most keys, first
-    const int G = a.Hq / a.Hkv, tt = TL_ROWS / G, kvh = blockIdx.x % a.Hkv, tok0 = (int)((gridDim.x - 1 - blockIdx.x) / a.Hkv) * tt;
+    const int G = a.Hq / a.Hkv, tt = TL_ROWS / G, kvh = blockIdx.x % a.Hkv;
+    int tok0, end;   // this tile's tokens
+    if (a.seq_start != nullptr) {
+        tile_tokens((int)(blockIdx.x / a.Hkv), tt, a.seq_start, a.n_seqs, tid, tok0, end);
+        if (tok0 >= end) return;
+    } else {
+        tok0 = (int)((gridDim.x - 1 - blockIdx.x) / a.Hkv) * tt;
+        end = min(a.T, tok0 + tt);
+    }
     const float inv_scale = sqrtf((float)HD);
 
     for (int i = tid; i < tt; i += TL_THREADS) {
-        const bool in = tok0 + i < a.T;
+        const bool in = tok0 + i < end;
         t_seq[i] = in ? a.tok_seq[tok0 + i] : -1;
         t_pos[i] = in ? a.tok_pos[tok0 + i] : -1;
     }
     // row r: token r / G, head r % G
     for (int c = tid; c < TL_ROWS * PIECES; c += TL_THREADS) {
         const int r = c / PIECES, piece = c % PIECES, tok = tok0 + r / G;
-        const bool in = r < tt * G && tok < a.T;
+        const bool in = r < tt * G && tok < end;
         cp16(qs + r * HD + ((piece ^ (r & 7)) << 2),
              in ? a.q + (size_t)tok * a.q_stride + (size_t)(kvh * G + r % G) * HD + piece * 4 : a.q, in);
     }
@@ -567,7 +620,7 @@ __global__ void __launch_bounds__(TL_THREADS, 2) attention_f32_tile_kernel(const
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         const int r = ty + 16 * i, tok = tok0 + r / G;
-        if (r >= tt * G || tok >= a.T || t_seq[r / G] < 0) continue;
+        if (r >= tt * G || tok >= end || t_seq[r / G] < 0) continue;
         const int h = kvh * G + r % G;
         float l = row_l[r], corr = 1.f;
         if (a.sink != nullptr) {
@@ -598,7 +651,10 @@ int launch_tile(const F32Attn& a, cudaStream_t s) {
     const cudaError_t e = cudaFuncSetAttribute(attention_f32_tile_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, tile_smem<HD>());
     if (e != cudaSuccess) return (int)e;
     const int tt = TL_ROWS / (a.Hq / a.Hkv);
-    odin_launch(attention_f32_tile_kernel<HD>, dim3((unsigned)((a.T + tt - 1) / tt * a.Hkv)), dim3(TL_THREADS), (size_t)tile_smem<HD>(), s, a);
+    // a sequence's last tile may be a part of one: at most one more per sequence than the tokens fill
+    const long long tiles = a.seq_start != nullptr ? (long long)a.T / tt + a.n_seqs : (a.T + tt - 1) / tt;
+    if (tiles * a.Hkv > 2147483647LL) return -1;
+    odin_launch(attention_f32_tile_kernel<HD>, dim3((unsigned)(tiles * a.Hkv)), dim3(TL_THREADS), (size_t)tile_smem<HD>(), s, a);
     return 0;
 }
 
@@ -616,11 +672,14 @@ bool aligned16(const void* p) { return ((uintptr_t)p & 15) == 0; }
 
 // q: [T, Hq*hd] with row stride q_row_stride (elements); out: [T, Hq*vd] with row stride out_row_stride.
 // single: every sequence brings at most one of the T tokens.
+// seq_start (may be null): [n_seqs + 1], sequence b's tokens being seq_start[b] .. seq_start[b + 1]; tokens of no sequence
+// (tok_seq -1) may follow the last.
 extern "C" int odin_attention_plain(const void* q, long long q_row_stride, void* out, long long out_row_stride,
                                     int dtype, int T, int Hq, int Hkv, int hd, int vd, const void* k_cache,
                                     const void* v_cache, int page_size, const int* tok_pos, const int* tok_seq,
                                     const int* block_table, int bt_stride, int window, int chunk, float scale,
-                                    float softcap, const float* sink, int single, void* stream) {
+                                    float softcap, const float* sink, int single, const int* seq_start,
+                                    int n_seqs, void* stream) {
     if (T <= 0) return 0;
     if (hd <= 0 || hd > AP_MAX_HD || vd <= 0 || vd > AP_MAX_HD || Hkv <= 0 || Hq % Hkv != 0 ||
         window < 0 || chunk < 0)
@@ -634,8 +693,8 @@ extern "C" int odin_attention_plain(const void* q, long long q_row_stride, void*
     if (dtype == ODIN_F32 && hd == vd && hd % 4 == 0 && hd <= SG_MAX_HD && group <= SG_MAX_G && q_row_stride % 4 == 0 &&
         aligned16(q) && aligned16(k_cache) && aligned16(v_cache) && page_size % SG_KEYS == 0) {
         const F32Attn a{(const float*)q, (float*)out, (const float*)k_cache, (const float*)v_cache, tok_pos, tok_seq, block_table,
-                        sink, (size_t)q_row_stride, (size_t)out_row_stride, T, Hq, Hkv, hd, page_size, bt_stride, window, chunk,
-                        scale, softcap};
+                        sink, n_seqs > 0 ? seq_start : nullptr, (size_t)q_row_stride, (size_t)out_row_stride, T, Hq, Hkv, hd,
+                        page_size, bt_stride, window, chunk, n_seqs, scale, softcap};
         int rc = -1;
         if (single) rc = launch_single(a, s);
         else if (window == 0 && chunk == 0 && hd == 128) rc = launch_tile<128>(a, s);

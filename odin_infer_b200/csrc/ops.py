@@ -1187,10 +1187,12 @@ def attention_plain(q: torch.Tensor, out: torch.Tensor, n_q: int, n_kv: int, hea
                     k_cache: torch.Tensor, v_cache: torch.Tensor, tok_pos: torch.Tensor, tok_seq: torch.Tensor,
                     block_table: torch.Tensor, window: int = 0, chunk: int = 0, scale: float = 0.0,
                     softcap: float = 0.0, v_head_dim: int | None = None, sink: torch.Tensor | None = None,
-                    single: bool = False) -> None:
+                    single: bool = False, seq_start: torch.Tensor | None = None) -> None:
     """Causal attention of each token over its sequence's cache; q may be a strided view.
     sink: float32 [n_q]; exp(sink[h]) joins the softmax's denominator of head h (no key, no value).
     single: every sequence brings one token (the kernel for decoding in 32-bit; the same bits either way).
+    seq_start: int32 [sequences + 1], the first token row of every sequence; 32-bit prompts then take a sequence's tokens
+    together (the same bits with and without it).
 
     window > 0: only the last `window` keys; chunk > 0: only the keys of the query's own chunk of
     `chunk` positions; scale > 0 replaces 1 / sqrt(head_dim); softcap > 0: scores pass through
@@ -1205,7 +1207,8 @@ def attention_plain(q: torch.Tensor, out: torch.Tensor, n_q: int, n_kv: int, hea
         _ptr(q), c_longlong(q.stride(0)), _ptr(out), c_longlong(out.stride(0)), c_int(dtype_code(q.dtype)),
         c_int(T), c_int(n_q), c_int(n_kv), c_int(head_dim), c_int(vd), _ptr(k_cache), _ptr(v_cache), c_int(PAGE),
         _ptr(tok_pos), _ptr(tok_seq), _ptr(block_table), c_int(block_table.stride(0)), c_int(window), c_int(chunk),
-        c_float(scale), c_float(softcap), _ptr(_sink(sink, n_q)), c_int(1 if single else 0), _stream()), "attention_plain")
+        c_float(scale), c_float(softcap), _ptr(_sink(sink, n_q)), c_int(1 if single else 0), _ptr(seq_start),
+        c_int(0 if seq_start is None else seq_start.numel() - 1), _stream()), "attention_plain")
 
 
 def _sink(sink: torch.Tensor | None, n_q: int) -> torch.Tensor | None:

@@ -333,4 +333,4 @@ class Runtime:
                                   step.seq_start, step.seq_len_after, block_table, window, chunk, scale, softcap, sink)
             return
         ops.attention_plain(q, out, n_q, n_kv, head_dim, k_line, v_line, step.tok_pos, step.tok_seq, block_table,
-                            window, chunk, scale, softcap, v_head_dim, sink, single=step.all_single)
+                            window, chunk, scale, softcap, v_head_dim, sink, single=step.all_single, seq_start=step.seq_start)

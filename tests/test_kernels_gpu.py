@@ -329,6 +329,59 @@ def test_attention_32bit_same_bits_in_every_kernel(geom, options):
         assert general[:3].isfinite().all()
 
 
+def steps_rows(news, contexts, n_kv, hd):
+    """Cache and tables of a 32-bit step whose sequences bring `news` tokens behind `contexts` cached ones."""
+    lengths = [c + n for c, n in zip(contexts, news)]
+    k, v, bt = paged_cache(len(news), lengths, n_kv, hd, torch.float32)
+    k.normal_(), v.normal_()
+    tok_pos = torch.cat([torch.arange(c, c + n) for c, n in zip(contexts, news)]).to(torch.int32).to(DEV)
+    tok_seq = torch.repeat_interleave(torch.arange(len(news)), torch.tensor(news)).to(torch.int32).to(DEV)
+    start = torch.tensor([0] + list(news)).cumsum(0).to(torch.int32).to(DEV)
+    return k, v, bt, tok_pos, tok_seq, start
+
+
+@pytest.mark.parametrize("geom", [(2, 1, 64), (3, 3, 128), (3, 1, 64), (8, 1, 128), (5, 1, 128)])
+@pytest.mark.parametrize("news", [[1], [64, 1, 63, 65], [0, 5, 0, 0, 200, 1, 0], [1] * 40 + [2], [2, 1, 0] * 100, [1] * 255 + [0, 3]])
+def test_attention_32bit_tiles_per_sequence(geom, news):
+    """With the sequences' first rows given, a tile of a 32-bit prompt step holds tokens of one sequence: the general kernel's
+    bits, for sequences of none to several tiles, more sequences than a block has threads, and rows of no sequence behind
+    the last, which stay as they are."""
+    from odin_infer_b200.csrc import ops
+    n_q, n_kv, hd = geom
+    torch.manual_seed(len(news) + hd)
+    k, v, bt, tok_pos, tok_seq, start = steps_rows(news, [(37 * i) % 150 for i in range(len(news))], n_kv, hd)
+    tok_pos = torch.cat([tok_pos, torch.zeros(3, dtype=torch.int32, device=DEV)])
+    tok_seq = torch.cat([tok_seq, torch.full((3,), -1, dtype=torch.int32, device=DEV)])
+    T = tok_seq.numel()
+    q = torch.randn(T, n_q * hd, device=DEV)
+    general, tiles = torch.full((T, n_q * hd), 7.0, device=DEV), torch.full((T, n_q * hd), 7.0, device=DEV)
+    ops.attention_plain(q, general, n_q, n_kv, hd, k, v, tok_pos, tok_seq, bt, window=1 << 29)   # a window is the general kernel's
+    ops.attention_plain(q, tiles, n_q, n_kv, hd, k, v, tok_pos, tok_seq, bt, seq_start=start)
+    assert torch.equal(tiles, general) and (tiles[-3:] == 7.0).all() and not (tiles[:-3] == 7.0).all(dim=1).any()
+
+
+def test_a_32bit_prompt_that_joins_a_batch_does_not_wait_for_its_sequences_one_by_one():
+    """31 sequences with a token behind 2,000 cached ones beside a prompt of two tokens: the step's attention takes no longer
+    than in the general kernel (it took nine times as long when a tile went through its sequences one after the other;
+    now well under half)."""
+    from odin_infer_b200.csrc import ops
+    n_q, n_kv, hd, news = 16, 8, 128, [1] * 31 + [2]
+    k, v, bt, tok_pos, tok_seq, start = steps_rows(news, [2000] * 31 + [0], n_kv, hd)
+    q = torch.randn(sum(news), n_q * hd, device=DEV)
+    out = torch.empty_like(q)
+    times = {}
+    for what, opt in (("tiles", {"seq_start": start}), ("general", {"window": 1 << 29})):
+        for i in range(13):
+            if i == 3:
+                a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+                a.record()
+            ops.attention_plain(q, out, n_q, n_kv, hd, k, v, tok_pos, tok_seq, bt, **opt)
+        b.record()
+        torch.cuda.synchronize()
+        times[what] = a.elapsed_time(b)
+    assert times["tiles"] < times["general"], times
+
+
 @pytest.mark.parametrize("counts", [[1, 16, 17], [0, 15, 128, 129], [144, 145, 3]])
 @pytest.mark.parametrize("dual", [True, False])
 def test_grouped_products_of_tiles_with_few_rows(counts, dual):

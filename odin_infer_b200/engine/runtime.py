@@ -124,8 +124,9 @@ class Runtime:
         return {"gemm_tc", "attention_decode", "attention_prefill"}
 
     def context_class(self, longest: int) -> int:
-        """Contexts of one class launch the same kernels (see decode_key_splits)."""
-        return context_class_of(longest)
+        """Contexts of one class launch the same kernels (see decode_key_splits); no launch of the 32-bit path depends on
+        the context, so there all are one class."""
+        return context_class_of(longest) if self.dtype == torch.bfloat16 else 0
 
     def run(self, model, batch):
         """Run one step of `model`; returns the logits at the wanted rows."""

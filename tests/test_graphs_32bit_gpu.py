@@ -61,3 +61,18 @@ def test_a_request_has_the_same_bits_alone_and_beside_others(name):
                 for j in range(len(prompts)):
                     assert torch.equal(got[j:j + 1], alone[j][i]), (name, lens, turn, i, j)
     engine.destroy()
+
+
+def graphs_of(engine):
+    keys = engine.graphs_32bit._graphs
+    return {k for k in keys if k[0] == "prompt"}, {k for k in keys if k[0] != "prompt"}
+
+
+def test_a_decode_graph_serves_every_context_length():
+    """Decoding from 500 to 530 tokens, across the border of what are two classes of contexts in bfloat16."""
+    on, off = engine_of("qwen3", True, max_ctx=640), engine_of("qwen3", False, max_ctx=640)
+    prompt = prompts_of(on, (500,), 300)
+    for a, b in zip(request(on, prompt, 30), request(off, prompt, 30)):
+        assert torch.equal(a, b)
+    assert len(graphs_of(on)[1]) == 1
+    on.destroy(), off.destroy()

@@ -43,3 +43,11 @@ def test_k_parts_fill_whole_rounds_and_never_depend_on_the_tokens():
                 assert 1 <= s <= 16 and s <= max(1, kb)
                 per = (kb + s - 1) // s
                 assert (kb + per - 1) // per == s, "an empty part"
+
+
+def test_contexts_of_the_32_bit_path_are_one_class():
+    import torch
+    from odin_infer_b200.engine.runtime import Runtime, context_class_of
+    lengths = (1, 511, 512, 513, 5000)
+    assert len({Runtime("cpu", torch.float32).context_class(n) for n in lengths}) == 1
+    assert [Runtime("cpu", torch.bfloat16).context_class(n) for n in lengths] == [context_class_of(n) for n in lengths]

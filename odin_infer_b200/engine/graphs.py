@@ -10,6 +10,10 @@ Only a model whose parts all say `graph_safe` is captured (the engine asks befor
 builds this object).  A step that finds no graph yet runs eagerly, and that run IS the
 step: the capture that follows records the same launches for later steps without
 executing them, so nothing (keys, values, a mixer's fixed-size state) is applied twice.
+
+In 32-bit the capture waits until a shape of step comes for the second time.  A capture costs as much as several
+eager steps (it waits for the device and gives the allocator's cache back), and 32-bit engines often see each shape
+once: a port of weights is checked with a few prompts of different lengths.
 """
 from __future__ import annotations
 
@@ -45,6 +49,7 @@ class DecodeGraphs:
     def __init__(self, rt, model, cache):
         self.rt, self.model, self.cache = rt, model, cache
         self._graphs: dict[tuple, tuple] = {}
+        self._seen: set[tuple] = set()   # 32-bit: keys of steps that came once and ran eagerly
         # In 32-bit, whose logits are copied out right behind a replay, the graphs share their scratch memory: they replay one
         # after the other on one stream, and nothing of a replay but its logits is read after it.
         self._pool = torch.cuda.graph_pool_handle() if rt.dtype == torch.float32 else None
@@ -60,6 +65,13 @@ class DecodeGraphs:
         return (len(entries) <= PROMPT_SEQ_BUCKETS[-1] and sum(len(e.tokens) for e in entries) <= PROMPT_BUCKETS[-1]
                 and any(e.want for e in entries))
 
+    def _not_yet(self, key) -> bool:
+        """Shall a step without a graph run eagerly and not be captured?"""
+        if self.rt.dtype != torch.float32 or key in self._seen:
+            return False
+        self._seen.add(key)
+        return True
+
     def _run_prompt(self, entries: list[StepEntry], starts: list[int]) -> torch.Tensor | None:
         """A few sequences' tokens (prompts or pieces of them) in a bucket of rows and of sequences."""
         n = sum(len(e.tokens) for e in entries)
@@ -73,6 +85,8 @@ class DecodeGraphs:
         key = ("prompt", rows, seqs, sum(len(e.want) for e in entries), form)
         hit = self._graphs.get(key)
         if hit is None:
+            if self._not_yet(key):
+                return NotImplemented
             batch = StepBatch(self.cache, entries, starts, self.rt.device, pad_rows_to=rows, pad_seqs_to=seqs,
                               exact_forms=exact)
             return self._first_run(key, batch)
@@ -108,7 +122,8 @@ class DecodeGraphs:
 
     def run(self, entries: list[StepEntry], starts: list[int], device_tokens=None) -> torch.Tensor | None:
         """Logits [wanted, vocab] of a one-token-per-sequence step (or of one sequence's short
-        prompt), or NotImplemented if the batch is larger than the largest bucket."""
+        prompt), or NotImplemented if the batch is larger than the largest bucket or a 32-bit step
+        of its shape came for the first time: such a step runs eagerly."""
         if any(len(e.tokens) > 1 for e in entries):
             return self._run_prompt(entries, starts)
         bucket = bucket_for(len(entries))
@@ -120,6 +135,8 @@ class DecodeGraphs:
         bucket = (bucket, self.rt.context_class(longest))
         hit = self._graphs.get(bucket)
         if hit is None:
+            if self._not_yet(bucket):
+                return NotImplemented
             batch = StepBatch(self.cache, entries, starts, self.rt.device, pad_rows_to=bucket[0], pad_seqs_to=bucket[0],
                               all_rows_wanted=True)
             logits = self._first_run(bucket, batch, device_tokens)
@@ -140,3 +157,4 @@ class DecodeGraphs:
 
     def clear(self) -> None:
         self._graphs.clear()
+        self._seen.clear()

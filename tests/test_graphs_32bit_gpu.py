@@ -43,7 +43,7 @@ def test_replayed_steps_are_the_eager_steps_bit_for_bit(name):
     for lens in ((200,), (130, 100), (40, 40), (20,), (3, 9, 2), (65,), (127, 2), (128,), (255,), (256,), (100, 27, 128)):
         prompts = prompts_of(on, lens, 100)
         want = request(off, prompts)
-        for turn in range(3):       # eagerly, captured, replayed
+        for turn in range(4):       # eagerly, captured, replayed twice
             for i, (a, b) in enumerate(zip(request(on, prompts), want)):
                 assert torch.equal(a, b), (name, lens, turn, i, float((a - b).abs().max() / b.abs().max()))
     on.destroy(), off.destroy()
@@ -56,7 +56,7 @@ def test_a_request_has_the_same_bits_alone_and_beside_others(name):
     for lens in ((120, 100) if name == "fugavik" else (130, 100), (40, 40), (20, 9), (90, 100, 30)):
         prompts = prompts_of(engine, lens, 200)
         alone = [request(engine, [p]) for p in prompts]
-        for turn in range(3):
+        for turn in range(4):
             for i, got in enumerate(request(engine, prompts)):
                 for j in range(len(prompts)):
                     assert torch.equal(got[j:j + 1], alone[j][i]), (name, lens, turn, i, j)
@@ -76,3 +76,18 @@ def test_a_decode_graph_serves_every_context_length():
         assert torch.equal(a, b)
     assert len(graphs_of(on)[1]) == 1
     on.destroy(), off.destroy()
+
+
+def test_a_shape_of_step_is_captured_when_it_comes_again():
+    """Prompts of lengths that come once run eagerly; the second step of a bucket is captured."""
+    engine = engine_of("qwen3")
+    for n in (10, 30, 60, 120):
+        request(engine, prompts_of(engine, (n,), n), steps=0)
+    assert graphs_of(engine) == (set(), set())
+    request(engine, prompts_of(engine, (50,), 1), steps=1)
+    prompts, decodes = graphs_of(engine)
+    assert [k[1] for k in prompts] == [64] and not decodes
+    request(engine, prompts_of(engine, (200,), 1), steps=1)
+    prompts, decodes = graphs_of(engine)
+    assert [k[1] for k in prompts] == [64] and [k[0] for k in decodes] == [1]
+    engine.destroy()

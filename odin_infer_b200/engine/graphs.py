@@ -12,8 +12,14 @@ step: the capture that follows records the same launches for later steps without
 executing them, so nothing (keys, values, a mixer's fixed-size state) is applied twice.
 
 In 32-bit the capture waits until a shape of step comes for the second time.  A capture costs as much as several
-eager steps (it waits for the device and gives the allocator's cache back), and 32-bit engines often see each shape
-once: a port of weights is checked with a few prompts of different lengths.
+eager steps, and 32-bit engines often see each shape once: a port of weights is checked with a few prompts of
+different lengths.
+
+Engines in several threads do not disturb one another's captures: each records on a stream of its own, in
+the mode in which other threads may allocate, and nothing here waits for the whole device or gives the
+allocator's cache back, as `torch.cuda.graph` does on its way in (a wait for the device ends any capture under
+way).  The same holds for what the caller's other threads do: `torch.cuda.synchronize()` in one of them
+ends a capture with an error; waiting for a stream or an event does not.
 """
 from __future__ import annotations
 
@@ -53,6 +59,7 @@ class DecodeGraphs:
         # In 32-bit, whose logits are copied out right behind a replay, the graphs share their scratch memory: they replay one
         # after the other on one stream, and nothing of a replay but its logits is read after it.
         self._pool = torch.cuda.graph_pool_handle() if rt.dtype == torch.float32 else None
+        self._stream = None              # the captures' own, made at the first of them
         self.last_h2d_bytes = 0
 
     def takes(self, entries: list[StepEntry]) -> bool:
@@ -110,15 +117,39 @@ class DecodeGraphs:
             batch.take_tokens(*device_tokens)
         logits = self.rt.run(self.model, batch)
         torch.cuda.current_stream().synchronize()
-        graph = torch.cuda.CUDAGraph()
         n0 = ops.launch_count()
-        with torch.cuda.graph(graph, pool=self._pool):
-            captured = self.rt.run(self.model, batch)
+        try:
+            graph, captured = self._capture(batch)
+        except torch.cuda.OutOfMemoryError:
+            ops.add_launches(n0 - ops.launch_count())
+            torch.cuda.empty_cache()          # the eager run's scratch memory, which the capture needs anew in its own pool
+            graph, captured = self._capture(batch)
         n_kernels = ops.launch_count() - n0
         ops.add_launches(-n_kernels)          # recorded, not launched
         self._graphs[key] = (graph, batch, captured, n_kernels)
         self.last_h2d_bytes = batch.h2d_bytes
         return logits
+
+    def _capture(self, batch: StepBatch) -> tuple:
+        if self._stream is None:
+            self._stream = torch.cuda.Stream(self.rt.device)
+        graph = torch.cuda.CUDAGraph()
+        try:
+            with torch.cuda.stream(self._stream):
+                graph.capture_begin(pool=self._pool, capture_error_mode="thread_local")
+                try:
+                    captured = self.rt.run(self.model, batch)
+                finally:
+                    graph.capture_end()
+        except Exception:
+            self._fresh_pool()
+            raise
+        return graph, captured
+
+    def _fresh_pool(self) -> None:
+        """A pool that no graph holds any more cannot be used again."""
+        if self._pool is not None and not self._graphs:
+            self._pool = torch.cuda.graph_pool_handle()
 
     def run(self, entries: list[StepEntry], starts: list[int], device_tokens=None) -> torch.Tensor | None:
         """Logits [wanted, vocab] of a one-token-per-sequence step (or of one sequence's short
@@ -158,3 +189,4 @@ class DecodeGraphs:
     def clear(self) -> None:
         self._graphs.clear()
         self._seen.clear()
+        self._fresh_pool()

@@ -1,5 +1,7 @@
 """32-bit steps replayed as CUDA graphs: the same bits as the steps run eagerly, whatever shares the step, for every architecture;
 what a step hands out stays as it is; which steps are captured, and when."""
+import threading
+
 import pytest
 import torch
 
@@ -90,4 +92,78 @@ def test_a_shape_of_step_is_captured_when_it_comes_again():
     request(engine, prompts_of(engine, (200,), 1), steps=1)
     prompts, decodes = graphs_of(engine)
     assert [k[1] for k in prompts] == [64] and [k[0] for k in decodes] == [1]
+    engine.destroy()
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+def test_engines_in_several_threads_capture_side_by_side(dtype):
+    """Three engines of the same weights, each in a thread of its own on a stream of its own, that allocate, copy and capture at
+    the same time: no step fails, and all hand out the same logits."""
+    engines = [Engine.random(config_from_dict(tiny.TINY_D), 5, Engine_Opts(max_ctx=320, max_batch=4, dtype=dtype, verbose=False))
+               for _ in range(3)]
+    torch.cuda.synchronize()
+    outs, errors = [[] for _ in engines], []
+
+    def work(k):
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                for n in (3, 20, 60, 130, 250):
+                    for batch in (1, 2, 3):
+                        prompts = [[1 + b] * max(2, n // batch) for b in range(batch)]
+                        for turn in range(3):
+                            outs[k] += [x.cpu() for x in request(engines[k], prompts)]
+                            torch.full((1 << 20,), turn, device="cuda:0")
+        except Exception as e:   # noqa: BLE001
+            errors.append(repr(e))
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(3)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors, errors
+    for o in outs[1:]:
+        assert len(o) == len(outs[0]) and all(torch.equal(a, b) for a, b in zip(o, outs[0]))
+    for e in engines:
+        e.destroy()
+
+
+def test_a_capture_that_failed_leaves_the_engine_able_to_capture(monkeypatch):
+    """The failure is made on the host, while the first capture is under way; the step raises, and the next ones are captured
+    and replayed."""
+    on, off = engine_of("qwen3", True), engine_of("qwen3", False)
+    prompt = prompts_of(on, (20,), 400)
+    want = request(off, prompt)
+    request(on, prompt, steps=0)                    # eagerly
+    run = on.rt.run
+    calls = []
+
+    def fails_while_capturing(model, batch):
+        out = run(model, batch)
+        calls.append(torch.cuda.is_current_stream_capturing())
+        if calls[-1]:
+            raise RuntimeError("made by the test")
+        return out
+    monkeypatch.setattr(on.rt, "run", fails_while_capturing)
+    slot = on.take_slot()
+    with pytest.raises(RuntimeError, match="made by the test"):
+        on.step([StepEntry(slot, prompt[0], [19])])
+    on.give_back_slot(slot)
+    assert calls == [False, True] and graphs_of(on) == (set(), set())
+    monkeypatch.setattr(on.rt, "run", run)
+    for turn in range(3):
+        for a, b in zip(request(on, prompt), want):
+            assert torch.equal(a, b)
+    assert all(graphs_of(on))
+    on.destroy(), off.destroy()
+
+
+def test_graphs_thrown_away_are_captured_anew():
+    engine = engine_of("qwen3")
+    prompt = prompts_of(engine, (20,), 400)
+    first = request(engine, prompt)
+    for turn in range(2):
+        for again in range(3):
+            assert all(torch.equal(a, b) for a, b in zip(request(engine, prompt), first))
+        assert all(graphs_of(engine))
+        engine.graphs_32bit.clear()
     engine.destroy()

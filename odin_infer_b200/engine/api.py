@@ -96,17 +96,12 @@ class Engine:
         nstate = self.cache.state_bytes_per_slot
         self.cache.state = torch.zeros(self.cache.max_slots, nstate, dtype=torch.uint8, device=self.rt.device)
         self.cache.zero_state = (lambda slot: self.cache.state[slot].zero_()) if nstate else None
-        # decode steps and short prompts replay CUDA graphs: `graphs` those of the serving precision, `graphs_32bit` the
-        # 32-bit path's (fewer prompts, logits of the caller's own)
+        # decode steps and short prompts replay CUDA graphs (in 32-bit fewer prompts, and logits of the caller's own)
         self.last_step_h2d_bytes = 0
-        self.graphs = self.graphs_32bit = None
+        self.graphs = None
         if opts.cuda_graphs:
             if self.model.graph_safe:
-                g = DecodeGraphs(self.rt, self.model, self.cache)
-                if self.rt.dtype == torch.bfloat16:
-                    self.graphs = g
-                else:
-                    self.graphs_32bit = g
+                self.graphs = DecodeGraphs(self.rt, self.model, self.cache)
             elif opts.verbose and self.rt.dtype == torch.bfloat16:
                 print("odin_infer_b200: steps run eagerly, not as CUDA graphs: these parts do not declare graph_safe: "
                       + ", ".join(self.model.parts_not_graph_safe()), file=sys.stderr, flush=True)
@@ -187,10 +182,9 @@ class Engine:
                 starts.append(self.cache.extend(e.slot, len(e.tokens)))
                 grown.append(e)
             logits = NotImplemented
-            graphs = self.graphs or self.graphs_32bit
-            if graphs is not None and graphs.takes(entries):
-                logits = graphs.run(entries, starts, device_tokens)
-                self.last_step_h2d_bytes = graphs.last_h2d_bytes
+            if self.graphs is not None and self.graphs.takes(entries):
+                logits = self.graphs.run(entries, starts, device_tokens)
+                self.last_step_h2d_bytes = self.graphs.last_h2d_bytes
             if logits is NotImplemented:
                 batch = StepBatch(self.cache, entries, starts, self.rt.device)
                 if device_tokens is not None:
@@ -236,9 +230,8 @@ class Engine:
         for g in self.cache.groups.values():
             g.k = g.v = None
         self.cache.state = None
-        for g in (self.graphs, self.graphs_32bit):
-            if g is not None:
-                g.clear()
+        if self.graphs is not None:
+            self.graphs.clear()
         self.model = None
         torch.cuda.empty_cache()
 

@@ -66,7 +66,7 @@ def test_a_request_has_the_same_bits_alone_and_beside_others(name):
 
 
 def graphs_of(engine):
-    keys = engine.graphs_32bit._graphs
+    keys = engine.graphs._graphs
     return {k for k in keys if k[0] == "prompt"}, {k for k in keys if k[0] != "prompt"}
 
 
@@ -165,5 +165,5 @@ def test_graphs_thrown_away_are_captured_anew():
         for again in range(3):
             assert all(torch.equal(a, b) for a, b in zip(request(engine, prompt), first))
         assert all(graphs_of(engine))
-        engine.graphs_32bit.clear()
+        engine.graphs.clear()
     engine.destroy()

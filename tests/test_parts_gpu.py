@@ -409,8 +409,9 @@ def toy_plain(w, cfg, tokens):
 def test_toy_architecture_registers_builds_and_steps(tmp_path, dtype, by_rows):
     """With the engine's default options.  by_rows = 0: the parts written the natural way (host
     copies of slots and row ranges, shapes that follow the data): the engine runs such a model
-    eagerly.  by_rows = 1: the same parts written to the contract of `graph_safe`: the bfloat16
-    steps are captured and replayed, also across a page border and a border of context classes."""
+    eagerly.  by_rows = 1: the same parts written to the contract of `graph_safe`: steps are captured and
+    replayed (in 32-bit one-token steps only, since these prompts want every place), also across a page border
+    and a border of context classes."""
     register_toy()
     from odin_infer_b200 import Engine, Engine_Opts
     from odin_infer_b200.config import config_from_dict
@@ -437,11 +438,12 @@ def test_toy_architecture_registers_builds_and_steps(tmp_path, dtype, by_rows):
         assert e.cache.line_of[3] == e.cache.line_of[0]     # the reading entry has no line of its own
         assert e.cache.line_of[2] != e.cache.line_of[0]     # the second run of layer 0 has
         assert e.cache.state_bytes_per_slot >= 4 * 65
-        assert (e.graphs is not None) == (bool(by_rows) and dtype == "bfloat16")
+        assert (e.graphs is not None) == bool(by_rows)
         got = traces.collect(recs, replay(e, recs))
         e.cache.check()
         if e.graphs is not None:
-            assert len(e.graphs._graphs) >= (1 if what == "whole" else 2), "steps were captured and replayed"
+            fewest = {"bfloat16": 1 if what == "whole" else 2, "float32": 0 if what == "whole" else 1}[dtype]
+            assert len(e.graphs._graphs) >= fewest, "steps were captured and replayed"
         for rid, ref in refs.items():
             for pos in range(ref.shape[0]):
                 if leads[rid][pos] <= 0.05:  # a near tie between experts: rounding may decide it the other way

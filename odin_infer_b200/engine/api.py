@@ -102,7 +102,7 @@ class Engine:
         if opts.cuda_graphs:
             if self.model.graph_safe:
                 self.graphs = DecodeGraphs(self.rt, self.model, self.cache)
-            elif opts.verbose and self.rt.dtype == torch.bfloat16:
+            elif opts.verbose:
                 print("odin_infer_b200: steps run eagerly, not as CUDA graphs: these parts do not declare graph_safe: "
                       + ", ".join(self.model.parts_not_graph_safe()), file=sys.stderr, flush=True)
         self.notes = self.model.notes(self.rt)

@@ -451,3 +451,15 @@ def test_toy_architecture_registers_builds_and_steps(tmp_path, dtype, by_rows):
                 err = tiny.rel_err(got[rid][pos], ref[pos])
                 assert err <= tol, f"toy {what} {dtype} by_rows={by_rows}: request {rid} first differs at position {pos}: {err:.3e}"
         e.destroy()
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+def test_the_engine_names_the_parts_that_keep_it_from_graphs(capsys, dtype):
+    """At load, in both precisions; a model of capturable parts says nothing of the kind."""
+    register_toy()
+    from odin_infer_b200 import Engine, Engine_Opts
+    from odin_infer_b200.config import config_from_dict
+    for by_rows in (0, 1):
+        e = Engine.random(config_from_dict(dict(TOY, by_rows=by_rows)), 3, Engine_Opts(max_ctx=128, max_batch=1, dtype=dtype))
+        assert ("do not declare graph_safe" in capsys.readouterr().err) == (by_rows == 0)
+        e.destroy()

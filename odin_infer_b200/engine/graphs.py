@@ -67,7 +67,7 @@ class DecodeGraphs:
         if all(len(e.tokens) == 1 for e in entries):
             return True
         if self.rt.dtype == torch.float32 and (sum(len(e.tokens) for e in entries) > PROMPT_ROWS_32BIT
-                                               or sum(len(e.want) for e in entries) > len(entries)):
+                                               or any(len(e.want) > 1 for e in entries)):
             return False
         return (len(entries) <= PROMPT_SEQ_BUCKETS[-1] and sum(len(e.tokens) for e in entries) <= PROMPT_BUCKETS[-1]
                 and any(e.want for e in entries))

@@ -167,3 +167,17 @@ def test_graphs_thrown_away_are_captured_anew():
         assert all(graphs_of(engine))
         engine.graphs.clear()
     engine.destroy()
+
+
+def test_steps_that_want_several_places_of_a_sequence_run_eagerly():
+    """Also where another sequence of the step wants none."""
+    engine = engine_of("qwen3")
+    for wants in (([3, 9], []), ([9], [0, 11])):
+        for turn in range(3):
+            slots = [engine.take_slot() for _ in wants]
+            logits = engine.step([StepEntry(s, list(range(1, 13)), w) for s, w in zip(slots, wants)])
+            assert len(logits) == sum(map(len, wants))
+            for s in slots:
+                engine.give_back_slot(s)
+    assert not graphs_of(engine)[0]
+    engine.destroy()

@@ -33,7 +33,10 @@ BUCKETS = (1, 2, 4, 8, 12, 16, 24, 32, 48, 64, 96, 128, 192, 256)
 # Short prompts are launch-bound too when they run eagerly (a few hundred launches of ~25 us of host
 # time each: 8 ms for what the device does in 3): steps of a few sequences with up to 1,024 tokens in
 # all are captured as well, per bucket of their token count and of their number of sequences, padded
-# with rows of sequence -1 and with empty sequences.
+# with rows of sequence -1 and with empty sequences.  16 rows: the products then take tiles of 16 tokens and cut K
+# otherwise than at 32, so bfloat16 logits of prompts of up to 16 tokens differ from those of a bucket of 32 by rounding.  9
+# tokens on the 1.7B size: 1.31 ms (1.57 padded to 32), on the 8B size 3.19 (3.54), on eight layers of recurrences 0.76 (1.07),
+# on eight with experts 1.05 (1.03).
 PROMPT_BUCKETS = (16, 32, 64, 128, 192, 256, 384, 512, 768, 1024)
 PROMPT_SEQ_BUCKETS = (1, 2, 4, 8, 16)
 

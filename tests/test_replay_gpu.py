@@ -184,6 +184,31 @@ def test_short_prompts_replayed_as_graphs(folders):
         assert (a - b).abs().max().item() <= 2e-2 * b.abs().max().item()
 
 
+def test_prompts_of_up_to_sixteen_tokens_have_a_bucket_of_their_own(folders):
+    """bfloat16 prompt steps around the smallest bucket's edge, alone, beside others and as a piece that goes on: the eager
+    step's logits beyond rounding, and 16 rows captured."""
+    from odin_infer_b200 import Engine, Engine_Opts, StepEntry
+    raw, _ = tiny.TINIES["D"]
+    out = {}
+    for graphs in (False, True):
+        e = Engine.load(folders["D"], Engine_Opts(max_ctx=256, max_batch=4, dtype="bfloat16", verbose=False, cuda_graphs=graphs))
+        rows = []
+        for i, lens in enumerate(((2,), (15,), (16,), (17,), (5, 11), (6, 11), (2, 2, 2, 2), (9, 1, 3))):
+            for turn in range(2):
+                slots = [e.take_slot() for _ in lens]
+                toks = [tiny.random_tokens(n + 7, raw["vocab_size"], 900 + 10 * i + j) for j, n in enumerate(lens)]
+                rows.append(e.step([StepEntry(s, t[:n], [n - 1]) for s, t, n in zip(slots, toks, lens)]).float().cpu())
+                rows.append(e.step([StepEntry(slots[0], toks[0][lens[0]:], [6])]).float().cpu())
+                for s in slots:
+                    e.give_back_slot(s)
+        if graphs:
+            assert {k[1] for k in e.graphs._graphs if k[0] == "prompt"} == {16, 32}
+        e.destroy()
+        out[graphs] = rows
+    for a, b in zip(out[True], out[False]):
+        assert a.shape == b.shape and (a - b).abs().max().item() <= 2e-2 * b.abs().max().item()
+
+
 def test_trace_run_program(folders, requests_and_refs, tmp_path):
     """The program itself: JSON lines in, .f32 files and `done` lines out."""
     reqs, refs = requests_and_refs["A"]

@@ -672,7 +672,9 @@ int launch2(const CUtensorMap& ma, const CUtensorMap& mw, Params2 p, cudaStream_
     CUtensorMap mc;
     // Row tiles of a band: enough that the weights pass by seldom, few enough that the band's tokens stay in L2 beside
     // them.  12001 x 24576 x 4096 with the SwiGLU: 1,861, 1,774 and 1,742 us with 4, 8 and 16; 12001 x 4096 x 12288 added
-    // to C: 981, 976, 997; 66048 x 2048 x 6144: 1,350, 1,364, 1,410.
+    // to C: 981, 976, 997; 66048 x 2048 x 6144: 1,350, 1,364, 1,410.  The line by K is drawn between the measured 4,096 and
+    // 6,144, and 1 to 4 % lie on either side of it: a band of 16 tiles holds 32 MB of tokens at K = 4,096 (8 tiles: 48 MB at
+    // 12,288), which need not be the best on a K or a number of column tiles that were not measured.
     p.band = p.K <= 4096 ? 16 : 8;
     if (make_map_c(&mc, p.out, std::is_same<TO, float>::value ? ODIN_F32 : ODIN_BF16, p.M, p.N, p.ldc))
         return launch2_as<TO, DUAL, false, true>(ma, mw, mc, p, s);
@@ -684,7 +686,10 @@ int launch2(const CUtensorMap& ma, const CUtensorMap& mw, Params2 p, cudaStream_
 // C[M, N] = A[M, K] W[N, K]^T on pairs of SMs (tiles of 256 x 256); for many tokens.  A: bfloat16, row
 // stride lda; W: bfloat16, row stride ldw; C of c_dtype (bfloat16 or float32), row stride ldc.
 // Strides and K multiples of 8 elements, pointers 16-byte aligned, else ODIN_ERR_UNSUPPORTED.
-// accumulate (float32 C only): C += A W^T, each element read once and written once by the thread that holds its sum.
+// accumulate (float32 C only): C += A W^T.  Each element is read once and written once, by the cluster that forms its tile: in
+// boxes of 32 rows x 128 bytes through shared memory, read up to three boxes ahead of the one at work and so before the
+// products of the next tile are there (see TMA_C), or, where TMA cannot write C, by the thread that holds its sum.  Nothing
+// else may write C while the kernel runs.
 // act (bfloat16 C only): 1 = C is max(z, 0)^2 of the product, formed as the sums are read back.
 extern "C" int odin_gemm_tc2(const void* A, const void* W, void* C, int c_dtype, int M, int N, int K, long long lda,
                              long long ldw, long long ldc, int accumulate, int act, void* stream) {

@@ -19,6 +19,7 @@
 // elements (keys and queries hd).  sink (optional, one 32-bit number per query head): exp(sink[h]) is
 // added to the softmax's denominator once.
 #include "common.cuh"
+#include "async_copy.cuh"
 #include <math_constants.h>
 
 #define AP_WARPS 4
@@ -170,15 +171,6 @@ struct F32Attn {
     int T, Hq, Hkv, hd, page_size, bt_stride, window, chunk, n_seqs;
     float scale, softcap;
 };
-
-__device__ __forceinline__ void cp16(float* dst, const float* src, bool inside) {
-    const int n = inside ? 16 : 0;  // 0: zeros, nothing is read
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(n)
-                 : "memory");
-}
-__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
 // One chunk of 32 keys of one row, lane = key, as attention_plain_kernel does it: s is the dot product (-inf where there
 // is no key), m and l the row's running maximum and sum.  Returns p; corr is the factor on what was summed before.
@@ -665,8 +657,6 @@ int launch_single(const F32Attn& a, cudaStream_t s) {
     odin_launch(attention_f32_single_kernel, dim3((unsigned)(a.T * a.Hkv)), dim3(SG_THREADS), (size_t)(4 * SG_KEYS * (a.hd + 4) * 4), s, a);
     return 0;
 }
-
-bool aligned16(const void* p) { return ((uintptr_t)p & 15) == 0; }
 
 }  // namespace
 

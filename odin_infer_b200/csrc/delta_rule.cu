@@ -26,6 +26,7 @@
 // Everything is 32-bit.  The walk's multiply-adds run two channels at a time (fma.rn.f32x2: each half rounds as a single
 // fma does).
 #include "recurrence_blocks.cuh"
+#include "async_copy.cuh"
 
 typedef unsigned long long f32x2;   // two 32-bit floats of neighbouring channels, the first in the low half
 
@@ -253,13 +254,10 @@ struct DeltaChunks {
 __device__ __forceinline__ void cp_async16(float* smem, const float* gmem) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(smem)), "l"(gmem) : "memory");
 }
-__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 // n floats (a multiple of 4) by all threads of the CTA
 __device__ __forceinline__ void cp_run(float* smem, const float* gmem, int n) {
     for (int e = threadIdx.x * 4; e < n; e += blockDim.x * 4) cp_async16(smem + e, gmem + e);
 }
-template <int N>
-__device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
 // (1) grid (items, H).  Shared memory: K and Q [64][dkp + 4] (Q's place later holds solved rows), A transposed [64][68],
 // numbers per token.

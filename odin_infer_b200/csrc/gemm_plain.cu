@@ -8,6 +8,7 @@
 // It restates the reference's row-times-vector product (infer/matmul.odin:63-70)
 // for many rows of A at once.
 #include "common.cuh"
+#include "async_copy.cuh"
 
 #define TM 64
 #define TN 64
@@ -71,15 +72,6 @@ __global__ void __launch_bounds__(256) gemm_plain_kernel(const TA* __restrict__ 
 // 32-bit operands whose rows are whole 16-byte vectors
 // ---------------------------------------------------------------------------
 namespace {
-
-__device__ __forceinline__ void cp16(float* dst, const float* src, bool inside) {
-    const int n = inside ? 16 : 0;  // 0: the destination is filled with zeros, nothing is read
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(n)
-                 : "memory");
-}
-__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
 // ---- few rows of A ---------------------------------------------------------
 // A block owns 32 weight rows and walks the whole of K; lane = weight row, the four warps share the rows of A
@@ -343,8 +335,6 @@ int launch_tiles(const float* A, const float* W, float* C, int M, int N, int K, 
     if (189.0 * rounds_large < 106.0 * rounds_small) return launch_tile<8, 8, 16, 8, 3, 2>(A, W, C, M, N, K, lda, ldw, ldc, s);
     return launch_tile<4, 4, 8, 16, 4, 4>(A, W, C, M, N, K, lda, ldw, ldc, s);
 }
-
-bool aligned16(const void* p) { return ((uintptr_t)p & 15) == 0; }
 
 }  // namespace
 

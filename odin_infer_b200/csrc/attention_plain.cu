@@ -463,7 +463,8 @@ __global__ void __launch_bounds__(TL_THREADS, 2) attention_f32_tile_kernel(const
     const int tx = (lane & 1) + 2 * (lane >> 4) + 4 * (warp & 3), ty = ((lane >> 1) & 7) + 8 * (warp >> 2);
     // the last tiles, whose tokens see most keys, first
     const int G = a.Hq / a.Hkv, tt = TL_ROWS / G, kvh = blockIdx.x % a.Hkv;
-    int tok0, end;   // this tile's tokens
+    __shared__ int first_token;   // kept here to the end, not in a register
+    int tok0, end;                // this tile's tokens
     if (a.seq_start != nullptr) {
         tile_tokens((int)(blockIdx.x / a.Hkv), tt, a.seq_start, a.n_seqs, tid, tok0, end);
         if (tok0 >= end) return;
@@ -471,6 +472,7 @@ __global__ void __launch_bounds__(TL_THREADS, 2) attention_f32_tile_kernel(const
         tok0 = (int)((gridDim.x - 1 - blockIdx.x) / a.Hkv) * tt;
         end = min(a.T, tok0 + tt);
     }
+    if (tid == 0) first_token = tok0;
     const float inv_scale = sqrtf((float)HD);
 
     for (int i = tid; i < tt; i += TL_THREADS) {
@@ -611,8 +613,8 @@ __global__ void __launch_bounds__(TL_THREADS, 2) attention_f32_tile_kernel(const
     cp_wait<0>();
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-        const int r = ty + 16 * i, tok = tok0 + r / G;
-        if (r >= tt * G || tok >= end || t_seq[r / G] < 0) continue;
+        const int r = ty + 16 * i, tok = first_token + r / G;
+        if (r >= tt * G || t_seq[r / G] < 0) continue;   // beyond the tile's last token as well
         const int h = kvh * G + r % G;
         float l = row_l[r], corr = 1.f;
         if (a.sink != nullptr) {
@@ -643,8 +645,9 @@ int launch_tile(const F32Attn& a, cudaStream_t s) {
     const cudaError_t e = cudaFuncSetAttribute(attention_f32_tile_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, tile_smem<HD>());
     if (e != cudaSuccess) return (int)e;
     const int tt = TL_ROWS / (a.Hq / a.Hkv);
-    // a sequence's last tile may be a part of one: at most one more per sequence than the tokens fill
-    const long long tiles = a.seq_start != nullptr ? (long long)a.T / tt + a.n_seqs : (a.T + tt - 1) / tt;
+    // a sequence of n tokens has (n - 1) / tt + 1 tiles: the most that n_seqs sequences of T tokens in all can have
+    const int seqs = min(a.T, a.n_seqs);
+    const long long tiles = a.seq_start != nullptr ? (long long)(a.T - seqs) / tt + seqs : (a.T + tt - 1) / tt;
     if (tiles * a.Hkv > 2147483647LL) return -1;
     odin_launch(attention_f32_tile_kernel<HD>, dim3((unsigned)(tiles * a.Hkv)), dim3(TL_THREADS), (size_t)tile_smem<HD>(), s, a);
     return 0;
@@ -683,7 +686,7 @@ extern "C" int odin_attention_plain(const void* q, long long q_row_stride, void*
     if (dtype == ODIN_F32 && hd == vd && hd % 4 == 0 && hd <= SG_MAX_HD && group <= SG_MAX_G && q_row_stride % 4 == 0 &&
         aligned16(q) && aligned16(k_cache) && aligned16(v_cache) && page_size % SG_KEYS == 0) {
         const F32Attn a{(const float*)q, (float*)out, (const float*)k_cache, (const float*)v_cache, tok_pos, tok_seq, block_table,
-                        sink, n_seqs > 0 ? seq_start : nullptr, (size_t)q_row_stride, (size_t)out_row_stride, T, Hq, Hkv, hd,
+                        sink, n_seqs > 1 ? seq_start : nullptr, (size_t)q_row_stride, (size_t)out_row_stride, T, Hq, Hkv, hd,
                         page_size, bt_stride, window, chunk, n_seqs, scale, softcap};
         int rc = -1;
         if (single) rc = launch_single(a, s);

@@ -368,8 +368,8 @@ __global__ void __launch_bounds__(SG_THREADS) attention_f32_single_kernel(const 
 // No window and no chunk mask: every row's chunks then start at key 0, which is what lets rows share them and keeps the
 // bits those of attention_plain_kernel.
 // What bounds it: shared loads and multiply-adds, and on short prompts the tile that sees most keys.  16 query heads on 8
-// kv heads of 128: one prompt of 2,000 tokens 690 us (862 with the tiles in order of their tokens), four of 61 to 400
-// tokens 135 us.  Prompts of up to 20 tokens take 2 us longer than in attention_plain_kernel (19 and 17).
+// kv heads of 128: one prompt of 2,000 tokens 693 us (862 with the tiles in order of their tokens), four of 61 to 400
+// tokens 138 us (145 with tiles of consecutive tokens).
 constexpr int TL_THREADS = 256;
 constexpr int TL_ROWS = 64;
 constexpr int TL_KEYS = 32;

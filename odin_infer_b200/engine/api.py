@@ -34,7 +34,8 @@ class Engine_Opts:
     that live sequences hold together, each rounded up to a page of 64; it sizes the
     cache (0: max_batch sequences of max_ctx).  dtype: "bfloat16" (the kernels and
     precisions of serving) or "float32" (everything in true 32-bit).  cuda_graphs: replay
-    captured graphs for one-token-per-sequence steps and short prompts.  run_ahead: generation
+    captured graphs for one-token-per-sequence steps and short prompts (while a step is captured - in bfloat16 the
+    first of its shape, in 32-bit the second - no other thread may wait for the whole device).  run_ahead: generation
     launches a decode step before the host has read the tokens it continues from."""
     max_ctx: int = DEFAULT_MAX_CONTEXT
     max_tokens: int = 0

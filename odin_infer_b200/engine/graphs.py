@@ -58,6 +58,10 @@ class DecodeGraphs:
     def __init__(self, rt, model, cache):
         self.rt, self.model, self.cache = rt, model, cache
         self._graphs: dict[tuple, tuple] = {}
+        # In 32-bit a step keeps the forms that its own lengths choose, whatever the bucket and whoever shares it, so that its
+        # bits are those of the eager step; in bfloat16 the bucket's rows choose.
+        self._exact_forms = rt.dtype == torch.float32
+        self._forms_from = model.forms_from if self._exact_forms else ()
         self._seen: set[tuple] = set()   # 32-bit: keys of steps that came once and ran eagerly
         # In 32-bit, whose logits are copied out right behind a replay, the graphs share their scratch memory: they replay one
         # after the other on one stream, and nothing of a replay but its logits is read after it.
@@ -87,18 +91,17 @@ class DecodeGraphs:
         n = sum(len(e.tokens) for e in entries)
         rows = next(b for b in PROMPT_BUCKETS if n <= b)
         seqs = next(b for b in PROMPT_SEQ_BUCKETS if len(entries) <= b)
-        # In 32-bit a step keeps the forms that its own lengths choose, whatever the bucket and whoever shares it, so that its
-        # bits are those of the eager step; in bfloat16 the bucket's rows choose.
-        exact = self.rt.dtype == torch.float32
-        longest = max(len(e.tokens) for e in entries)
-        form = sum(longest >= n for n in self.model.forms_from) if exact else 0
+        form = 0   # on which side of the lines between the parts' forms
+        if self._forms_from:
+            longest = max(len(e.tokens) for e in entries)
+            form = sum(longest >= line for line in self._forms_from)
         key = ("prompt", rows, seqs, sum(len(e.want) for e in entries), form)
         hit = self._graphs.get(key)
         if hit is None:
             if self._not_yet(key):
                 return NotImplemented
             batch = StepBatch(self.cache, entries, starts, self.rt.device, pad_rows_to=rows, pad_seqs_to=seqs,
-                              exact_forms=exact)
+                              exact_forms=self._exact_forms)
             return self._first_run(key, batch)
         graph, batch, logits, n_kernels = hit
         batch.fill(entries, starts)

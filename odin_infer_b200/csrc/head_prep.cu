@@ -344,6 +344,137 @@ head_prep_token_kernel(const TI* qkv, int n_split, size_t split_stride, bf16* q_
     }
 }
 
+// The same for heads of 128 in a bfloat16 projection of one part: eight lanes hold a head, lane l the elements [8 l, 8 l + 8)
+// and [64 + 8 l, 64 + 8 l + 8), so that an element and its rotation partner lie in one lane, a head costs two 16-byte loads
+// and two stores a lane, and its sum of squares six exchanges for four heads instead of twenty (and none for the rotation).
+// With a warp per head the instructions bound the kernel; here it is the memory.  A warp takes a token's heads four at a
+// time, CH fours in flight; `parts` warps share a token where tokens are few.  The sum of squares is added in the same tree
+// as there (sums of four neighbours; those 64 elements apart, then 32, 16, 8, 4), so the bits are the same.
+template <int CH>
+__global__ void __launch_bounds__(HP_WARPS * 32)
+head_prep_wide_kernel(const bf16* qkv, bf16* q_out, size_t q_out_stride, int T, int Hq, int Hkv, size_t row_stride, VecRef qw,
+                      VecRef kw, int has_norm, float eps, const float* __restrict__ cos_t, const float* __restrict__ sin_t,
+                      int table_len, const int* __restrict__ tok_pos, const int* __restrict__ tok_seq,
+                      const int* __restrict__ block_table, int bt_stride, bf16* __restrict__ k_cache, bf16* __restrict__ v_cache,
+                      int page_size, int write_kv, VMix<bf16> vmix, int parts) {
+    constexpr int HD = 128;
+    __shared__ __align__(16) float w_s[2][HD];   // the norms' weights, q's and k's
+    pdl_trigger();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, sub = lane >> 3, l8 = (lane & 7) * 8;
+    const int item = blockIdx.x * HP_WARPS + warp, t = item / parts, part = item - t * parts;
+    if (has_norm) {
+        w_s[0][threadIdx.x] = qw.at(threadIdx.x);
+        w_s[1][threadIdx.x] = kw.at(threadIdx.x);
+    }
+    const int seq = t < T ? tok_seq[t] : -1;
+    const int pos = t < T ? tok_pos[t] : 0;
+    pdl_wait();
+    __syncthreads();
+    if (seq < 0) return;
+    const int n_heads = Hq + 2 * Hkv;
+    const bf16* row = qkv + (size_t)t * row_stride + l8;
+    uint4 lo[CH], hi[CH];
+    auto load = [&](int h0) {
+#pragma unroll
+        for (int u = 0; u < CH; ++u) {
+            const int head = h0 + 4 * u + sub;
+            lo[u] = hi[u] = make_uint4(0, 0, 0, 0);
+            if (head < n_heads && (head < Hq || write_kv)) {
+                lo[u] = *reinterpret_cast<const uint4*>(row + (size_t)head * HD);
+                hi[u] = *reinterpret_cast<const uint4*>(row + (size_t)head * HD + HD / 2);
+            }
+        }
+    };
+    load(part * 4 * CH);   // ahead of the loads that hang on the token's position
+    const int page = write_kv ? block_table[(size_t)seq * bt_stride + pos / page_size] : -1;
+    const bool in_table = (pos >= 0 && pos < table_len);
+    float c[8], sn[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) { c[e] = 1.f; sn[e] = 0.f; }
+    if (in_table) {
+#pragma unroll
+        for (int e = 0; e < 8; e += 4) {
+            *reinterpret_cast<float4*>(c + e) = *reinterpret_cast<const float4*>(cos_t + (size_t)pos * (HD / 2) + l8 + e);
+            *reinterpret_cast<float4*>(sn + e) = *reinterpret_cast<const float4*>(sin_t + (size_t)pos * (HD / 2) + l8 + e);
+        }
+    }
+    const size_t cache_at = ((size_t)max(page, 0) * Hkv * page_size + pos % page_size) * HD + l8;   // of kv head 0
+    for (int h0 = part * 4 * CH; h0 < n_heads; h0 += parts * 4 * CH) {
+        if (h0 != part * 4 * CH) load(h0);
+#pragma unroll
+        for (int u = 0; u < CH; ++u) {
+            const int head = h0 + 4 * u + sub;
+            const bool is_q = head < Hq, is_v = head >= Hq + Hkv;
+            const int kvh = head - Hq - (is_v ? Hkv : 0);
+            bf16* dst = is_q ? q_out + (size_t)t * q_out_stride + (size_t)head * HD + l8
+                             : (is_v ? v_cache : k_cache) + cache_at + (size_t)kvh * page_size * HD;
+            const bool store = head < n_heads && (is_q || page >= 0);
+            float x[8], y[8];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const float2 f = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162*>(&lo[u])[e]);
+                const float2 g = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162*>(&hi[u])[e]);
+                x[2 * e] = f.x; x[2 * e + 1] = f.y;
+                y[2 * e] = g.x; y[2 * e + 1] = g.y;
+            }
+            if (!__all_sync(0xffffffffu, is_v)) {
+                float rx[8], ry[8];
+#pragma unroll
+                for (int e = 0; e < 8; ++e) { rx[e] = x[e]; ry[e] = y[e]; }
+                if (has_norm) {
+                    float p[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) { p[0] += x[e] * x[e]; p[1] += x[4 + e] * x[4 + e]; p[2] += y[e] * y[e]; p[3] += y[4 + e] * y[4 + e]; }
+                    float a = p[0] + p[2], b = p[1] + p[3];
+#pragma unroll
+                    for (int o = 4; o > 0; o >>= 1) {
+                        a += __shfl_xor_sync(0xffffffffu, a, o);
+                        b += __shfl_xor_sync(0xffffffffu, b, o);
+                    }
+                    float ss = a + b;
+                    ss /= (float)HD;
+                    ss += eps;
+                    const float r = 1.0f / sqrtf(ss);
+                    const float* wn = w_s[is_q ? 0 : 1] + l8;
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) { rx[e] = wn[e] * (r * x[e]); ry[e] = wn[HD / 2 + e] * (r * y[e]); }
+                }
+                if (!is_v) {
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) {
+                        x[e] = in_table ? rx[e] * c[e] - ry[e] * sn[e] : rx[e];
+                        y[e] = in_table ? rx[e] * sn[e] + ry[e] * c[e] : ry[e];
+                    }
+                }
+            }
+            if (is_v && store && (vmix.keep != nullptr || vmix.first != nullptr)) {
+                const size_t at = ((size_t)t * Hkv + kvh) * HD + l8;
+                if (vmix.keep != nullptr) {
+                    *reinterpret_cast<uint4*>(vmix.keep + at) = lo[u];
+                    *reinterpret_cast<uint4*>(vmix.keep + at + HD / 2) = hi[u];
+                }
+                if (vmix.first != nullptr) {
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) {
+                        x[e] = (1.0f - vmix.lambda) * x[e] + vmix.lambda * __bfloat162float(vmix.first[at + e]);
+                        y[e] = (1.0f - vmix.lambda) * y[e] + vmix.lambda * __bfloat162float(vmix.first[at + HD / 2 + e]);
+                    }
+                }
+            }
+            if (store) {
+                uint4 ox, oy;
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    reinterpret_cast<__nv_bfloat162*>(&ox)[e] = __floats2bfloat162_rn(x[2 * e], x[2 * e + 1]);
+                    reinterpret_cast<__nv_bfloat162*>(&oy)[e] = __floats2bfloat162_rn(y[2 * e], y[2 * e + 1]);
+                }
+                *reinterpret_cast<uint4*>(dst) = ox;
+                *reinterpret_cast<uint4*>(dst + HD / 2) = oy;
+            }
+        }
+    }
+}
+
 // qkv: [n_split][T, (Hq + 2 Hkv) hd] of in_dtype (row stride row_stride, parts split_stride
 // elements apart).  q_out: [T, Hq hd] of dtype (row stride q_out_stride); it may be qkv
 // itself when there is one part of the same type (q is then normalised and rotated in place).
@@ -376,6 +507,21 @@ extern "C" int odin_head_prep(const void* qkv, int in_dtype, int n_split, long l
         ((((uintptr_t)qkv) | ((uintptr_t)q_out) | ((uintptr_t)cos_t) | ((uintptr_t)sin_t) | ((uintptr_t)v_first) |
           ((uintptr_t)v_keep)) & 15) == 0) {
         const VMix<bf16> vmix{(const bf16*)v_first, (bf16*)v_keep, v_lambda};
+        // Prompts: a warp per head spends more instructions than the memory asks for (66,048 tokens of 16 + 2 x 8 heads: see
+        // head_prep_wide_kernel).  From 2,048 tokens on one warp takes a whole token and its angles are fetched once; below,
+        // its heads are shared out so that there are warps enough.
+        if (hd == 128 && in_dtype == ODIN_BF16 && n_split == 1 && T >= 256 && row_stride % 8 == 0 && q_out_stride % 8 == 0) {
+            constexpr int CH = 4;
+            const int chunks = ((n_heads + 3) / 4 + CH - 1) / CH, parts = T >= 2048 ? 1 : chunks;
+            const long long items = (long long)T * parts;
+            if (items > 0x7fffffffLL - HP_WARPS) return ODIN_ERR_UNSUPPORTED;
+            odin_launch(head_prep_wide_kernel<CH>, dim3((unsigned)((items + HP_WARPS - 1) / HP_WARPS)), dim3(HP_WARPS * 32), 0, s,
+                        (const bf16*)qkv, (bf16*)q_out, (size_t)q_out_stride, T, Hq, Hkv, (size_t)row_stride, qw, kw, has_norm, eps,
+                        cos_t, sin_t, table_len, tok_pos, tok_seq, block_table, bt_stride, (bf16*)k_cache, (bf16*)v_cache, page_size,
+                        write_kv, vmix, parts);
+            ODIN_LAUNCH_CHECK();
+            return 0;
+        }
 #define FAST(VEC, TI, TOK)                                                                                         \
     odin_launch(head_prep_fast_kernel<VEC, TI, TOK>, dim3((T + TOK - 1) / TOK, grid.y), dim3(HP_WARPS * 32), 0, s,     \
                 (const TI*)qkv, n_split, (size_t)split_stride, (bf16*)q_out, (size_t)q_out_stride, T, Hq, Hkv,         \

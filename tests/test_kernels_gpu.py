@@ -414,6 +414,37 @@ def test_grouped_products_of_tiles_with_few_rows(counts, dual):
     ops.moe_tc_check()
 
 
+@pytest.mark.parametrize("T", [256, 259, 2050])
+@pytest.mark.parametrize("n_q,n_kv", [(16, 8), (5, 1), (32, 8), (3, 2)])
+@pytest.mark.parametrize("values", ["plain", "keep", "mix"])
+def test_head_prep_of_prompts_has_the_bits_of_few_tokens(T, n_q, n_kv, values):
+    """Eight lanes a head (prompts) against a warp a head: numbers of heads that fill no group of four or straddle q, k and v,
+    several warps a token and one, with and without the norm, positions beyond the table, a padding row, q in place."""
+    from odin_infer_b200.csrc import ops
+    hd = 128
+    torch.manual_seed(T + n_q)
+    width = (n_q + 2 * n_kv) * hd
+    k_cache, v_cache, bt = paged_cache(1, [T], n_kv, hd, torch.bfloat16)
+    tok_seq, tok_pos = torch.zeros(T, dtype=torch.int32, device=DEV), torch.arange(T, dtype=torch.int32, device=DEV)
+    tok_seq[77] = -1
+    qkv = torch.randn(T, width, device=DEV).bfloat16()
+    ang = torch.randn(T - 3, hd // 2, device=DEV)
+    cos, sin = torch.cos(ang).contiguous(), torch.sin(ang).contiguous()
+    first = torch.randn(T, n_kv * hd, device=DEV).bfloat16()
+    for norm in (None, (1 + 0.1 * torch.randn(hd, device=DEV)).bfloat16()):
+        got = []
+        for step in (T, 100):
+            kc, vc, src = k_cache.clone(), v_cache.clone(), qkv.clone()
+            kept = torch.full((T, n_kv * hd), 3.0, device=DEV, dtype=torch.bfloat16)
+            for a in range(0, T, step):
+                b = min(T, a + step)
+                more = {"plain": {}, "keep": dict(v_keep=kept[a:b]), "mix": dict(v_first=first[a:b].contiguous(), v_lambda=0.3125)}[values]
+                ops.head_prep(src[a:b], n_q, n_kv, hd, norm, norm, 1e-6, cos, sin, hd, tok_pos[a:b].contiguous(),
+                              tok_seq[a:b].contiguous(), bt, kc, vc, **more)   # q over the projection
+            got.append([torch.nan_to_num(t.float(), nan=-1.0) for t in (src, kc, vc, kept)])
+        assert all(torch.equal(x, y) for x, y in zip(*got))
+
+
 @pytest.mark.parametrize("n_seqs", [39, 64, 128, 130])
 @pytest.mark.parametrize("window", [0, 100])
 def test_decode_attention_of_many_unequal_sequences(n_seqs, window):

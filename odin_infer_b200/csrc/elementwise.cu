@@ -232,14 +232,16 @@ add_rmsnorm_kernel(float* __restrict__ x, const TD* __restrict__ delta, int n_sp
     add_rmsnorm_body<TD, TO, VEC, MAX_THREADS>(x, delta, n_split, split_stride, w, eps, out, rows, d, red, rowbuf);
 }
 
-// The variant of 1,024 threads for a few wide rows (decoding): NV groups of four per thread, kept in registers
-// (no staging in shared memory), the parts' loads of a group issued together; the same order of additions as the
-// kernel above, so the same bits.  Its registers are capped so that a block leaves more than a third of an SM's
+// The variant for a few wide rows (decoding): NV groups of four per thread, kept in registers (no staging in shared
+// memory), the loads of PARTS parts of a group issued together; the same order of additions as the kernel above with as
+// many threads, so the same bits.  1,024 threads from 4,096 columns on, 512 below: there a product's update comes in eight
+// or nine parts, and with two of them in flight a row's loads were five trips to L2 (a request of one 37-token question and
+// 24 tokens on the 1.7B size 28.06 ms, with nine in flight 26.34).  Its registers are capped so that a block leaves more than a third of an SM's
 // registers free: the product that follows starts its CTAs while this kernel runs, to fetch weights, and on the
 // SMs that hold a row it could not (with 64 registers a thread the block took them all; those CTAs then started 4
 // to 7 us after the others and the whole product ended that much later).
-template <typename TD, typename TO, int NV>
-__global__ void __maxnreg__(NV == 1 ? 40 : 48)
+template <typename TD, typename TO, int NV, int THREADS, int PARTS>
+__global__ void __maxnreg__(THREADS == 512 ? 64 : NV == 1 ? 40 : 48)
 add_rmsnorm_wide_kernel(float* __restrict__ x, const TD* __restrict__ delta, int n_split, size_t split_stride, VecRef w,
                         float eps, TO* __restrict__ out, const int* __restrict__ rows, int d) {
     __shared__ float red[32];
@@ -261,19 +263,19 @@ add_rmsnorm_wide_kernel(float* __restrict__ x, const TD* __restrict__ delta, int
     float ss = 0.f;
 #pragma unroll
     for (int k = 0; k < NV; ++k) {
-        const int j = j0 + k * 4096;
+        const int j = j0 + k * (THREADS * 4);
         v[k] = make_float4(0.f, 0.f, 0.f, 0.f);
         if (j < d) {
             v[k] = load4<float>(xr + j);
             if (delta != nullptr) {
                 const TD* dp = delta + (size_t)src * d + j;
-                for (int s0 = 0; s0 < n_split; s0 += 4) {
-                    float4 dv[4];
+                for (int s0 = 0; s0 < n_split; s0 += PARTS) {
+                    float4 dv[PARTS];
 #pragma unroll
-                    for (int u = 0; u < 4; ++u)
+                    for (int u = 0; u < PARTS; ++u)
                         if (s0 + u < n_split) dv[u] = load4<TD>(dp + (size_t)(s0 + u) * split_stride);
 #pragma unroll
-                    for (int u = 0; u < 4; ++u)
+                    for (int u = 0; u < PARTS; ++u)
                         if (s0 + u < n_split) { v[k].x += dv[u].x; v[k].y += dv[u].y; v[k].z += dv[u].z; v[k].w += dv[u].w; }
                 }
             }
@@ -289,7 +291,7 @@ add_rmsnorm_wide_kernel(float* __restrict__ x, const TD* __restrict__ delta, int
     const bool write_back = (delta != nullptr) && (rows == nullptr);
 #pragma unroll
     for (int k = 0; k < NV; ++k) {
-        const int j = j0 + k * 4096;
+        const int j = j0 + k * (THREADS * 4);
         if (j < d) {
             if (write_back) store4(xr + j, v[k]);
             const float4 wv = (k == 0) ? w0 : load4w(w, j);
@@ -392,11 +394,19 @@ static int launch_add_rmsnorm(float* x, const void* delta, int n_split, size_t s
         // rows on the kernel of 512 threads runs, as it does for prompts.
         const bool big = !std::is_same<TO, float>::value && d >= 4096 && d <= 8192 && n_rows <= 128;
         if (big) {
-            auto wide = d <= 4096 ? add_rmsnorm_wide_kernel<TD, TO, 1> : add_rmsnorm_wide_kernel<TD, TO, 2>;
+            auto wide = d <= 4096 ? add_rmsnorm_wide_kernel<TD, TO, 1, 1024, 4> : add_rmsnorm_wide_kernel<TD, TO, 2, 1024, 4>;
             odin_launch(wide, dim3(n_rows), dim3(1024), 0, s, x, (const TD*)delta, n_split, split_stride, w, eps, (TO*)out,
                         rows, d);
             ODIN_LAUNCH_CHECK();
             return 0;
+        }
+        if constexpr (!std::is_same<TO, float>::value) {
+            if (d >= 2048 && d < 4096 && n_rows <= 128) {
+                auto wide = d <= 2048 ? add_rmsnorm_wide_kernel<TD, TO, 1, 512, 9> : add_rmsnorm_wide_kernel<TD, TO, 2, 512, 4>;
+                odin_launch(wide, dim3(n_rows), dim3(512), 0, s, x, (const TD*)delta, n_split, split_stride, w, eps, (TO*)out, rows, d);
+                ODIN_LAUNCH_CHECK();
+                return 0;
+            }
         }
         const int threads = d >= 2048 ? 512 : (d >= 1024 ? 256 : 128);
         auto kern = add_rmsnorm_kernel<TD, TO, true, 512>;

@@ -445,6 +445,24 @@ def test_head_prep_of_prompts_has_the_bits_of_few_tokens(T, n_q, n_kv, values):
         assert all(torch.equal(x, y) for x, y in zip(*got))
 
 
+@pytest.mark.parametrize("d,parts", [(2048, 1), (2048, 8), (2048, 9), (2048, 13), (2052, 3), (3072, 5), (4092, 6)])
+@pytest.mark.parametrize("delta_dtype", [torch.float32, torch.bfloat16])
+def test_add_rmsnorm_of_few_rows_has_the_bits_of_more(d, parts, delta_dtype):
+    """Up to 128 rows keep their row in registers and more parts in flight; 129 rows take the kernel of more rows."""
+    from odin_infer_b200.csrc import ops
+    torch.manual_seed(d + parts)
+    x = torch.randn(129, d, device=DEV)
+    delta = torch.randn(parts, 129, d, device=DEV).to(delta_dtype)
+    w = (1 + 0.1 * torch.randn(d, device=DEV)).bfloat16()
+    got = {}
+    for rows in (129, 128, 1):
+        xs, out = x[:rows].clone(), torch.empty(rows, d, device=DEV, dtype=torch.bfloat16)
+        ops.add_rmsnorm(xs, delta[:, :rows].contiguous(), w, 1e-6, out)
+        got[rows] = (xs, out)
+    for rows in (128, 1):
+        assert torch.equal(got[rows][0], got[129][0][:rows]) and torch.equal(got[rows][1], got[129][1][:rows])
+
+
 @pytest.mark.parametrize("n_seqs", [39, 64, 128, 130])
 @pytest.mark.parametrize("window", [0, 100])
 def test_decode_attention_of_many_unequal_sequences(n_seqs, window):

@@ -463,6 +463,39 @@ def test_add_rmsnorm_of_few_rows_has_the_bits_of_more(d, parts, delta_dtype):
         assert torch.equal(got[rows][0], got[129][0][:rows]) and torch.equal(got[rows][1], got[129][1][:rows])
 
 
+@pytest.mark.parametrize("V", [2, 31, 384, 1024])
+def test_top_p_of_short_rows_draws_the_references_token(V):
+    """One candidate a thread: flat rows, ties inside the kept set and at the cut, candidates at minus infinity and at the
+    type's lowest value, the smallest row; a row without any candidate gives a valid token."""
+    from odin_infer_b200.csrc import ops
+    from tests.plain import qwen3_plain as P
+    torch.manual_seed(V)
+    rows = [torch.randn(V) * 4, torch.randn(V) * 0.3, torch.zeros(V), torch.randn(V)]
+    rows[2][:V // 2] = torch.randint(0, 3, (V // 2,)).float()
+    rows[3][1::2] = float("-inf")
+    rows.append(torch.where(torch.arange(V) % 3 == 0, torch.randn(V), torch.finfo(torch.float32).min))
+    rows.append(torch.full((V,), float("-inf")))
+    logits = torch.stack(rows).to(DEV)
+    B = logits.shape[0]
+    out = torch.empty(B, dtype=torch.int32, device=DEV)
+    checked = 0
+    for temp, tp in ((1.0, 0.9), (0.7, 0.5), (1.3, 0.95), (1.0, 0.999), (1.0, 0.05)):
+        probs = [P.temperature_probs(logits[b].double().cpu(), temp) for b in range(B - 1)]
+        for coin in (0.0, 0.013, 0.2, 0.37, 0.5, 0.77, 0.93, 0.9999):
+            ops.sample(logits, temp, tp, torch.full((B,), coin, device=DEV), out)
+            got = out.tolist()
+            assert all(0 <= token < V for token in got)
+            for b in range(B - 1):
+                if float(probs[b].max()) < (1 - tp) / (V - 1):
+                    continue   # no candidate reaches the cutoff: there is no token of the reference's
+                tok, margin = P.sample_topp(probs[b], tp, coin)
+                assert got[b] in P.top_p_keep(probs[b], tp) or margin < 1e-5, (V, temp, tp, coin, b)
+                if margin > 1e-5:
+                    assert got[b] == tok, (V, temp, tp, coin, b, got[b], tok)
+                    checked += 1
+    assert checked > 60
+
+
 @pytest.mark.parametrize("n_seqs", [39, 64, 128, 130])
 @pytest.mark.parametrize("window", [0, 100])
 def test_decode_attention_of_many_unequal_sequences(n_seqs, window):

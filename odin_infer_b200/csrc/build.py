@@ -35,7 +35,7 @@ GROUPS = {
     "gated_unit": ["gated_unit.cu"],
     "streams": ["streams.cu"],
     "moe": ["moe.cu"],
-    "moe_tc": ["moe_tc.cu"],
+    "moe_tc": ["moe_tc.cu", "moe_few_tc.cu"],
     "latent": ["latent.cu"],
     "gemm_plain": ["gemm_plain.cu"],
     "head_prep": ["head_prep.cu"],

@@ -15,22 +15,16 @@
 // one lane of warp 1 issues the MMAs (128 x 256 each) into tensor memory, warps 2..5 read the accumulator back and
 // store.  With many tiles two CTAs share an SM, so one's epilogue runs beside the other's products; with few, each has
 // a longer ring.  Every wait is bounded (tc::mbar_wait).
-#include <mutex>
-#include <unordered_map>
-
 #include "head_gate.cuh"
-#include "tc_common.cuh"
+#include "moe_tc_host.cuh"
+
+using namespace moe_tc;
 
 namespace {
 
 constexpr int BM = 128;   // sorted rows per tile (MMA M)
 constexpr int BN = 128;   // output columns per accumulator of the gated product (MMA N); the plain product takes 2 BN
-constexpr int BK = 64;    // K elements per stage: one 128-byte swizzle row
 constexpr int UMMA_K = 16;
-
-#define MOE_ACT_SILU 1
-#define MOE_ACT_GELU_TANH 2
-#define MOE_ACT_RELU2 4
 
 // ------------------------------------------------------------------------------------------------ plan
 // One CTA.  ids: [rows] expert of every row (-1: none).  Outputs: place_of_row [rows] (-1: none), row_of_place
@@ -140,15 +134,16 @@ moe_gather_kernel(const bf16* __restrict__ h, size_t h_stride, const int* __rest
 // ------------------------------------------------------------------------------------------------ combine
 __global__ void __launch_bounds__(256)
 moe_combine_kernel(const float* __restrict__ c, const int* __restrict__ place_of_row, const float* __restrict__ wts, int per,
-                   int d, float* __restrict__ y) {
+                   int d, float* __restrict__ y, int in_order) {
     pdl_trigger();
     pdl_wait();
     const int t = blockIdx.x;
     for (int i = threadIdx.x * 4; i < d; i += blockDim.x * 4) {
         float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
         for (int k = 0; k < per; ++k) {
-            const int place = place_of_row[t * per + k];
+            int place = place_of_row[t * per + k];
             if (place < 0) continue;
+            if (in_order) place = t * per + k;
             const float w = wts != nullptr ? wts[t * per + k] : 1.0f;
             const float4 v = *reinterpret_cast<const float4*>(c + (size_t)place * d + i);
             acc.x = fmaf(w, v.x, acc.x); acc.y = fmaf(w, v.y, acc.y); acc.z = fmaf(w, v.z, acc.z); acc.w = fmaf(w, v.w, acc.w);
@@ -188,18 +183,6 @@ struct GCfg {
     static constexpr int HEAD = 1024;  // barriers and flags, before the stages (which start 1024-byte aligned)
     static constexpr int smem(int stages) { return 1024 + HEAD + stages * STAGE; }
 };
-
-__device__ __forceinline__ float act_gate(int act, float g) {
-    if (act == MOE_ACT_SILU) return __fdividef(g, 1.0f + __expf(-g));
-    const float y2 = 1.5957691216057308f * g * fmaf(0.044715f * g, g, 1.0f);   // g sigmoid(2 y) = tanh-GELU
-    return __fdividef(g, 1.0f + __expf(-y2));
-}
-
-// an expert without a gate matrix: the activation of its one accumulator (relu2: max(z, 0)^2)
-__device__ __forceinline__ float act_alone(int act, float z) {
-    if (act == MOE_ACT_RELU2) { const float r = fmaxf(z, 0.f); return r * r; }
-    return act_gate(act, z);
-}
 
 // A tile of 128 places of an expert with a handful of rows is nearly all padding.  Up to FEW rows their box alone is copied
 // (2 KB instead of 16 a stage beside 32 KB of weights) and the other rows of the stage hold whatever was there: a row of the
@@ -390,58 +373,6 @@ moe_grouped_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
 }
 
 // ------------------------------------------------------------------------------------------------ host
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
-                                  const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-EncodeTiledFn encode_fn() {
-    static EncodeTiledFn fn = nullptr;
-    static std::once_flag once;
-    std::call_once(once, [] {
-        void* f = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &q) == cudaSuccess &&
-            q == cudaDriverEntryPointSuccess)
-            fn = reinterpret_cast<EncodeTiledFn>(f);
-    });
-    return fn;
-}
-
-// A row-major [rows, K] bfloat16 matrix with row stride ld, read in boxes of 64 (K) x box_rows rows, 128-byte
-// swizzle, zeros beyond the edges.
-int make_map(CUtensorMap* out, const void* ptr, long long rows, long long K, long long ld, int box_rows) {
-    EncodeTiledFn fn = encode_fn();
-    if (fn == nullptr) return ODIN_ERR_UNSUPPORTED;
-    cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)rows};
-    cuuint64_t strides[1] = {(cuuint64_t)ld * 2};
-    cuuint32_t box[2] = {(cuuint32_t)BK, (cuuint32_t)box_rows};
-    cuuint32_t estr[2] = {1, 1};
-    CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(ptr), dims, strides, box, estr,
-                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    return r == CUDA_SUCCESS ? 0 : ODIN_ERR_BAD_ARG;
-}
-
-int* error_flag() {
-    static int* flag = nullptr;
-    static std::once_flag once;
-    std::call_once(once, [] {
-        if (cudaMalloc(&flag, sizeof(int)) == cudaSuccess) cudaMemset(flag, 0, sizeof(int));
-        else flag = nullptr;
-    });
-    return flag;
-}
-
-int sm_count() {
-    static int n = 0;
-    if (n == 0) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
-    }
-    return n;
-}
-
 template <bool DUAL, typename TO, bool PER_ELEMENT = false>
 int launch_grouped(const CUtensorMap& ma, const CUtensorMap& mw, const CUtensorMap& mf, GroupedParams p, int tiles_m, cudaStream_t s, int heads = 1) {
     using C = GCfg;
@@ -492,11 +423,12 @@ extern "C" int odin_moe_gather(const void* h, long long h_stride, const int* row
     return 0;
 }
 
+// in_order: c holds row r at place r, and place_of_row (then the choices' experts) says by its sign alone which rows there are.
 extern "C" int odin_moe_combine(const float* c, const int* place_of_row, const float* wts, int T, int per, int d, float* y,
-                                void* stream) {
+                                int in_order, void* stream) {
     if (T <= 0) return 0;
     if (d % 4 != 0 || ((((uintptr_t)c) | ((uintptr_t)y)) & 15) != 0) return ODIN_ERR_UNSUPPORTED;
-    odin_launch(moe_combine_kernel, dim3(T), dim3(256), 0, (cudaStream_t)stream, c, place_of_row, wts, per, d, y);
+    odin_launch(moe_combine_kernel, dim3(T), dim3(256), 0, (cudaStream_t)stream, c, place_of_row, wts, per, d, y, in_order);
     ODIN_LAUNCH_CHECK();
     return 0;
 }

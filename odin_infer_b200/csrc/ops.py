@@ -534,16 +534,37 @@ def moe_grouped(a: torch.Tensor, w: torch.Tensor, tile_expert: torch.Tensor, out
         c_longlong(out.stride(0)), _stream()), "moe_grouped")
 
 
-def moe_combine(c: torch.Tensor, place_of_row: torch.Tensor, wts: torch.Tensor | None, out: torch.Tensor) -> None:
+def moe_few(h: torch.Tensor, w_gate_up: torch.Tensor, w_down: torch.Tensor, ids: torch.Tensor, kind: str, a: torch.Tensor,
+            c: torch.Tensor, gated: bool = True, in_wts: torch.Tensor | None = None) -> bool:
+    """The grouped products for a step of few tokens, straight from the choices: a[r] (bfloat16) = the activations of row
+    r = t * per + k, c[r] (float32) = Wd[e] a[r]; the same bits.  Rows of choices without an expert are left as they are.
+    Returns False, and launches nothing, for sizes that the kernels do not take."""
+    T, d = h.shape
+    per, ff = ids.shape[1], w_down.shape[2]
+    assert moe_grouped_supported(h, w_gate_up, w_down) and w_gate_up.is_contiguous() and w_down.is_contiguous()
+    assert tuple(w_gate_up.shape[1:]) == ((2 if gated else 1) * ff, d) and w_down.shape[1] == d and w_gate_up.shape[0] == w_down.shape[0]
+    assert a.dtype == torch.bfloat16 and a.is_contiguous() and tuple(a.shape) == (T * per, ff)
+    assert c.dtype == torch.float32 and c.is_contiguous() and tuple(c.shape) == (T * per, d)
+    assert ids.dtype == torch.int32 and ids.is_contiguous() and ids.shape[0] == T
+    code = _fn("moe_tc", "odin_moe_few")(
+        _ptr(h), c_longlong(h.stride(0)), _ptr(w_gate_up), _ptr(w_down), _ptr(ids), _wts(in_wts, ids), c_int(T), c_int(per),
+        c_int(w_down.shape[0]), c_int(ff), c_int(d), c_int(ACTIVATIONS[kind]), c_int(1 if gated else 0), _ptr(a), _ptr(c), _stream())
+    if code == -1:
+        return False
+    _check(code, "moe_few", kernels=2)
+    return True
+
+
+def moe_combine(c: torch.Tensor, place_of_row: torch.Tensor, wts: torch.Tensor | None, out: torch.Tensor, in_order: bool = False) -> None:
     """out[t] = sum_k wts[t, k] * c[place_of_row[t * per + k]] (float32), the choices in their order (wts None: weights
-    of one)."""
+    of one).  in_order: c holds row r at place r, and place_of_row is the choices' experts (-1: none)."""
     T, d = out.shape
     per = place_of_row.numel() // T
     assert c.dtype == out.dtype == torch.float32 and c.is_contiguous() and out.is_contiguous() and c.shape[1] == d
     assert place_of_row.numel() == T * per
     assert wts is None or (wts.dtype == torch.float32 and tuple(wts.shape) == (T, per) and wts.is_contiguous())
     _check(_fn("moe_tc", "odin_moe_combine")(_ptr(c), _ptr(place_of_row), _ptr(wts), c_int(T), c_int(per), c_int(d),
-                                             _ptr(out), _stream()), "moe_combine")
+                                             _ptr(out), c_int(1 if in_order else 0), _stream()), "moe_combine")
 
 
 def moe_tc_check() -> None:

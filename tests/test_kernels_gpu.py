@@ -496,6 +496,43 @@ def test_top_p_of_short_rows_draws_the_references_token(V):
     assert checked > 60
 
 
+@pytest.mark.parametrize("T", [1, 8, 16, 17, 32])
+@pytest.mark.parametrize("E,per,d,ff", [(3, 2, 72, 40), (34, 6, 264, 136), (5, 8, 2048, 64), (200, 4, 136, 328), (1, 1, 64, 64)])
+@pytest.mark.parametrize("kind,gated,weigh_input", [("silu", True, False), ("gelu_tanh", True, True), ("relu2", False, False)])
+def test_experts_of_few_tokens_have_the_grouped_products_bits(T, E, per, d, ff, kind, gated, weigh_input):
+    """A decode step's experts straight from the choices against the sorted rows: choices without an expert, an expert named
+    twice by a token (more rows than the MMA has columns), K that is no whole block, widths that are no whole items, more
+    and fewer items than CTAs; several steps in a row, whose second product starts while the first one runs."""
+    from odin_infer_b200.csrc import ops
+    torch.manual_seed(T * 100 + d)
+    w1 = (torch.randn(E, (2 if gated else 1) * ff, d, device=DEV) / math.sqrt(d)).bfloat16()
+    w2 = (torch.randn(E, d, ff, device=DEV) / math.sqrt(ff)).bfloat16()
+    rows, places = T * per, ops.moe_places(T * per, E)
+    for repeat in range(3):
+        h = torch.randn(T, d, device=DEV).bfloat16()
+        ids = torch.randint(-1, E, (T, per), device=DEV, dtype=torch.int32)
+        wts = torch.rand(T, per, device=DEV)
+        in_wts, out_wts = (wts, None) if weigh_input else (None, wts)
+        por, rop = torch.empty(rows, dtype=torch.int32, device=DEV), torch.empty(places, dtype=torch.int32, device=DEV)
+        tile_expert = torch.empty(places // 128, dtype=torch.int32, device=DEV)
+        ops.moe_plan(ids, E, por, rop, tile_expert)
+        hs, a = torch.empty(places, d, device=DEV).bfloat16(), torch.empty(places, ff, device=DEV).bfloat16()
+        c, ref = torch.empty(places, d, device=DEV), torch.empty(T, d, device=DEV)
+        ops.moe_gather(h, rop, per, hs, in_wts)
+        ops.moe_grouped(hs, w1, tile_expert, a, kind, gated=gated)
+        ops.moe_grouped(a, w2, tile_expert, c)
+        ops.moe_combine(c, por, out_wts, ref)
+        a1, c1 = torch.full((rows, ff), float("nan"), device=DEV).bfloat16(), torch.full((rows, d), float("nan"), device=DEV)
+        y = torch.empty(T, d, device=DEV)
+        assert ops.moe_few(h, w1, w2, ids, kind, a1, c1, gated=gated, in_wts=in_wts)
+        ops.moe_combine(c1, ids, out_wts, y, in_order=True)
+        named = (ids.flatten() >= 0)
+        assert torch.equal(a1[named], a[por[named].long()])
+        assert ref.isfinite().all() and torch.equal(y, ref)
+        assert c1[~named].isnan().all(), "rows without an expert are left alone"
+    ops.moe_tc_check()
+
+
 @pytest.mark.parametrize("n_seqs", [39, 64, 128, 130])
 @pytest.mark.parametrize("window", [0, 100])
 def test_decode_attention_of_many_unequal_sequences(n_seqs, window):

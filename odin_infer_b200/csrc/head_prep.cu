@@ -46,12 +46,14 @@ head_prep_kernel(const TI* qkv, int n_split, size_t split_stride, T* q_out,  // 
     __shared__ float buf[HP_WARPS][HP_MAX_HD];
     __shared__ float whole_ss[2][HP_WARPS];
     pdl_trigger();
-    pdl_wait();
     const int t = blockIdx.x;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int head = blockIdx.y * HP_WARPS + warp;
     const int n_heads = Hq + (v_is_k ? 1 : 2) * Hkv;
-    const int seq = tok_seq[t];
+    // the step's tables are there before the step: a chain of three trips to memory that need not follow the wait
+    const int seq = tok_seq[t], pos = tok_pos[t];
+    const int own_page = seq >= 0 && write_kv ? block_table[(size_t)seq * bt_stride + pos / page_size] : -1;
+    pdl_wait();
     if (seq < 0) return;  // padding token (the whole CTA: it belongs to one token)
     if (norm_mode == 3) {
         // the sums of squares of the token's whole q and whole k projection, by the CTA's warps together and in an order
@@ -76,7 +78,6 @@ head_prep_kernel(const TI* qkv, int n_split, size_t split_stride, T* q_out,  // 
         __syncthreads();
     }
     if (head >= n_heads) return;
-    const int pos = tok_pos[t];
 
     const bool is_q = head < Hq;
     const bool is_k = !is_q && head < Hq + Hkv;
@@ -89,20 +90,38 @@ head_prep_kernel(const TI* qkv, int n_split, size_t split_stride, T* q_out,  // 
 
     T* dst = q_out + (size_t)t * q_out_stride + (size_t)head * hd;
     if (!is_q) {
-        const int page = block_table[(size_t)seq * bt_stride + pos / page_size];
-        if (page < 0) return;
+        if (own_page < 0) return;
         T* base = is_k ? k_cache : v_cache;
-        dst = base + (((size_t)page * Hkv + kvh) * page_size + (pos % page_size)) * n;
+        dst = base + (((size_t)own_page * Hkv + kvh) * page_size + (pos % page_size)) * n;
     }
 
     float* b = buf[warp];
     float ss = 0.f;
-    for (int j = lane; j < n; j += 32) {
-        float v = to_f32(src[j]);
-        for (int sp = 1; sp < n_split; ++sp) v += to_f32(src[(size_t)sp * split_stride + j]);
-        if (bias.p != nullptr) v += bias.at((int)col0 + j);
-        b[j] = v;
-        ss += v * v;
+    for (int j0 = lane; j0 < n; j0 += 128) {   // four elements of four parts at a time, an element's parts in their order
+        float v[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) v[e] = j0 + 32 * e < n ? to_f32(src[j0 + 32 * e]) : 0.f;
+        for (int s0 = 1; s0 < n_split; s0 += 4) {
+            float part[4][4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    if (s0 + u < n_split && j0 + 32 * e < n) part[u][e] = to_f32(src[(size_t)(s0 + u) * split_stride + j0 + 32 * e]);
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    if (s0 + u < n_split && j0 + 32 * e < n) v[e] += part[u][e];
+        }
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const int j = j0 + 32 * e;
+            if (j >= n) break;
+            if (bias.p != nullptr) v[e] += bias.at((int)col0 + j);
+            b[j] = v[e];
+            ss += v[e] * v[e];
+        }
     }
     if (is_k && v_is_k) {   // the same place of the value cache (dst is its key's place)
         T* vdst = v_cache + (dst - k_cache);

@@ -41,10 +41,26 @@ latent_prep_kernel(const TI* __restrict__ down, int n_split, size_t split_stride
     if (seq >= 0 && write_cache) page = block_table[(size_t)seq * bt_stride + pos / page_size];
     pdl_wait();
     const int n = q_rank + kv_rank + rot;
-    for (int j = threadIdx.x; j < n; j += blockDim.x) {
-        float v = 0.f;
-        for (int s = 0; s < n_split; ++s) v += to_f32(down[(size_t)s * split_stride + (size_t)t * row_stride + j]);
-        rowbuf[j] = v;
+    for (int j0 = threadIdx.x; j0 < n; j0 += 4 * blockDim.x) {   // four elements of four parts at a time, an element's parts in their order
+        float v[4] = {0.f, 0.f, 0.f, 0.f};
+        for (int s0 = 0; s0 < n_split; s0 += 4) {
+            float part[4][4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const int j = j0 + e * (int)blockDim.x;
+                    if (s0 + u < n_split && j < n) part[u][e] = to_f32(down[(size_t)(s0 + u) * split_stride + (size_t)t * row_stride + j]);
+                }
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    if (s0 + u < n_split && j0 + e * (int)blockDim.x < n) v[e] += part[u][e];
+        }
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+            if (j0 + e * (int)blockDim.x < n) rowbuf[j0 + e * (int)blockDim.x] = v[e];
     }
     __syncthreads();
     if (q_rank > 0) {

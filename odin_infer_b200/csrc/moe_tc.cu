@@ -140,13 +140,25 @@ moe_combine_kernel(const float* __restrict__ c, const int* __restrict__ place_of
     const int t = blockIdx.x;
     for (int i = threadIdx.x * 4; i < d; i += blockDim.x * 4) {
         float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-        for (int k = 0; k < per; ++k) {
-            int place = place_of_row[t * per + k];
-            if (place < 0) continue;
-            if (in_order) place = t * per + k;
-            const float w = wts != nullptr ? wts[t * per + k] : 1.0f;
-            const float4 v = *reinterpret_cast<const float4*>(c + (size_t)place * d + i);
-            acc.x = fmaf(w, v.x, acc.x); acc.y = fmaf(w, v.y, acc.y); acc.z = fmaf(w, v.z, acc.z); acc.w = fmaf(w, v.w, acc.w);
+        constexpr int B = 8;   // choices whose loads go out together
+        for (int k0 = 0; k0 < per; k0 += B) {
+            int place[B];
+            float w[B];
+            float4 v[B];
+#pragma unroll
+            for (int k = 0; k < B; ++k) {
+                place[k] = k0 + k < per ? place_of_row[t * per + k0 + k] : -1;
+                w[k] = k0 + k < per && wts != nullptr ? wts[t * per + k0 + k] : 1.0f;
+            }
+#pragma unroll
+            for (int k = 0; k < B; ++k)
+                if (place[k] >= 0) v[k] = *reinterpret_cast<const float4*>(c + (size_t)(in_order ? t * per + k0 + k : place[k]) * d + i);
+#pragma unroll
+            for (int k = 0; k < B; ++k)
+                if (place[k] >= 0) {
+                    acc.x = fmaf(w[k], v[k].x, acc.x); acc.y = fmaf(w[k], v[k].y, acc.y);
+                    acc.z = fmaf(w[k], v[k].z, acc.z); acc.w = fmaf(w[k], v[k].w, acc.w);
+                }
         }
         *reinterpret_cast<float4*>(y + (size_t)t * d + i) = acc;
     }

@@ -61,18 +61,10 @@ row_update_kernel(float* x, const TD* __restrict__ delta, int n_split, size_t sp
         for (int j = threadIdx.x * 4; j < d; j += blockDim.x * 4) {
             const float4 x0 = ld4(xr + j);
             float4 v = scaled ? make_float4(0.f, 0.f, 0.f, 0.f) : x0;
-            if (delta != nullptr)
-                for (int s = 0; s < n_split; ++s) {
-                    const float4 dv = ld4(delta + (size_t)s * split_stride + (size_t)src * d + j);
-                    v.x += dv.x; v.y += dv.y; v.z += dv.z; v.w += dv.w;
-                }
+            if (delta != nullptr) add_parts4<8>(v, delta + (size_t)src * d + j, split_stride, n_split);
 #pragma unroll
             for (int m = 0; m < 2; ++m)
-                if (more.p[m] != nullptr)
-                    for (int s = 0; s < more.n_split[m]; ++s) {
-                        const float4 dv = ld4(more.p[m] + (size_t)s * more.stride[m] + (size_t)src * d + j);
-                        v.x += dv.x; v.y += dv.y; v.z += dv.z; v.w += dv.w;
-                    }
+                if (more.p[m] != nullptr) add_parts4<8>(v, more.p[m] + (size_t)src * d + j, more.stride[m], more.n_split[m]);
             if (bias.p != nullptr) {
                 const float4 bv = bias.at4(j);
                 v.x += bv.x; v.y += bv.y; v.z += bv.z; v.w += bv.w;
@@ -330,10 +322,7 @@ activation_kernel(const TI* __restrict__ in, int n_split, size_t split_stride, s
         for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total4; i += (long long)gridDim.x * blockDim.x) {
             const int t = (int)(i / n4), c = (int)(i % n4) * 4;
             float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
-            for (int s = 0; s < n_split; ++s) {
-                const float4 v = ld4(in + (size_t)s * split_stride + (size_t)t * in_stride + c);
-                z.x += v.x; z.y += v.y; z.z += v.z; z.w += v.w;
-            }
+            add_parts4<8>(z, in + (size_t)t * in_stride + c, split_stride, n_split);
             const float f = row_scale != nullptr ? row_scale[t] : 1.0f;
             st4(out + (size_t)t * out_stride + c, make_float4(activate(act, z.x, c0, c1) * f, activate(act, z.y, c0, c1) * f,
                                                                activate(act, z.z, c0, c1) * f, activate(act, z.w, c0, c1) * f));
@@ -496,10 +485,7 @@ sigmoid_gate_vec_kernel(TO* __restrict__ o, size_t o_stride, const TG* __restric
             for (int s = 0; s < n_split; ++s) zh += to_f32(gate[(size_t)s * split_stride + (size_t)t * gate_stride + c / vd]);
             z = make_float4(zh, zh, zh, zh);
         } else {
-            for (int s = 0; s < n_split; ++s) {
-                const float4 g = ld4(gate + (size_t)s * split_stride + (size_t)t * gate_stride + c);
-                z.x += g.x; z.y += g.y; z.z += g.z; z.w += g.w;
-            }
+            add_parts4<8>(z, gate + (size_t)t * gate_stride + c, split_stride, n_split);
         }
         TO* p = o + (size_t)t * o_stride + c;
         const float4 v = ld4(p);

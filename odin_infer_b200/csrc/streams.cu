@@ -182,12 +182,29 @@ mix_streams_fast_kernel(StreamArgs a, TO* __restrict__ out) {
 #pragma unroll
         for (int i = 0; i < NV; ++i) load_streams(i, X[EARLY ? i : 0]);
     }
+    // one group of four a thread (decoding): the first parts of every term go out together, before any of them is added
+    constexpr int B = NV != 1 ? 1 : NT < 2 ? 9 : 6;
+    float4 early[NT > 0 ? NT : 1][B];
+    const int own = threadIdx.x * 4;
+    if (NV == 1 && own < d) {
+#pragma unroll
+        for (int n = 0; n < NT; ++n)
+#pragma unroll
+            for (int sp = 0; sp < B; ++sp)
+                if (sp < a.terms.t[n].n_split)
+                    early[n][sp] = ld4((const float*)a.terms.t[n].p + (size_t)sp * a.terms.t[n].split_stride + (size_t)r * d + own);
+    }
 #pragma unroll
     for (int n = 0; n < NT; ++n) {
         const CombineTerm& tm = a.terms.t[n];
 #pragma unroll
         for (int i = 0; i < NV; ++i) t[n][i] = make_float4(0.f, 0.f, 0.f, 0.f);
-        for (int sp = 0; sp < tm.n_split; ++sp) {
+        if (NV == 1 && own < d) {
+#pragma unroll
+            for (int sp = 0; sp < B; ++sp)
+                if (sp < tm.n_split) { t[n][0].x += early[n][sp].x; t[n][0].y += early[n][sp].y; t[n][0].z += early[n][sp].z; t[n][0].w += early[n][sp].w; }
+        }
+        for (int sp = NV == 1 ? B : 0; sp < tm.n_split; ++sp) {
 #pragma unroll
             for (int i = 0; i < NV; ++i) {
                 const int j = (threadIdx.x + i * blockDim.x) * 4;

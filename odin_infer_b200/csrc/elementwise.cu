@@ -20,6 +20,23 @@ __global__ void embed_kernel(const TW* __restrict__ table, const int* __restrict
     const TW* row = table + (size_t)(ok ? id : 0) * d;
     float* o = out + (size_t)t * d;
     const size_t next = (size_t)gridDim.x * d;   // a residual of several streams starts with as many copies of the rows
+    if (ok && (d & 3) == 0 && (((uintptr_t)table | (uintptr_t)out) & 15) == 0) {   // (a row's loads go out together)
+        constexpr int U = 4;
+        for (int j0 = threadIdx.x * 4; j0 < d; j0 += blockDim.x * 4 * U) {
+            float4 v[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                if (j0 + u * (int)blockDim.x * 4 < d) v[u] = ld4(row + j0 + u * (int)blockDim.x * 4);
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int j = j0 + u * (int)blockDim.x * 4;
+                if (j < d)
+                    for (int k = 0; k < copies; ++k)
+                        st4(o + k * next + j, make_float4(v[u].x * scale, v[u].y * scale, v[u].z * scale, v[u].w * scale));
+            }
+        }
+        return;
+    }
     for (int j = threadIdx.x; j < d; j += blockDim.x) {
         const float v = ok ? to_f32(row[j]) * scale : 0.f;
         for (int k = 0; k < copies; ++k) o[k * next + j] = v;

@@ -533,6 +533,28 @@ def test_experts_of_few_tokens_have_the_grouped_products_bits(T, E, per, d, ff, 
     ops.moe_tc_check()
 
 
+@pytest.mark.parametrize("V,ld", [(16383, 16383), (16384, 16384), (16389, 16392), (16389, 16389), (151936, 151936), (32771, 40000)])
+@pytest.mark.parametrize("B", [1, 5])
+def test_argmax_of_long_rows_is_the_first_maximum(V, ld, B):
+    """Rows shared by a cluster of blocks: the maximum at the edges of the blocks' shares and of their vectors, twice (the first
+    counts), rows whose distance is no whole vector, a row of equal values, a row at minus infinity."""
+    from odin_infer_b200.csrc import ops
+    torch.manual_seed(V + B)
+    share = ((V + 7) // 8 + 3) // 4 * 4
+    for first in (0, 1, 3, share - 1, share, 2 * share + 2047, V - 5, V - 1):
+        logits = torch.randn(B, ld, device=DEV)
+        logits[:, first] = 50.0
+        logits[:, (first + 1 + torch.randint(0, 9, (1,)).item()) % V] = 50.0
+        logits[:, V:] = 99.0
+        out = torch.empty(B, dtype=torch.int32, device=DEV)
+        ops.argmax(logits[:, :V], out)
+        want = int((logits[0, :V] == 50.0).nonzero().min())
+        assert out.tolist() == [want] * B
+    for value in (0.0, float("-inf")):
+        ops.argmax(torch.full((B, ld), value, device=DEV)[:, :V], out)
+        assert out.tolist() == [0] * B
+
+
 @pytest.mark.parametrize("n_seqs", [39, 64, 128, 130])
 @pytest.mark.parametrize("window", [0, 100])
 def test_decode_attention_of_many_unequal_sequences(n_seqs, window):

@@ -38,8 +38,28 @@ def _ptr(t: torch.Tensor | None) -> c_void_p:
     return c_void_p(t.data_ptr())
 
 
+_current_raw_stream = torch._C._cuda_getCurrentRawStream if hasattr(torch._C, "_cuda_getCurrentRawStream") else None
+
+
 def _stream() -> c_void_p:
-    return c_void_p(torch.cuda.current_stream().cuda_stream)
+    """The current stream's handle, without a Stream object on the way (several microseconds a launch)."""
+    if _current_raw_stream is None:
+        return c_void_p(torch.cuda.current_stream().cuda_stream)
+    return c_void_p(_current_raw_stream(torch.cuda.current_device()))
+
+
+_streams: dict = {}
+
+
+def current_stream() -> torch.cuda.Stream:
+    """`torch.cuda.current_stream()` from a table of the streams seen so far (a handful: torch's streams are a fixed pool)."""
+    if _current_raw_stream is None:
+        return torch.cuda.current_stream()
+    key = torch._C._cuda_getCurrentStream(torch.cuda.current_device())
+    s = _streams.get(key)
+    if s is None:
+        s = _streams[key] = torch.cuda.current_stream()
+    return s
 
 
 _ERRORS = {-1: "unsupported size or element type", -2: "bad argument", -3: "device wait ran out"}

@@ -19,6 +19,7 @@ import numpy as np
 import torch
 
 from ..cache.groups import PAGE
+from ..csrc import ops
 
 
 @dataclasses.dataclass
@@ -177,7 +178,7 @@ class StepBatch:
         if self._dev.is_cuda:
             if self._copied is None:
                 self._copied = torch.cuda.Event()
-            self._copied.record()
+            self._copied.record(ops.current_stream())
 
     def _advance(self, entries: list[StepEntry], start_positions: list[int]) -> bool:
         """The usual decode step: the sequences of the last fill, in the same order, one token

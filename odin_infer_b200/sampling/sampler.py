@@ -122,13 +122,14 @@ class PendingTokens:
 
     def __init__(self, device_tokens):
         import torch
+        from ..csrc import ops
         self.device_tokens = device_tokens
         self._host = torch.empty(device_tokens.shape, dtype=device_tokens.dtype, pin_memory=device_tokens.is_cuda)
         self._host.copy_(device_tokens, non_blocking=True)
         self._event = None
         if device_tokens.is_cuda:
             self._event = torch.cuda.Event()
-            self._event.record()
+            self._event.record(ops.current_stream())
 
     def tokens(self) -> list[int]:
         if self._event is not None:

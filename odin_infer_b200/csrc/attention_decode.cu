@@ -231,7 +231,7 @@ using attn_decode::DecodeTcParams;
 using attn_decode::DecodeTcSmem;
 
 // The kernel of its own: a CTA of four warps per (key split, kv head, sequence).
-template <int HD, int SLOTS, int PREP>
+template <int HD, int SLOTS, int PREP, bool TOG>
 __global__ void __launch_bounds__(128)
 attn_decode_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
                       const DecodeTcParams p) {
@@ -241,7 +241,7 @@ attn_decode_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
     int t = (int)blockIdx.z;
     if (p.by_length > 0)
         t = attn_decode::token_by_length(p, t, (int)threadIdx.x, reinterpret_cast<int*>(smem + DecodeTcSmem<HD, SLOTS>::PAGES_AT));
-    attn_decode::attn_decode_tc_body<HD, SLOTS, PREP, 0>(map_k, map_v, p, smem, (int)threadIdx.x, (int)blockIdx.x,
+    attn_decode::attn_decode_tc_body<HD, SLOTS, PREP, TOG, 0>(map_k, map_v, p, smem, (int)threadIdx.x, (int)blockIdx.x,
                                                          (int)blockIdx.y, t, [] { pdl_wait(); });
 }
 
@@ -335,17 +335,17 @@ int* device_symbol(const T& symbol) {
 int* decode_error_flag() { return device_symbol(g_decode_error); }
 int* split_counters() { return device_symbol(g_split_counters); }
 
-template <int HD, int SLOTS, int PREP>
+template <int HD, int SLOTS, int PREP, bool TOG>
 int launch_decode_tc_slots(const CUtensorMap& mk, const CUtensorMap& mv, const DecodeTcParams& p, dim3 grid, cudaStream_t s) {
     constexpr int SMEM = DecodeTcSmem<HD, SLOTS>::BYTES;
     static bool configured = false;
     if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(attn_decode_tc_kernel<HD, SLOTS, PREP>,
+        cudaError_t e = cudaFuncSetAttribute(attn_decode_tc_kernel<HD, SLOTS, PREP, TOG>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
         if (e != cudaSuccess) return (int)e;
         configured = true;
     }
-    odin_launch(attn_decode_tc_kernel<HD, SLOTS, PREP>, grid, dim3(128), (size_t)SMEM, s, mk, mv, p);
+    odin_launch(attn_decode_tc_kernel<HD, SLOTS, PREP, TOG>, grid, dim3(128), (size_t)SMEM, s, mk, mv, p);
     ODIN_LAUNCH_CHECK();
     return 0;
 }
@@ -362,6 +362,7 @@ struct PrepArgs {
     const float* sin_t;
     int table_len;
     int write_kv;
+    int short_ctx;   // no sequence has more than a few pages
 };
 
 template <int HD>
@@ -412,12 +413,14 @@ int launch_decode_tc(const bf16* q, size_t q_stride, bf16* out, size_t out_strid
     const bool deep = ctas <= deep_upto;
     // more CTAs than are resident together (two an SM): the longest sequences first
     p.by_length = (ctas > 2LL * sms && B > 1 && B <= attn_decode::BY_LENGTH_MAX) ? B : 0;
-#define GO(PREP)                                                                  \
-    (deep ? launch_decode_tc_slots<HD, 6, PREP>(mk, mv, p, grid, s)               \
-          : launch_decode_tc_slots<HD, 3, PREP>(mk, mv, p, grid, s))
-    if (mode == 0) return GO(0);
-    if (mode == 1) return GO(1);
-    return GO(2);
+    // short contexts in one split: the kernel that shares a page among the warps
+    const bool tog = prep != nullptr && prep->short_ctx && n_split == 1;
+#define GO(PREP, TOG)                                                                  \
+    (deep ? launch_decode_tc_slots<HD, 6, PREP, TOG>(mk, mv, p, grid, s)               \
+          : launch_decode_tc_slots<HD, 3, PREP, TOG>(mk, mv, p, grid, s))
+    if (mode == 0) return GO(0, false);
+    if (mode == 1) return tog ? GO(1, true) : GO(1, false);
+    return tog ? GO(2, true) : GO(2, false);
 #undef GO
 }
 
@@ -518,7 +521,7 @@ extern "C" int odin_attention_decode_fused(const void* qkv, int in_dtype, int pa
                                            int table_len, void* k_cache, void* v_cache, int page_size, int n_pages,
                                            const int* tok_pos, const int* tok_seq, const int* block_table,
                                            int bt_stride, int window, float* scratch, int n_split, int write_kv,
-                                           void* stream) {
+                                           int short_ctx, void* stream) {
     if (B <= 0) return 0;
     if (Hkv <= 0 || Hq % Hkv != 0 || n_split < 1 || scratch == nullptr || parts < 1) return ODIN_ERR_BAD_ARG;
     if (B > 65535 || Hq > 65535 || n_split > 65535) return ODIN_ERR_UNSUPPORTED;
@@ -535,6 +538,7 @@ extern "C" int odin_attention_decode_fused(const void* qkv, int in_dtype, int pa
     prep.k_norm = VecRef{k_norm_w, w_dtype == ODIN_BF16};
     prep.has_norm = has_norm; prep.eps = eps; prep.cos_t = cos_t; prep.sin_t = sin_t; prep.table_len = table_len;
     prep.write_kv = write_kv;
+    prep.short_ctx = short_ctx;
     cudaStream_t s = (cudaStream_t)stream;
     float* part_acc = scratch;
     float* part_ml = scratch + (size_t)B * Hq * n_split * hd;

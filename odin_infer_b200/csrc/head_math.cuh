@@ -71,6 +71,28 @@ __device__ __forceinline__ void load_parts(const TI* src, int n_split, size_t sp
     }
 }
 
+// The same for two heads (the second where `both`), whose loads are in flight together.
+template <int VEC, typename TI>
+__device__ __forceinline__ void load_parts2(const TI* src0, const TI* src1, bool both, int n_split, size_t split_stride, float (&v)[2][VEC]) {
+    load_vec<VEC>(src0, v[0]);
+    if (both) load_vec<VEC>(src1, v[1]);
+    for (int s0 = 1; s0 < n_split; s0 += 4) {
+        float w2[2][4][VEC];
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (s0 + u < n_split) {
+                load_vec<VEC>(src0 + (size_t)(s0 + u) * split_stride, w2[0][u]);
+                if (both) load_vec<VEC>(src1 + (size_t)(s0 + u) * split_stride, w2[1][u]);
+            }
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (s0 + u < n_split) {
+#pragma unroll
+                for (int e = 0; e < VEC; ++e) { v[0][e] += w2[0][u][e]; v[1][e] += w2[1][u][e]; }
+            }
+    }
+}
+
 // v: this lane's elements of the head; wn: the norm's weights at the same places; c, sn: the
 // cosines and sines of the position's angles at this lane's places of the first half.
 template <int VEC>

@@ -1294,9 +1294,11 @@ def attention_decode_fused(qkv: torch.Tensor, out: torch.Tensor, n_q: int, n_kv:
                            q_norm: torch.Tensor | None, k_norm: torch.Tensor | None, eps: float, cos: torch.Tensor,
                            sin: torch.Tensor, rotary_dim: int, k_cache: torch.Tensor, v_cache: torch.Tensor,
                            tok_pos: torch.Tensor, tok_seq: torch.Tensor, block_table: torch.Tensor, window: int,
-                           scratch: torch.Tensor, n_split: int, write_kv: bool = True) -> bool:
+                           scratch: torch.Tensor, n_split: int, write_kv: bool = True, short: bool = False) -> bool:
     """`head_prep` and `attention_decode` in one kernel, for one token per sequence: qkv is the
     fused projection's output ([B, width] bfloat16, or float32 partial sums [parts, B, width]).
+    short: the contexts are of a page or two: a kernel whose warps share a sequence's only page (any context is right, with
+    the same bits).
     Returns False, and launches nothing, where the tensor-core kernel does not apply; the
     caller then runs the two kernels."""
     width = (n_q + 2 * n_kv) * head_dim
@@ -1324,7 +1326,7 @@ def attention_decode_fused(qkv: torch.Tensor, out: torch.Tensor, n_q: int, n_kv:
         _ptr(k_norm), c_int(dtype_code(q_norm.dtype) if has_norm else 0), c_int(1 if has_norm else 0), c_float(eps),
         _ptr(cos), _ptr(sin), c_int(rotary_dim), c_int(cos.shape[0]), _ptr(k_cache), _ptr(v_cache), c_int(PAGE),
         c_int(k_cache.shape[0]), _ptr(tok_pos), _ptr(tok_seq), _ptr(block_table), c_int(block_table.stride(0)),
-        c_int(window), _ptr(scratch), c_int(n_split), c_int(1 if write_kv else 0), _stream())
+        c_int(window), _ptr(scratch), c_int(n_split), c_int(1 if write_kv else 0), c_int(1 if short else 0), _stream())
     if code == -1:  # unsupported: nothing was launched
         return False
     _check(code, "attention_decode_fused")

@@ -67,6 +67,13 @@ LIGHT_STAGES = int(os.environ.get("ODIN_GEMM_LIGHT_STAGES", "5"))
 STAGED_BLOCKS = int(os.environ.get("ODIN_GEMM_STAGED", "15"))
 
 
+# Up to this many keys a decode step's attention runs the kernel whose warps share a sequence's only page (with head
+# preparation, one key split).  A step of one sequence on the 1.7B size at 20 to 50 keys 1.02 -> 0.958 ms, at 90 to 120 (two
+# pages, a warp each) 1.02 -> 0.99, at 180 to 210 0.98 -> 1.00; on the 8B size at 30 to 60 2.70 -> 2.66, at 200 to 230 2.69 -> 2.72.
+# In one kernel with the code of more pages it cost those steps 2 to 5 %.
+SHORT_CONTEXT = 128
+
+
 def context_class_of(longest: int, page: int = 64) -> int:
     """Contexts of one class launch the same kernels: the number of 8-page groups of the
     longest sequence."""
@@ -311,7 +318,7 @@ class Runtime:
         scratch = self.empty(ops.attention_decode_scratch(B, n_q, head_dim, n_split), dtype=torch.float32)
         return ops.attention_decode_fused(qkv, out, n_q, n_kv, head_dim, q_norm, k_norm, eps, cos, sin, rotary_dim,
                                           k_line, v_line, step.tok_pos, step.tok_seq, block_table, window, scratch,
-                                          n_split, write_kv)
+                                          n_split, write_kv, short=step.max_len_after <= SHORT_CONTEXT)
 
     def settle(self, x: torch.Tensor, delta, bias) -> torch.Tensor:
         """Adds an update that was still pending (and its bias) to the residual stream x, and returns x in

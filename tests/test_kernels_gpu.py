@@ -555,6 +555,44 @@ def test_argmax_of_long_rows_is_the_first_maximum(V, ld, B):
         assert out.tolist() == [0] * B
 
 
+@pytest.mark.parametrize("geom", [(16, 8, 128), (32, 8, 128), (8, 1, 64), (6, 2, 64), (20, 2, 128)])
+@pytest.mark.parametrize("parts", [0, 1, 4, 9])
+@pytest.mark.parametrize("window", [0, 20])
+def test_decode_attention_of_short_contexts_has_the_bits_of_any(geom, parts, window):
+    """The kernel whose warps share a sequence's only page (up to eight query heads a kv head; ten take it a warp alone) against
+    the kernel of every context: numbers of keys around a page's sixteens, more pages than one, stale NaN behind the
+    sequences' ends, padding rows; what both write to the cache."""
+    from odin_infer_b200.csrc import ops
+    n_q, n_kv, hd = geom
+    lengths = [1, 2, 15, 16, 17, 32, 33, 48, 63, 64, 65, 128, 200, 641]
+    B = len(lengths)
+    torch.manual_seed(hd + parts)
+    k_cache, v_cache, bt = paged_cache(B, lengths, n_kv, hd, torch.bfloat16)
+    for s, n in enumerate(lengths):
+        pages = bt[s, : (n + 63) // 64].long()
+        for cache in (k_cache, v_cache):
+            cache[pages] = torch.randn(pages.numel(), n_kv, 64, hd, device=DEV).bfloat16()
+            cache[int(pages[-1]), :, (n - 1) % 64:] = float("nan")   # the newest token's place and what lies behind it
+    order = [3, 0, -1, 6, 1, 5, 2, 4, 13, 12, 11, 10, 9, 8, 7]
+    tok_seq = torch.tensor(order, dtype=torch.int32, device=DEV)
+    tok_pos = torch.tensor([lengths[s] - 1 if s >= 0 else 0 for s in order], dtype=torch.int32, device=DEV)
+    T, width = len(order), (n_q + 2 * n_kv) * hd
+    qkv = torch.randn(T, width, device=DEV).bfloat16() if parts == 0 else torch.randn(parts, T, width, device=DEV) / math.sqrt(parts)
+    norm = (1 + 0.1 * torch.randn(hd, device=DEV)).bfloat16()
+    ang = torch.randn(700, hd // 2, device=DEV)
+    cos, sin = torch.cos(ang).contiguous(), torch.sin(ang).contiguous()
+    for n_split in (1, 3):
+        scratch = torch.empty(ops.attention_decode_scratch(T, n_q, hd, n_split), device=DEV)
+        got = []
+        for short in (False, True):
+            kc, vc, out = k_cache.clone(), v_cache.clone(), torch.full((T, n_q * hd), 7.0, device=DEV, dtype=torch.bfloat16)
+            assert ops.attention_decode_fused(qkv, out, n_q, n_kv, hd, norm, norm, 1e-6, cos, sin, hd, kc, vc, tok_pos, tok_seq, bt,
+                                              window, scratch, n_split, short=short)
+            got.append([out] + [torch.nan_to_num(t.float(), nan=-1.0) for t in (kc, vc)])
+        assert got[0][0].isfinite().all() and all(torch.equal(a, b) for a, b in zip(*got))
+    ops.attention_decode_check()
+
+
 @pytest.mark.parametrize("n_seqs", [39, 64, 128, 130])
 @pytest.mark.parametrize("window", [0, 100])
 def test_decode_attention_of_many_unequal_sequences(n_seqs, window):

@@ -133,7 +133,6 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
     float* s_max = reinterpret_cast<float*>(bars + 16);  // [2 buffers][2 halves][128 rows]: the pair's exchange
 
-    pdl_trigger();
     pdl_wait();
     if ((uint32_t)(smem - smem_raw) > 896u) {  // the shared-memory window is less aligned than assumed
         if (threadIdx.x == 0 && p.error != nullptr) atomicExch(p.error, 2);
@@ -145,6 +144,9 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
+    // Only now: the product after this kernel may take all 512 columns before its own wait.  Had it come to this SM ahead of the
+    // allocation above, that would wait for the product's columns and the product for this kernel's end.
+    pdl_trigger();
     const uint32_t tmem_base = *tmem_slot;
 
     // The CTAs are persistent (two per SM) and take the (head, sequence, tile) triples themselves: the triples are

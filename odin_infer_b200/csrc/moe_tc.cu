@@ -219,7 +219,6 @@ moe_grouped_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
     uint8_t* smem = base + 1024;   // the stages: 1024-byte aligned for the 128-byte swizzle
     const uint32_t n_stages = (uint32_t)p.stages;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    pdl_trigger();
     if (threadIdx.x == 0) {
         for (int s = 0; s < C::MAX_STAGES; ++s) { tc::mbar_init(&full[s], 1); tc::mbar_init(&empty[s], 1); }
         tc::mbar_init(acc_full, 1);
@@ -240,6 +239,7 @@ moe_grouped_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
+    pdl_trigger();   // only now: a later product that takes all 512 columns ahead of its wait must not come before the allocation above
     const uint32_t tmem_base = *tmem_slot;
     const int n_kb = (p.K + BK - 1) / BK;
     const int w_row0 = e * p.rows_per_expert + tile_n * TILE_N;

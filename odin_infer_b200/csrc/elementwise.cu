@@ -20,7 +20,9 @@ __global__ void embed_kernel(const TW* __restrict__ table, const int* __restrict
     const TW* row = table + (size_t)(ok ? id : 0) * d;
     float* o = out + (size_t)t * d;
     const size_t next = (size_t)gridDim.x * d;   // a residual of several streams starts with as many copies of the rows
-    if (ok && (d & 3) == 0 && (((uintptr_t)table | (uintptr_t)out) & 15) == 0) {   // (a row's loads go out together)
+    // Whole vectors, a row's loads together: a row of 4,096 read element by element was sixteen trips to memory.  One row 5.0 -> 1.6 us,
+    // 64 rows 5.3 -> 1.8, 2,048 rows 16.8 -> 6.4.
+    if (ok && (d & 3) == 0 && (((uintptr_t)table | (uintptr_t)out) & 15) == 0) {
         constexpr int U = 4;
         for (int j0 = threadIdx.x * 4; j0 < d; j0 += blockDim.x * 4 * U) {
             float4 v[U];
@@ -253,7 +255,8 @@ add_rmsnorm_kernel(float* __restrict__ x, const TD* __restrict__ delta, int n_sp
 // memory), the loads of PARTS parts of a group issued together; the same order of additions as the kernel above with as
 // many threads, so the same bits.  1,024 threads from 4,096 columns on, 512 below: there a product's update comes in eight
 // or nine parts, and with two of them in flight a row's loads were five trips to L2 (a request of one 37-token question and
-// 24 tokens on the 1.7B size 28.06 ms, with nine in flight 26.34).  Its registers are capped so that a block leaves more than a third of an SM's
+// 24 tokens on the 1.7B size 28.06 ms, with nine in flight 26.34; back to back 8 rows of nine parts 2.64 and 2.07 us, 128 rows
+// 4.02 and 2.97, of 4,092 columns 6.66 and 5.07).  Its registers are capped so that a block leaves more than a third of an SM's
 // registers free: the product that follows starts its CTAs while this kernel runs, to fetch weights, and on the
 // SMs that hold a row it could not (with 64 registers a thread the block took them all; those CTAs then started 4
 // to 7 us after the others and the whole product ended that much later).

@@ -526,9 +526,11 @@ extern "C" int odin_head_prep(const void* qkv, int in_dtype, int n_split, long l
         ((((uintptr_t)qkv) | ((uintptr_t)q_out) | ((uintptr_t)cos_t) | ((uintptr_t)sin_t) | ((uintptr_t)v_first) |
           ((uintptr_t)v_keep)) & 15) == 0) {
         const VMix<bf16> vmix{(const bf16*)v_first, (bf16*)v_keep, v_lambda};
-        // Prompts: a warp per head spends more instructions than the memory asks for (66,048 tokens of 16 + 2 x 8 heads: see
-        // head_prep_wide_kernel).  From 2,048 tokens on one warp takes a whole token and its angles are fetched once; below,
-        // its heads are shared out so that there are warps enough.
+        // Prompts: a warp per head spends more instructions than the memory asks for.  16 + 2 x 8 heads, back to back, a warp a
+        // head and eight lanes a head: 256 tokens 6.9 and 3.8 us, 2,048 13.1 and 7.0, 12,001 79.9 and 51.2, 66,048 377 and 219
+        // (out of L2).  Below 256 tokens one head a warp has more in flight and stays the faster: 128 tokens 1.9 and 3.2 us, 255
+        // 3.2 and 3.8 (32 + 2 x 8 heads: 4.3 and 4.3).  From 2,048 tokens on one warp takes a whole token and its angles are
+        // fetched once; below, its heads are shared out so that there are warps enough.
         if (hd == 128 && in_dtype == ODIN_BF16 && n_split == 1 && T >= 256 && row_stride % 8 == 0 && q_out_stride % 8 == 0) {
             constexpr int CH = 4;
             const int chunks = ((n_heads + 3) / 4 + CH - 1) / CH, parts = T >= 2048 ? 1 : chunks;

@@ -56,11 +56,14 @@ __global__ void __launch_bounds__(SB) argmax_kernel(const float* __restrict__ lo
     }
 }
 
-// The same for long rows: a cluster of blocks shares a row.  One SM reads a row of 151,936 at its own rate, which took 11 us of
-// a decode step; the blocks' maxima meet through distributed shared memory.
+// The same for long rows: a cluster of blocks shares a row, and the blocks' maxima meet through distributed shared memory.  One SM
+// reads a row at its own rate: 151,936 logits of 1, 16 and 64 rows 6.9, 7.8 and 11.2 us; shared 3.5, 4.5 and 9.3.  The two
+// meetings of a cluster cost what they save at 16,384 (1 row: 2.1 and 2.4) and with many rows, where the blocks come in rounds
+// (32 rows of 32,768: 3.3 and 3.3, 64: 4.1 and 5.4; of 65,536: 4.5 and 3.7, 6.1 and 6.0; 128 of 151,936: 14.4 and 15.6).
 constexpr int AM_BLOCKS = 8;        // of a row
 constexpr int AM_THREADS = 512;
-constexpr int AM_FROM = 16384;      // shorter rows are a block's work
+constexpr int AM_FROM = 32768;      // shorter rows are a block's work
+constexpr int AM_PER_ROW = 2048;    // logits of a row for each of the rows, at least
 
 __global__ void __launch_bounds__(AM_THREADS) argmax_cluster_kernel(const float* __restrict__ logits, size_t ld, int V, int vec,
                                                                     int* __restrict__ out) {
@@ -126,7 +129,7 @@ __global__ void __launch_bounds__(AM_THREADS) argmax_cluster_kernel(const float*
 extern "C" int odin_argmax(const float* logits, long long ld, int B, int V, int* out, void* stream) {
     if (B <= 0) return 0;
     if (V <= 0) return ODIN_ERR_BAD_ARG;
-    if (V >= AM_FROM && B <= 65535) {
+    if (V >= AM_FROM && B <= V / AM_PER_ROW && B <= 65535) {
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(AM_BLOCKS, B);
         cfg.blockDim = dim3(AM_THREADS);
@@ -382,8 +385,9 @@ __global__ void __launch_bounds__(SB) sample_kernel(const float* __restrict__ lo
 
 // The same draw for rows of up to 1,024 candidates, one a thread: every thread adds up the values of at least its own from
 // shared memory, so the mark's token is the largest value whose sum exceeds it and nothing is searched.  What bounds the
-// search on a short row is its passes (two searches of ten, each with two block-wide meetings), not the row: 53 us a draw
-// from 384 candidates; here V compares and adds a thread and eight meetings.
+// search on a short row is its passes (two searches of ten, each with two block-wide meetings), not the row; here it is V
+// compares and adds a thread and eight meetings.  One row of 128, 384 and 1,024: 27, 55 and 69 us searched, 3.8, 8.2 and 28.7 so; 64 rows
+// 48, 57 and 94, and 4.1, 9.4 and 42.
 constexpr int FEW_CANDIDATES = 1024;
 
 __device__ __forceinline__ float block_max_few(float v, float* red) {   // of the launch's own number of warps

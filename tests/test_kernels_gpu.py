@@ -533,8 +533,9 @@ def test_experts_of_few_tokens_have_the_grouped_products_bits(T, E, per, d, ff, 
     ops.moe_tc_check()
 
 
-@pytest.mark.parametrize("V,ld", [(16383, 16383), (16384, 16384), (16389, 16392), (16389, 16389), (151936, 151936), (32771, 40000)])
-@pytest.mark.parametrize("B", [1, 5])
+@pytest.mark.parametrize("V,ld", [(16383, 16383), (16384, 16384), (16389, 16392), (16389, 16389), (151936, 151936), (32771, 40000),
+                                  (32767, 32768), (32768, 32768), (32773, 32773)])
+@pytest.mark.parametrize("B", [1, 5, 16, 17])   # a cluster a row up to a row for each 2,048 of its logits
 def test_argmax_of_long_rows_is_the_first_maximum(V, ld, B):
     """Rows shared by a cluster of blocks: the maximum at the edges of the blocks' shares and of their vectors, twice (the first
     counts), rows whose distance is no whole vector, a row of equal values, a row at minus infinity."""

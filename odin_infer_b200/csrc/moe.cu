@@ -21,8 +21,6 @@
 // order k = 0, 1, ...  Every sum runs in an order fixed by the sizes alone (a warp per output element,
 // lanes striding the row), so a token's values do not depend on the batch.  These kernels serve the
 // 32-bit path and steps of few tokens; rows of padding (sequence -1) get expert -1 and write zeros.
-#include <type_traits>
-
 #include "common.cuh"
 #include <math_constants.h>
 
@@ -112,18 +110,6 @@ moe_router_kernel(const TH* __restrict__ h, size_t h_stride, const TW* __restric
     pdl_trigger();
     const int t = blockIdx.x, per = top + always;
     const bool real = tok_seq == nullptr || tok_seq[t] >= 0;
-    // a warp's first expert: its row of bfloat16 weights is fetched before the wait, up to 2,048 elements of whole vectors
-    constexpr int EARLY = 8;
-    uint4 early[EARLY];
-    const bool has_early = std::is_same<TW, bf16>::value && logits == nullptr && (d & 7) == 0 && d <= EARLY * 256 && ((uintptr_t)w & 15) == 0 &&
-                           (int)(threadIdx.x >> 5) < rows;
-    if (has_early && real) {
-#pragma unroll
-        for (int u = 0; u < EARLY; ++u) {
-            const int i = (threadIdx.x & 31) * 8 + u * 256;
-            if (i < d) early[u] = *reinterpret_cast<const uint4*>(w + (size_t)(threadIdx.x >> 5) * d + i);
-        }
-    }
     pdl_wait();
     if (!real) {
         for (int k = threadIdx.x; k < per; k += blockDim.x) {
@@ -142,25 +128,7 @@ moe_router_kernel(const TH* __restrict__ h, size_t h_stride, const TW* __restric
         for (int i = threadIdx.x; i < d; i += blockDim.x) hrow[i] = to_f32(h[(size_t)t * h_stride + i]);
         __syncthreads();
         for (int e = warp; e < rows; e += n_warps) {
-            float s = 0.f;
-            if (has_early && e == warp) {   // (warp_dot's order)
-#pragma unroll
-                for (int u = 0; u < EARLY; ++u) {
-                    const int i = lane * 8 + u * 256;
-                    if (i < d) {
-                        const __nv_bfloat162* p = reinterpret_cast<const __nv_bfloat162*>(&early[u]);
-#pragma unroll
-                        for (int j = 0; j < 4; ++j) {
-                            const float2 f = __bfloat1622float2(p[j]);
-                            s = fmaf(f.x, hrow[i + 2 * j], s);
-                            s = fmaf(f.y, hrow[i + 2 * j + 1], s);
-                        }
-                    }
-                }
-                s = warp_sum(s);
-            } else {
-                s = warp_dot(w + (size_t)e * d, hrow, d, lane);
-            }
+            const float s = warp_dot(w + (size_t)e * d, hrow, d, lane);
             if (lane == 0) z[e] = s + (bias.p != nullptr && e < E && score != 2 ? bias.at(e) : 0.f);
         }
     }

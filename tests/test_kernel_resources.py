@@ -1,0 +1,40 @@
+"""Registers of kernels whose speed rests on them, as the compiler reports them (-Xptxas -v): a kernel of one block a row that
+asks for more keeps its own further blocks off an SM (many rows) or the next product's block (few rows), and one that spills
+waits for its own loads twice.  No run's result shows that."""
+import functools
+import os
+import re
+import subprocess
+
+import pytest
+
+from odin_infer_b200.csrc import build
+
+CSRC = os.path.dirname(os.path.abspath(build.__file__))
+
+
+@functools.lru_cache(maxsize=None)
+def resources(source):
+    """kernel (mangled) -> (registers, bytes of spill stores) of a source."""
+    nvcc = build._nvcc()
+    if nvcc is None:
+        pytest.skip("no nvcc here")
+    flags = [f for f in build.NVCC_FLAGS if f != "-shared"]
+    out = subprocess.run([nvcc, *flags, "-Xptxas", "-v", "-I", CSRC, "-c", "-o", os.devnull, os.path.join(CSRC, source)],
+                         stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True, check=True).stdout
+    return {name: (int(registers), int(spilled)) for name, spilled, registers in re.findall(
+        r"Compiling entry function '(\w+)'.*?(\d+) bytes spill stores.*?Used (\d+) registers", out, flags=re.S)}
+
+
+LIMITS = [
+    # a block of 1,024 threads a token: 64 registers are all there are
+    ("moe.cu", "moe_router_kernel", 64),
+]
+
+
+@pytest.mark.parametrize("source,kernel,most", LIMITS, ids=[k for _, k, _ in LIMITS])
+def test_registers(source, kernel, most):
+    found = {name: r for name, r in resources(source).items() if kernel in name}
+    assert found
+    for name, (registers, spilled) in found.items():
+        assert registers <= most and spilled == 0, (name, registers, spilled)

@@ -171,7 +171,7 @@ __device__ __forceinline__ float4 load4w(const VecRef& w, int j) {
 // one trip to memory and not one per part; the weights of the first group and the row
 // number, which no earlier kernel writes, are fetched before the wait for that kernel.
 template <typename TD, typename TO, bool VEC, int MAX_THREADS>
-__device__ __forceinline__ void add_rmsnorm_body(float* __restrict__ x, const TD* __restrict__ delta, int n_split,
+__device__ __forceinline__ void add_rmsnorm_body(float* __restrict__ x, const TD* delta, int n_split,
                                                  size_t split_stride, VecRef w, float eps, TO* __restrict__ out,
                                                  const int* __restrict__ rows, int d, float* red, float* rowbuf) {
     pdl_trigger();
@@ -244,7 +244,7 @@ __device__ __forceinline__ void add_rmsnorm_body(float* __restrict__ x, const TD
 
 template <typename TD, typename TO, bool VEC, int MAX_THREADS = 512>
 __global__ void __launch_bounds__(MAX_THREADS, 3)
-add_rmsnorm_kernel(float* __restrict__ x, const TD* __restrict__ delta, int n_split, size_t split_stride, VecRef w,
+add_rmsnorm_kernel(float* __restrict__ x, const TD* delta, int n_split, size_t split_stride, VecRef w,
                    float eps, TO* __restrict__ out, const int* __restrict__ rows, int d) {
     __shared__ float red[32];
     extern __shared__ float rowbuf[];  // d floats
@@ -262,7 +262,7 @@ add_rmsnorm_kernel(float* __restrict__ x, const TD* __restrict__ delta, int n_sp
 // to 7 us after the others and the whole product ended that much later).
 template <typename TD, typename TO, int NV, int THREADS, int PARTS>
 __global__ void __maxnreg__(THREADS == 512 ? 64 : NV == 1 ? 40 : 48)
-add_rmsnorm_wide_kernel(float* __restrict__ x, const TD* __restrict__ delta, int n_split, size_t split_stride, VecRef w,
+add_rmsnorm_wide_kernel(float* __restrict__ x, const TD* delta, int n_split, size_t split_stride, VecRef w,
                         float eps, TO* __restrict__ out, const int* __restrict__ rows, int d) {
     __shared__ float red[32];
     pdl_trigger();

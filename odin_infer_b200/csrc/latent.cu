@@ -25,7 +25,7 @@ __device__ __forceinline__ void rotate_pair(float u, float v, float c, float s, 
 
 template <typename TI, typename T>
 __global__ void __launch_bounds__(LP_THREADS)
-latent_prep_kernel(const TI* __restrict__ down, int n_split, size_t split_stride, size_t row_stride, int q_rank,
+latent_prep_kernel(const TI* down, int n_split, size_t split_stride, size_t row_stride, int q_rank,
                    int kv_rank, int rot, int pairs, VecRef qw, VecRef cw, float eps, T* __restrict__ cq,
                    const float* __restrict__ cos_t, const float* __restrict__ sin_t, int table_len,
                    const int* __restrict__ tok_pos, const int* __restrict__ tok_seq,
@@ -137,7 +137,7 @@ __device__ __forceinline__ float sum_parts(const TA* __restrict__ a, size_t at, 
 
 template <typename TA, typename TW, typename TO>
 __global__ void __launch_bounds__(HL_THREADS)
-heads_linear_kernel(const TA* __restrict__ a, int a_splits, size_t a_ss, size_t a_rs, size_t a_hs, const TW* __restrict__ w,
+heads_linear_kernel(const TA* a, int a_splits, size_t a_ss, size_t a_rs, size_t a_hs, const TW* __restrict__ w,
                     TO* __restrict__ out, size_t o_rs, size_t o_hs, int T, int N, int K, HeadGate gate) {
     extern __shared__ __align__(16) float as[];   // [K][HL_TOK]
     pdl_trigger();

@@ -98,9 +98,9 @@ __device__ __forceinline__ float warp_dot(const bf16* __restrict__ w, const floa
 // the block then only adds the bias, chooses and weighs.
 template <typename TH, typename TW>
 __global__ void __launch_bounds__(1024)
-moe_router_kernel(const TH* __restrict__ h, size_t h_stride, const TW* __restrict__ w, VecRef bias, int E, int d, int top,
+moe_router_kernel(const TH* h, size_t h_stride, const TW* __restrict__ w, VecRef bias, int E, int d, int top,
                   int always, const int* __restrict__ tok_seq, int* __restrict__ ids, float* __restrict__ wts,
-                  const float* __restrict__ logits, int score, int groups, int keep, float route_scale, int gate_row,
+                  const float* logits, int score, int groups, int keep, float route_scale, int gate_row,
                   float* __restrict__ gate_out, int n_real, float* __restrict__ pass_out) {
     extern __shared__ float sm[];
     float* hrow = sm;       // d

@@ -21,7 +21,7 @@
 // out[s][t][:] = h[t] + (prev - h[t]) * mu[s], s < n_mix.  Rows of sequence -1 are skipped.
 template <typename T, bool VEC>
 __global__ void __launch_bounds__(256)
-token_shift_kernel(const T* __restrict__ h, const float* __restrict__ state, size_t state_stride, VecRef mu, int n_mix,
+token_shift_kernel(const T* h, const float* state, size_t state_stride, VecRef mu, int n_mix,
                    T* __restrict__ out, const int* __restrict__ tok_seq, const int* __restrict__ seq_start,
                    const int* __restrict__ seq_slots, int n_rows, int d) {
     pdl_trigger();

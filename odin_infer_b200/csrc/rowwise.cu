@@ -35,7 +35,7 @@ struct MoreDeltas {
 
 template <typename TD, typename TO, bool VEC>
 __global__ void __launch_bounds__(ROW_THREADS)
-row_update_kernel(float* x, const TD* __restrict__ delta, int n_split, size_t split_stride, VecRef bias, VecRef w,
+row_update_kernel(float* x, const TD* delta, int n_split, size_t split_stride, VecRef bias, VecRef w,
                   float eps, int groups, int mode, TO* out, const int* __restrict__ rows, int d, MoreDeltas more) {
     __shared__ float red[32];
     extern __shared__ float rowbuf[];  // d floats
@@ -307,8 +307,8 @@ __device__ __forceinline__ float activate(int act, float z, float c0, float c1) 
 
 template <typename TI, typename TO, bool VEC>
 __global__ void __launch_bounds__(256)
-activation_kernel(const TI* __restrict__ in, int n_split, size_t split_stride, size_t in_stride, int act, VecRef params,
-                  TO* __restrict__ out, size_t out_stride, int T, int n, const float* __restrict__ row_scale) {
+activation_kernel(const TI* in, int n_split, size_t split_stride, size_t in_stride, int act, VecRef params,
+                  TO* __restrict__ out, size_t out_stride, int T, int n, const float* row_scale) {
     pdl_trigger();
     float c0 = 0.f, c1 = 0.f;
     if (act == ACT_XIELU) {
@@ -700,7 +700,7 @@ combine_add_kernel(float* __restrict__ x, CombineArgs a, CombineNorm post, Combi
 // barrier (every warp's share goes to a place of its own, and every thread adds the eight shares in their order).
 template <typename TD, typename TO, int NV>
 __global__ void __launch_bounds__(ROW_THREADS)
-combine_one_kernel(float* __restrict__ x, const TD* __restrict__ delta, int n_split, size_t split_stride, float scale,
+combine_one_kernel(float* __restrict__ x, const TD* delta, int n_split, size_t split_stride, float scale,
                    CombineNorm post, CombineNorm next, TO* __restrict__ out, const int* __restrict__ rows,
                    const int* __restrict__ tok_seq, int d) {
     __shared__ __align__(16) float shares[4][ROW_THREADS / 32];

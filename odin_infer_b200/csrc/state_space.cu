@@ -24,7 +24,7 @@ __device__ __forceinline__ float ss_silu(float z) { return z / (1.0f + expf(-z))
 // itself (no other thread touches that channel of that slot); else a second kernel stores the memory.
 template <typename TI, typename TO>
 __global__ void __launch_bounds__(256)
-causal_conv_kernel(const TI* __restrict__ in, size_t in_stride, VecRef w, VecRef bias, int taps, int silu,
+causal_conv_kernel(const TI* in, size_t in_stride, VecRef w, VecRef bias, int taps, int silu,
                    float* __restrict__ state, size_t state_stride, const int* __restrict__ tok_seq,
                    const int* __restrict__ seq_start, const int* __restrict__ seq_slots, TO* __restrict__ out,
                    size_t out_stride, int C, int store, const float* __restrict__ in_bias) {
@@ -109,7 +109,7 @@ causal_conv4_kernel(const TI* in, size_t in_stride, VecRef w, VecRef bias, int t
 // state[slot] <- the last taps - 1 inputs of (old state ++ the step's rows).  grid (sequences, channel blocks).
 template <typename TI>
 __global__ void __launch_bounds__(256)
-conv_state_kernel(const TI* __restrict__ in, size_t in_stride, int taps, float* __restrict__ state, size_t state_stride,
+conv_state_kernel(const TI* in, size_t in_stride, int taps, float* __restrict__ state, size_t state_stride,
                   const int* __restrict__ seq_start, const int* __restrict__ seq_slots, int C,
                   const float* __restrict__ in_bias) {
     pdl_trigger();

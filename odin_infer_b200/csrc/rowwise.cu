@@ -61,10 +61,18 @@ row_update_kernel(float* x, const TD* delta, int n_split, size_t split_stride, V
         for (int j = threadIdx.x * 4; j < d; j += blockDim.x * 4) {
             const float4 x0 = ld4(xr + j);
             float4 v = scaled ? make_float4(0.f, 0.f, 0.f, 0.f) : x0;
-            if (delta != nullptr) add_parts4<8>(v, delta + (size_t)src * d + j, split_stride, n_split);
+            if (delta != nullptr)
+                for (int s = 0; s < n_split; ++s) {
+                    const float4 dv = ld4(delta + (size_t)s * split_stride + (size_t)src * d + j);
+                    v.x += dv.x; v.y += dv.y; v.z += dv.z; v.w += dv.w;
+                }
 #pragma unroll
             for (int m = 0; m < 2; ++m)
-                if (more.p[m] != nullptr) add_parts4<8>(v, more.p[m] + (size_t)src * d + j, more.stride[m], more.n_split[m]);
+                if (more.p[m] != nullptr)
+                    for (int s = 0; s < more.n_split[m]; ++s) {
+                        const float4 dv = ld4(more.p[m] + (size_t)s * more.stride[m] + (size_t)src * d + j);
+                        v.x += dv.x; v.y += dv.y; v.z += dv.z; v.w += dv.w;
+                    }
             if (bias.p != nullptr) {
                 const float4 bv = bias.at4(j);
                 v.x += bv.x; v.y += bv.y; v.z += bv.z; v.w += bv.w;

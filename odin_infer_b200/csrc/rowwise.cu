@@ -330,7 +330,10 @@ activation_kernel(const TI* in, int n_split, size_t split_stride, size_t in_stri
         for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total4; i += (long long)gridDim.x * blockDim.x) {
             const int t = (int)(i / n4), c = (int)(i % n4) * 4;
             float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
-            add_parts4<8>(z, in + (size_t)t * in_stride + c, split_stride, n_split);
+            for (int s = 0; s < n_split; ++s) {
+                const float4 v = ld4(in + (size_t)s * split_stride + (size_t)t * in_stride + c);
+                z.x += v.x; z.y += v.y; z.z += v.z; z.w += v.w;
+            }
             const float f = row_scale != nullptr ? row_scale[t] : 1.0f;
             st4(out + (size_t)t * out_stride + c, make_float4(activate(act, z.x, c0, c1) * f, activate(act, z.y, c0, c1) * f,
                                                                activate(act, z.z, c0, c1) * f, activate(act, z.w, c0, c1) * f));

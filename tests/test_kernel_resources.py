@@ -31,6 +31,7 @@ LIMITS = [   # source, kernel, registers, bytes spilled
     ("moe.cu", "moe_router_kernel", 64, 0),
     # prompts: five blocks of 256 threads an SM
     ("rowwise.cu", "row_update_kernel", 48, 4),
+    ("rowwise.cu", "17activation_kernel", 40, 0),
 ]
 
 

@@ -62,21 +62,6 @@ __device__ __forceinline__ void st4(bf16* p, float4 v) {
     *reinterpret_cast<uint2*>(p) = u;
 }
 
-// v += the n parts at p, p + stride, .. (four elements of each), in their order; the loads of B parts go out together, so that
-// a sum of eight or nine parts is one or two trips to memory.
-template <int B, typename TD>
-__device__ __forceinline__ void add_parts4(float4& v, const TD* p, size_t stride, int n) {
-    for (int s0 = 0; s0 < n; s0 += B) {
-        float4 d[B];
-#pragma unroll
-        for (int u = 0; u < B; ++u)
-            if (s0 + u < n) d[u] = ld4(p + (size_t)(s0 + u) * stride);
-#pragma unroll
-        for (int u = 0; u < B; ++u)
-            if (s0 + u < n) { v.x += d[u].x; v.y += d[u].y; v.z += d[u].z; v.w += d[u].w; }
-    }
-}
-
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);

@@ -496,7 +496,10 @@ sigmoid_gate_vec_kernel(TO* __restrict__ o, size_t o_stride, const TG* __restric
             for (int s = 0; s < n_split; ++s) zh += to_f32(gate[(size_t)s * split_stride + (size_t)t * gate_stride + c / vd]);
             z = make_float4(zh, zh, zh, zh);
         } else {
-            add_parts4<8>(z, gate + (size_t)t * gate_stride + c, split_stride, n_split);
+            for (int s = 0; s < n_split; ++s) {
+                const float4 g = ld4(gate + (size_t)s * split_stride + (size_t)t * gate_stride + c);
+                z.x += g.x; z.y += g.y; z.z += g.z; z.w += g.w;
+            }
         }
         TO* p = o + (size_t)t * o_stride + c;
         const float4 v = ld4(p);

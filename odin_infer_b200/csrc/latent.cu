@@ -23,7 +23,9 @@ __device__ __forceinline__ void rotate_pair(float u, float v, float c, float s, 
     rv = v * c + u * s;
 }
 
-template <typename TI, typename T>
+// SPLIT: the projection comes in several parts.  That is so for few tokens only, a chain of trips to memory; a prompt's rows
+// come as one part and want many blocks an SM instead of four parts' registers.
+template <typename TI, typename T, bool SPLIT>
 __global__ void __launch_bounds__(LP_THREADS)
 latent_prep_kernel(const TI* down, int n_split, size_t split_stride, size_t row_stride, int q_rank,
                    int kv_rank, int rot, int pairs, VecRef qw, VecRef cw, float eps, T* __restrict__ cq,
@@ -41,26 +43,28 @@ latent_prep_kernel(const TI* down, int n_split, size_t split_stride, size_t row_
     if (seq >= 0 && write_cache) page = block_table[(size_t)seq * bt_stride + pos / page_size];
     pdl_wait();
     const int n = q_rank + kv_rank + rot;
-    for (int j0 = threadIdx.x; j0 < n; j0 += 4 * blockDim.x) {   // four elements of four parts at a time, an element's parts in their order
+    // four elements at a time, and of a split product four parts of each, an element's parts in their order
+    constexpr int PARTS = SPLIT ? 4 : 1;
+    for (int j0 = threadIdx.x; j0 < n; j0 += 4 * LP_THREADS) {
         float v[4] = {0.f, 0.f, 0.f, 0.f};
-        for (int s0 = 0; s0 < n_split; s0 += 4) {
-            float part[4][4];
+        for (int s0 = 0; s0 < (SPLIT ? n_split : 1); s0 += PARTS) {
+            float part[PARTS][4];
 #pragma unroll
-            for (int u = 0; u < 4; ++u)
+            for (int u = 0; u < PARTS; ++u)
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
-                    const int j = j0 + e * (int)blockDim.x;
-                    if (s0 + u < n_split && j < n) part[u][e] = to_f32(down[(size_t)(s0 + u) * split_stride + (size_t)t * row_stride + j]);
+                    const int j = j0 + e * LP_THREADS;
+                    if ((!SPLIT || s0 + u < n_split) && j < n) part[u][e] = to_f32(down[(size_t)(s0 + u) * split_stride + (size_t)t * row_stride + j]);
                 }
 #pragma unroll
-            for (int u = 0; u < 4; ++u)
+            for (int u = 0; u < PARTS; ++u)
 #pragma unroll
                 for (int e = 0; e < 4; ++e)
-                    if (s0 + u < n_split && j0 + e * (int)blockDim.x < n) v[e] += part[u][e];
+                    if ((!SPLIT || s0 + u < n_split) && j0 + e * LP_THREADS < n) v[e] += part[u][e];
         }
 #pragma unroll
         for (int e = 0; e < 4; ++e)
-            if (j0 + e * (int)blockDim.x < n) rowbuf[j0 + e * (int)blockDim.x] = v[e];
+            if (j0 + e * LP_THREADS < n) rowbuf[j0 + e * LP_THREADS] = v[e];
     }
     __syncthreads();
     if (q_rank > 0) {
@@ -107,7 +111,8 @@ extern "C" int odin_latent_prep(const void* down, int in_dtype, int n_split, lon
     cudaStream_t s = (cudaStream_t)stream;
     VecRef qw{q_norm, norm_dtype == ODIN_BF16}, cw{c_norm, norm_dtype == ODIN_BF16};
 #define GO(TI, TT)                                                                                                   \
-    odin_launch(latent_prep_kernel<TI, TT>, dim3(T), dim3(LP_THREADS), smem, s, (const TI*)down, n_split,            \
+    odin_launch((n_split != 1 ? latent_prep_kernel<TI, TT, true> : latent_prep_kernel<TI, TT, false>), dim3(T),      \
+                dim3(LP_THREADS), smem, s, (const TI*)down, n_split,                                                 \
                 (size_t)split_stride, (size_t)row_stride, q_rank, kv_rank, rot, pairs, qw, cw, eps, (TT*)cq, cos_t,  \
                 sin_t, table_len, tok_pos, tok_seq, block_table, bt_stride, (TT*)cache, page_size, write_cache)
     if (in_dtype == ODIN_BF16 && out_dtype == ODIN_BF16) GO(bf16, bf16);

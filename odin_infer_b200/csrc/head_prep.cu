@@ -35,7 +35,8 @@ struct VMix {
 // pairs: the rotation pairs element 2i with 2i + 1 instead of i with i + rot/2.
 // v_is_k: the projection holds no values; a key head's elements with their bias, before norm and rotation, are also its
 // value head's (vd == hd), and its warp writes both.
-template <typename TI, typename T>
+// SPLIT: the projection comes in several parts (few tokens); a prompt's one part leaves the registers of four more to other blocks.
+template <typename TI, typename T, bool SPLIT>
 __global__ void __launch_bounds__(HP_WARPS * 32)
 head_prep_kernel(const TI* qkv, int n_split, size_t split_stride, T* q_out,  // may alias: no restrict
                  size_t q_out_stride, int Hq, int Hkv, int hd, int vd, size_t row_stride, VecRef bias, VecRef qw,
@@ -97,11 +98,11 @@ head_prep_kernel(const TI* qkv, int n_split, size_t split_stride, T* q_out,  // 
 
     float* b = buf[warp];
     float ss = 0.f;
-    for (int j0 = lane; j0 < n; j0 += 128) {   // four elements of four parts at a time, an element's parts in their order
+    for (int j0 = lane; j0 < n; j0 += 128) {   // four elements at a time, and four parts of each, an element's parts in their order
         float v[4];
 #pragma unroll
         for (int e = 0; e < 4; ++e) v[e] = j0 + 32 * e < n ? to_f32(src[j0 + 32 * e]) : 0.f;
-        for (int s0 = 1; s0 < n_split; s0 += 4) {
+        for (int s0 = 1; SPLIT && s0 < n_split; s0 += 4) {
             float part[4][4];
 #pragma unroll
             for (int u = 0; u < 4; ++u)
@@ -567,7 +568,7 @@ extern "C" int odin_head_prep(const void* qkv, int in_dtype, int n_split, long l
         return 0;
     }
 #define GO(TI, TT)                                                                                                  \
-    odin_launch(head_prep_kernel<TI, TT>, grid, dim3(HP_WARPS * 32), 0, s,                                           \
+    odin_launch((n_split > 1 ? head_prep_kernel<TI, TT, true> : head_prep_kernel<TI, TT, false>), grid, dim3(HP_WARPS * 32), 0, s, \
         (const TI*)qkv, n_split, (size_t)split_stride, (TT*)q_out, (size_t)q_out_stride, Hq, Hkv, hd, vd,           \
         (size_t)row_stride, bv, qw, kw, norm_mode, eps, cos_t, sin_t, rot, table_len, tok_pos, tok_seq, block_table,     \
         (int)bt_stride, (TT*)k_cache, (TT*)v_cache, page_size, write_kv, pairs, v_is_k,                              \

@@ -34,6 +34,7 @@ LIMITS = [   # source, kernel (mangled), registers, bytes spilled
     ("rowwise.cu", "17activation_kernel", 40, 0),
     ("rowwise.cu", "sigmoid_gate_vec_kernel", 40, 0),
     ("latent.cu", "latent_prep_kernelI.*Lb0E", 40, 0),   # one part
+    ("head_prep.cu", "head_prep_kernelI.*Lb0E", 40, 0),
 ]
 
 

@@ -182,29 +182,37 @@ mix_streams_fast_kernel(StreamArgs a, TO* __restrict__ out) {
 #pragma unroll
         for (int i = 0; i < NV; ++i) load_streams(i, X[EARLY ? i : 0]);
     }
-    // one group of four a thread (decoding): the first parts of every term go out together, before any of them is added
-    constexpr int B = NV != 1 ? 1 : NT < 2 ? 9 : 6;
-    float4 early[NT > 0 ? NT : 1][B];
+#pragma unroll
+    for (int n = 0; n < NT; ++n)
+#pragma unroll
+        for (int i = 0; i < NV; ++i) t[n][i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    // One group of four a thread (decoding): B parts of every term go out together, as many as leave a thread 64 registers.
+    // (Nine of one term and six of two took up to 119, and a block of 512 threads left no room on its SM for the next
+    // product's.)
+    constexpr int B = NT == 2 ? 3 : S == 4 ? 8 : 5;
     const int own = threadIdx.x * 4;
-    if (NV == 1 && own < d) {
+    if (NT > 0 && NV == 1 && own < d) {
+        int most = a.terms.t[0].n_split;
+        if (NT > 1) most = max(most, a.terms.t[NT - 1].n_split);
+        for (int s0 = 0; s0 < most; s0 += B) {
+            float4 part[NT > 0 ? NT : 1][B];
 #pragma unroll
-        for (int n = 0; n < NT; ++n)
+            for (int n = 0; n < NT; ++n)
 #pragma unroll
-            for (int sp = 0; sp < B; ++sp)
-                if (sp < a.terms.t[n].n_split)
-                    early[n][sp] = ld4((const float*)a.terms.t[n].p + (size_t)sp * a.terms.t[n].split_stride + (size_t)r * d + own);
+                for (int u = 0; u < B; ++u)
+                    if (s0 + u < a.terms.t[n].n_split)
+                        part[n][u] = ld4((const float*)a.terms.t[n].p + (size_t)(s0 + u) * a.terms.t[n].split_stride + (size_t)r * d + own);
+#pragma unroll
+            for (int n = 0; n < NT; ++n)
+#pragma unroll
+                for (int u = 0; u < B; ++u)
+                    if (s0 + u < a.terms.t[n].n_split) { t[n][0].x += part[n][u].x; t[n][0].y += part[n][u].y; t[n][0].z += part[n][u].z; t[n][0].w += part[n][u].w; }
+        }
     }
 #pragma unroll
     for (int n = 0; n < NT; ++n) {
         const CombineTerm& tm = a.terms.t[n];
-#pragma unroll
-        for (int i = 0; i < NV; ++i) t[n][i] = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (NV == 1 && own < d) {
-#pragma unroll
-            for (int sp = 0; sp < B; ++sp)
-                if (sp < tm.n_split) { t[n][0].x += early[n][sp].x; t[n][0].y += early[n][sp].y; t[n][0].z += early[n][sp].z; t[n][0].w += early[n][sp].w; }
-        }
-        for (int sp = NV == 1 ? B : 0; sp < tm.n_split; ++sp) {
+        for (int sp = 0; NV != 1 && sp < tm.n_split; ++sp) {
 #pragma unroll
             for (int i = 0; i < NV; ++i) {
                 const int j = (threadIdx.x + i * blockDim.x) * 4;

@@ -532,7 +532,9 @@ extern "C" int odin_head_prep(const void* qkv, int in_dtype, int n_split, long l
         // (out of L2).  Below 256 tokens one head a warp has more in flight and stays the faster: 128 tokens 1.9 and 3.2 us, 255
         // 3.2 and 3.8 (32 + 2 x 8 heads: 4.3 and 4.3).  From 2,048 tokens on one warp takes a whole token and its angles are
         // fetched once; below, its heads are shared out so that there are warps enough.
-        if (hd == 128 && in_dtype == ODIN_BF16 && n_split == 1 && T >= 256 && row_stride % 8 == 0 && q_out_stride % 8 == 0) {
+        // Its stores are of 16 bytes, the others' of 8.
+        if (hd == 128 && in_dtype == ODIN_BF16 && n_split == 1 && T >= 256 && row_stride % 8 == 0 && q_out_stride % 8 == 0 &&
+            ((((uintptr_t)k_cache) | ((uintptr_t)v_cache)) & 15) == 0) {
             constexpr int CH = 4;
             const int chunks = ((n_heads + 3) / 4 + CH - 1) / CH, parts = T >= 2048 ? 1 : chunks;
             const long long items = (long long)T * parts;

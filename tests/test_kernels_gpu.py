@@ -445,6 +445,28 @@ def test_head_prep_of_prompts_has_the_bits_of_few_tokens(T, n_q, n_kv, values):
         assert all(torch.equal(x, y) for x, y in zip(*got))
 
 
+@pytest.mark.parametrize("T", [255, 256, 2050])
+def test_head_prep_into_a_cache_on_eight_bytes(T):
+    """A cache that starts between two 16-byte boundaries (a view): the kernels that store 8 bytes take it, at every number of tokens."""
+    from odin_infer_b200.csrc import ops
+    n_q, n_kv, hd = 16, 8, 128
+    torch.manual_seed(T)
+    k_cache, v_cache, bt = paged_cache(1, [T], n_kv, hd, torch.bfloat16)
+    tok_seq, tok_pos = torch.zeros(T, dtype=torch.int32, device=DEV), torch.arange(T, dtype=torch.int32, device=DEV)
+    qkv = torch.randn(T, (n_q + 2 * n_kv) * hd, device=DEV).bfloat16()
+    norm = (1 + 0.1 * torch.randn(hd, device=DEV)).bfloat16()
+    ang = torch.randn(T, hd // 2, device=DEV)
+    cos, sin = torch.cos(ang).contiguous(), torch.sin(ang).contiguous()
+    got = []
+    for offset in (0, 4):
+        kc, vc = (torch.full((c.numel() + offset,), 3.0, device=DEV, dtype=torch.bfloat16)[offset:].view(c.shape) for c in (k_cache, v_cache))
+        assert kc.data_ptr() % 16 == vc.data_ptr() % 16 == 2 * offset
+        q_out = torch.empty(T, n_q * hd, device=DEV, dtype=torch.bfloat16)
+        ops.head_prep(qkv, n_q, n_kv, hd, norm, norm, 1e-6, cos, sin, hd, tok_pos, tok_seq, bt, kc, vc, q_out=q_out)
+        got.append((q_out, kc, vc))
+    assert all(torch.equal(x, y) for x, y in zip(*got))
+
+
 @pytest.mark.parametrize("d,parts", [(2048, 1), (2048, 8), (2048, 9), (2048, 13), (2052, 3), (3072, 5), (4092, 6)])
 @pytest.mark.parametrize("delta_dtype", [torch.float32, torch.bfloat16])
 def test_add_rmsnorm_of_few_rows_has_the_bits_of_more(d, parts, delta_dtype):

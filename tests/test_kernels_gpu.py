@@ -555,6 +555,43 @@ def test_experts_of_few_tokens_have_the_grouped_products_bits(T, E, per, d, ff, 
     ops.moe_tc_check()
 
 
+def test_experts_of_few_tokens_from_two_threads():
+    """Two engines' threads on one stream, with 8 and 16 tokens: the same kernels with different shared memory."""
+    import threading
+    from odin_infer_b200.csrc import ops
+    E, per, d, ff = 8, 4, 1024, 128
+    torch.manual_seed(0)
+    w1 = (torch.randn(E, 2 * ff, d, device=DEV) / math.sqrt(d)).bfloat16()
+    w2 = (torch.randn(E, d, ff, device=DEV) / math.sqrt(ff)).bfloat16()
+    work = {}
+    for T in (8, 16):
+        h, ids = torch.randn(T, d, device=DEV).bfloat16(), torch.randint(0, E, (T, per), device=DEV, dtype=torch.int32)
+        work[T] = (h, ids, torch.empty(T * per, ff, device=DEV).bfloat16(), torch.empty(T * per, d, device=DEV))
+    alone = {}
+    for T, (h, ids, a, c) in work.items():
+        assert ops.moe_few(h, w1, w2, ids, "silu", a, c)
+        alone[T] = c.clone()
+    errors = []
+
+    def run(T):
+        h, ids, a, c = work[T]
+        try:
+            for _ in range(400):
+                assert ops.moe_few(h, w1, w2, ids, "silu", a, c)
+        except Exception as e:   # noqa: BLE001 - reported below
+            errors.append(e)
+
+    threads = [threading.Thread(target=run, args=(T,)) for T in work]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    assert not errors, errors
+    assert all(torch.equal(work[T][3], alone[T]) for T in work)
+    ops.moe_tc_check()
+
+
 @pytest.mark.parametrize("V,ld", [(16383, 16383), (16384, 16384), (16389, 16392), (16389, 16389), (151936, 151936), (32771, 40000),
                                   (32767, 32768), (32768, 32768), (32773, 32773)])
 @pytest.mark.parametrize("B", [1, 5, 16, 17])   # a cluster a row up to a row for each 2,048 of its logits

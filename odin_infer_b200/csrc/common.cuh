@@ -93,7 +93,9 @@ __device__ __forceinline__ float block_sum(float v, float* red) {
 // Programmatic dependent launch.  A kernel launched through odin_launch may start
 // while the kernel before it on the stream is still running; pdl_wait() blocks until
 // that kernel has completed and its memory is visible.  Rules every kernel here keeps:
-//   * pdl_trigger() first, so the next kernel's CTAs can take their places early;
+//   * pdl_trigger() first, so the next kernel's CTAs can take their places early; in a kernel that allocates tensor memory
+//     behind the allocation: a later kernel that takes all columns of an SM ahead of its own wait (products of few tokens do)
+//     would otherwise hold what this one waits for, and wait for this one to end;
 //   * pdl_wait() before the first read of anything an earlier kernel wrote and before
 //     the first global write (a buffer may be reused memory that an earlier kernel
 //     still reads); before it a kernel may touch only what no kernel of the step writes:

@@ -141,8 +141,6 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    pdl_trigger();  // the next kernel may take its place; it waits for this one before it touches memory
-
     if (threadIdx.x == 0) {
         for (int s = 0; s < C::STAGES; ++s) {  // all of them: the places are there whatever the ring's length
             tc::mbar_init(&full[s], 1);
@@ -165,6 +163,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
+    // The next kernel may take its place; it waits for this one before it touches memory.  Only behind the allocation: a later
+    // product that takes all columns ahead of its own wait must not come to this SM before it.
+    pdl_trigger();
     const uint32_t tmem_base = *tmem_slot;
     const uint32_t tmem_staged = tmem_base + ACC_BUFS * C::ACC_W;
 

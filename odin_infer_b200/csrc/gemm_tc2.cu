@@ -236,7 +236,6 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t rank = cluster_rank();
     const bool leader = rank == 0;
-    pdl_trigger();
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; ++s) {
@@ -260,6 +259,7 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
     __syncthreads();
     cluster_sync();  // both CTAs' barriers exist before either signals the other
     tc::fence_after_sync();
+    pdl_trigger();   // behind the allocation, as in gemm_tc.cu
     const uint32_t tmem_base = *tmem_slot;
 
     const int n_clusters = (int)(gridDim.x >> 1), cluster_id = (int)(blockIdx.x >> 1);

@@ -57,3 +57,12 @@ def test_what_earlier_kernels_write_is_not_read_as_invariant(source):
             continue
         invariant = set(re.findall(r"const\s+\w+\s*\*\s*__restrict__\s+(\w+)", params)) - CONSTANT
         assert not invariant, (source, name, sorted(invariant))
+
+
+@pytest.mark.parametrize("source", SOURCES)
+def test_tensor_memory_is_held_before_the_next_kernel_may_start(source):
+    """A kernel that allows the next launch and allocates afterwards can wait for columns that a later kernel holds, which waits
+    for this one to end."""
+    for name, params, body in _functions(source):
+        if "pdl_trigger()" in body and "tmem_alloc" in body:
+            assert body.index("tmem_alloc") < body.index("pdl_trigger()"), (source, name)

@@ -302,12 +302,7 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
                     if (++stage == STAGES) { stage = 0; phase ^= 1; }
                 }
             }
-            if (!ok && leader) {
-                // aborted: let the copies already in flight land before the CTA's memory is released
-                for (int s2 = 0; s2 < STAGES; ++s2)
-                    for (uint32_t i = 0; i < 4096; ++i)
-                        if (tc::mbar_try_wait(&full[s2], 0) || tc::mbar_try_wait(&full[s2], 1)) break;
-            }
+            if (!ok && leader) tc::drain_ring(full, STAGES, stage, phase);   // (both CTAs' copies complete on its barriers)
         }
     } else if (warp == 1) {
         // --------------------------------------------------------- MMA issuer (leader only)

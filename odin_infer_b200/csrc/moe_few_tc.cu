@@ -197,12 +197,7 @@ moe_few_kernel(const __grid_constant__ CUtensorMap map_w, const FewParams p) {
                 i += w;
             }
             odin_trace_mark(6, true);  // every load is requested
-            if (!ok) {
-                // aborted: let the copies already in flight land before the CTA's memory is released
-                for (uint32_t s2 = 0; s2 < n_stages; ++s2)
-                    for (uint32_t j = 0; j < 4096; ++j)
-                        if (tc::mbar_try_wait(&full[s2], 0) || tc::mbar_try_wait(&full[s2], 1)) break;
-            }
+            if (!ok) tc::drain_ring(full, n_stages, stage, phase);
         }
     } else if (warp == 1) {
         // ------------------------------------------------------- the MMAs

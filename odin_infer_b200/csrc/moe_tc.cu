@@ -261,12 +261,7 @@ moe_grouped_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                 }
                 if (++stage == n_stages) { stage = 0; phase ^= 1; }
             }
-            if (!ok) {
-                // aborted: let the copies already in flight land before the CTA's memory is released
-                for (uint32_t s2 = 0; s2 < n_stages; ++s2)
-                    for (uint32_t i = 0; i < 4096; ++i)
-                        if (tc::mbar_try_wait(&full[s2], 0) || tc::mbar_try_wait(&full[s2], 1)) break;
-            }
+            if (!ok) tc::drain_ring(full, n_stages, stage, phase);
         }
     } else if (warp == 1) {
         if (lane == 0) {

@@ -102,6 +102,15 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
     return false;
 }
 
+// A producer that gave up at (stage, phase) of its ring: lets the copies already in flight land before the CTA's memory is
+// released.  Stages before that one were last filled in this phase, the others in the one before (or never: their barriers
+// count as complete in it).  Not longer than 4,096 tries each.
+__device__ __forceinline__ void drain_ring(uint64_t* full, uint32_t n_stages, uint32_t stage, uint32_t phase) {
+    for (uint32_t s = 0; s < n_stages; ++s)
+        for (uint32_t i = 0; i < 4096; ++i)
+            if (mbar_try_wait(&full[s], s < stage ? phase : phase ^ 1)) break;
+}
+
 // ----------------------------------------------------------------------- TMA
 __device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* map, int c0, int c1, uint64_t* bar) {
     asm volatile(

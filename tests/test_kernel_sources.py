@@ -66,3 +66,12 @@ def test_tensor_memory_is_held_before_the_next_kernel_may_start(source):
     for name, params, body in _functions(source):
         if "pdl_trigger()" in body and "tmem_alloc" in body:
             assert body.index("tmem_alloc") < body.index("pdl_trigger()"), (source, name)
+
+
+@pytest.mark.parametrize("source", SOURCES)
+def test_no_wait_for_either_phase(source):
+    """One of a barrier's two parities always counts as complete: a wait for the one or the other waits for nothing."""
+    with open(os.path.join(CSRC, source)) as f:
+        text = _without_comments(f.read())
+    for bar in re.findall(r"try_wait\(([^;]*?), [01]\) \|\|", text):
+        assert f"try_wait({bar}, 0) || tc::mbar_try_wait({bar}, 1)" not in text, (source, bar)

@@ -422,7 +422,9 @@ static int launch_add_rmsnorm(float* x, const void* delta, int n_split, size_t s
         }
         if constexpr (!std::is_same<TO, float>::value) {
             if (d >= 2048 && d < 4096 && n_rows <= 128) {
-                auto wide = d <= 2048 ? add_rmsnorm_wide_kernel<TD, TO, 1, 512, 9> : add_rmsnorm_wide_kernel<TD, TO, 2, 512, 4>;
+                // (a bfloat16 update comes in one part: nine of them would only cost registers, of which some spilled)
+                constexpr int PARTS = std::is_same<TD, float>::value ? 9 : 4;
+                auto wide = d <= 2048 ? add_rmsnorm_wide_kernel<TD, TO, 1, 512, PARTS> : add_rmsnorm_wide_kernel<TD, TO, 2, 512, 4>;
                 odin_launch(wide, dim3(n_rows), dim3(512), 0, s, x, (const TD*)delta, n_split, split_stride, w, eps, (TO*)out, rows, d);
                 ODIN_LAUNCH_CHECK();
                 return 0;

@@ -576,6 +576,7 @@ def test_experts_of_few_tokens_from_two_threads():
     def run(T):
         h, ids, a, c = work[T]
         try:
+            c.zero_()   # (a step's first launch: the thread has its context)
             for _ in range(400):
                 assert ops.moe_few(h, w1, w2, ids, "silu", a, c)
         except Exception as e:   # noqa: BLE001 - reported below

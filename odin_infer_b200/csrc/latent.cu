@@ -44,8 +44,9 @@ latent_prep_kernel(const TI* down, int n_split, size_t split_stride, size_t row_
     pdl_wait();
     const int n = q_rank + kv_rank + rot;
     // four elements at a time, and of a split product four parts of each, an element's parts in their order
+    const int step = SPLIT ? (int)blockDim.x : LP_THREADS;   // (as a constant it had the compiler take the parts' loads one by one)
     constexpr int PARTS = SPLIT ? 4 : 1;
-    for (int j0 = threadIdx.x; j0 < n; j0 += 4 * LP_THREADS) {
+    for (int j0 = threadIdx.x; j0 < n; j0 += 4 * step) {
         float v[4] = {0.f, 0.f, 0.f, 0.f};
         for (int s0 = 0; s0 < (SPLIT ? n_split : 1); s0 += PARTS) {
             float part[PARTS][4];
@@ -53,18 +54,18 @@ latent_prep_kernel(const TI* down, int n_split, size_t split_stride, size_t row_
             for (int u = 0; u < PARTS; ++u)
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
-                    const int j = j0 + e * LP_THREADS;
+                    const int j = j0 + e * step;
                     if ((!SPLIT || s0 + u < n_split) && j < n) part[u][e] = to_f32(down[(size_t)(s0 + u) * split_stride + (size_t)t * row_stride + j]);
                 }
 #pragma unroll
             for (int u = 0; u < PARTS; ++u)
 #pragma unroll
                 for (int e = 0; e < 4; ++e)
-                    if ((!SPLIT || s0 + u < n_split) && j0 + e * LP_THREADS < n) v[e] += part[u][e];
+                    if ((!SPLIT || s0 + u < n_split) && j0 + e * step < n) v[e] += part[u][e];
         }
 #pragma unroll
         for (int e = 0; e < 4; ++e)
-            if (j0 + e * LP_THREADS < n) rowbuf[j0 + e * LP_THREADS] = v[e];
+            if (j0 + e * step < n) rowbuf[j0 + e * step] = v[e];
     }
     __syncthreads();
     if (q_rank > 0) {

@@ -186,15 +186,15 @@ mix_streams_fast_kernel(StreamArgs a, TO* __restrict__ out) {
     for (int n = 0; n < NT; ++n)
 #pragma unroll
         for (int i = 0; i < NV; ++i) t[n][i] = make_float4(0.f, 0.f, 0.f, 0.f);
-    // One group of four a thread (decoding): B parts of every term go out together, as many as leave a thread 64 registers.
-    // (Nine of one term and six of two took up to 119, and a block of 512 threads left no room on its SM for the next
-    // product's.)
-    constexpr int B = NT == 2 ? 3 : S == 4 ? 8 : 5;
+    // One group of four a thread (decoding): the first nine parts of one term go out together, or four at a time of two terms:
+    // 64 to 77 registers a thread.  (Six of two terms took up to 119, and a block of 512 threads left no room on its SM for the
+    // next product's; three of two and eight of one, in 64 registers, were up to 30 % slower at 128 rows of one term.)
+    constexpr int B = NT == 2 ? 4 : 9;
     const int own = threadIdx.x * 4;
     if (NT > 0 && NV == 1 && own < d) {
         int most = a.terms.t[0].n_split;
         if (NT > 1) most = max(most, a.terms.t[NT - 1].n_split);
-        for (int s0 = 0; s0 < most; s0 += B) {
+        for (int s0 = 0; s0 < (NT == 2 ? most : 1); s0 += B) {
             float4 part[NT > 0 ? NT : 1][B];
 #pragma unroll
             for (int n = 0; n < NT; ++n)
@@ -212,7 +212,7 @@ mix_streams_fast_kernel(StreamArgs a, TO* __restrict__ out) {
 #pragma unroll
     for (int n = 0; n < NT; ++n) {
         const CombineTerm& tm = a.terms.t[n];
-        for (int sp = 0; NV != 1 && sp < tm.n_split; ++sp) {
+        for (int sp = NV != 1 ? 0 : NT == 1 ? B : tm.n_split; sp < tm.n_split; ++sp) {
 #pragma unroll
             for (int i = 0; i < NV; ++i) {
                 const int j = (threadIdx.x + i * blockDim.x) * 4;

@@ -36,8 +36,8 @@ LIMITS = [   # source, kernel (mangled), registers, bytes spilled
     ("latent.cu", "latent_prep_kernelI.*Lb0E", 40, 0),   # one part
     ("head_prep.cu", "head_prep_kernelI.*Lb0E", 40, 0),
     ("elementwise.cu", "add_rmsnorm_wide_kernel", 64, 0),
-    # a decode step's rows, a block of 512 threads each: half of an SM's registers for the next product's block
-    ("streams.cu", r"mix_streams_fast_kernelILi\dELi\dELi1E", 64, 0),
+    # a decode step's rows, a block of 512 threads each: beside it the next product's block wants 14 k of the SM's 64 k registers
+    ("streams.cu", r"mix_streams_fast_kernelILi\dELi\dELi1E", 80, 0),
 ]
 
 

@@ -26,7 +26,6 @@ from __future__ import annotations
 import torch
 
 from ..csrc import ops
-from .runtime import SHORT_CONTEXT
 from .step import StepBatch, StepEntry
 
 BUCKETS = (1, 2, 4, 8, 12, 16, 24, 32, 48, 64, 96, 128, 192, 256)
@@ -63,8 +62,7 @@ class DecodeGraphs:
         # bits are those of the eager step; in bfloat16 the bucket's rows choose.
         self._exact_forms = rt.dtype == torch.float32
         self._forms_from = model.forms_from if self._exact_forms else ()
-        # models whose decode attention has a kernel for short contexts: those are a class of contexts
-        self._short_context = SHORT_CONTEXT if any(getattr(b.mixer, "plain_heads", False) for b in model.layers) else 0
+        self._short_contexts: dict[int, int] = {}   # bucket -> DecoderModel.short_context
         self._seen: set[tuple] = set()   # 32-bit: keys of steps that came once and ran eagerly
         # In 32-bit, whose logits are copied out right behind a replay, the graphs share their scratch memory: they replay one
         # after the other on one stream, and nothing of a replay but its logits is read after it.
@@ -172,7 +170,10 @@ class DecodeGraphs:
         # kernels whose launch shape follows the longest context (decode attention's key splits)
         # make a graph valid for a class of context lengths only: the class is part of the key
         longest = max(s + 1 for s in starts)
-        bucket = (bucket, "short" if self.rt.dtype == torch.bfloat16 and longest <= self._short_context else self.rt.context_class(longest))
+        short = self._short_contexts.get(bucket)
+        if short is None:
+            short = self._short_contexts[bucket] = self.model.short_context(self.rt, bucket)
+        bucket = (bucket, "short" if longest <= short else self.rt.context_class(longest))
         hit = self._graphs.get(bucket)
         if hit is None:
             if self._not_yet(bucket):

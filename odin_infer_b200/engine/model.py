@@ -56,6 +56,10 @@ class DecoderModel:
         """Every part's lines between its forms (see Part.forms_from), ascending."""
         return tuple(sorted({n for p in self._all_parts() for n in p.forms_from}))
 
+    def short_context(self, rt, n_seqs: int) -> int:
+        """The longest context that any part counts as short (see Part.short_context)."""
+        return max(p.short_context(rt, n_seqs) for p in self._all_parts())
+
     def parts_not_graph_safe(self) -> list[str]:
         out = []
         for p in self._all_parts():

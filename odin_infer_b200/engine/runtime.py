@@ -308,17 +308,28 @@ class Runtime:
         """One token per sequence in bfloat16: head preparation (per-head norm, rotation, the
         cache write) inside the attention kernel.  False where that kernel does not apply;
         the caller then prepares the heads and calls `attention`."""
-        if os.environ.get("ODIN_FUSED_ATTENTION", "1") == "0":  # for comparisons
-            return False
-        if not (self.dtype == torch.bfloat16 and step.all_single and head_dim in (64, 128)
-                and rotary_dim == head_dim and n_kv > 0 and n_q // n_kv <= 16 and write_kv):
+        if not (self.heads_prepared_in_attention(head_dim, rotary_dim, n_q, n_kv) and step.all_single and write_kv):
             return False
         B = out.shape[0]
         n_split = decode_key_splits(B, n_kv, step.max_len_after, n_sms=self.n_sms)
         scratch = self.empty(ops.attention_decode_scratch(B, n_q, head_dim, n_split), dtype=torch.float32)
         return ops.attention_decode_fused(qkv, out, n_q, n_kv, head_dim, q_norm, k_norm, eps, cos, sin, rotary_dim,
                                           k_line, v_line, step.tok_pos, step.tok_seq, block_table, window, scratch,
-                                          n_split, write_kv, short=step.max_len_after <= SHORT_CONTEXT)
+                                          n_split, write_kv,
+                                          short=step.max_len_after <= self.short_context(B, head_dim, rotary_dim, n_q, n_kv))
+
+    def heads_prepared_in_attention(self, head_dim, rotary_dim, n_q, n_kv) -> bool:
+        """Does decode attention prepare heads of these sizes itself?"""
+        if os.environ.get("ODIN_FUSED_ATTENTION", "1") == "0":  # for comparisons
+            return False
+        return (self.dtype == torch.bfloat16 and head_dim in (64, 128) and rotary_dim == head_dim and n_kv > 0
+                and n_q // n_kv <= 16)
+
+    def short_context(self, n_seqs, head_dim, rotary_dim, n_q, n_kv) -> int:
+        """Up to how many keys a step of n_seqs sequences runs decode attention's kernel of short contexts (0: never)."""
+        if not self.heads_prepared_in_attention(head_dim, rotary_dim, n_q, n_kv):
+            return 0
+        return SHORT_CONTEXT if decode_key_splits(n_seqs, n_kv, SHORT_CONTEXT, n_sms=self.n_sms) == 1 else 0
 
     def settle(self, x: torch.Tensor, delta, bias) -> torch.Tensor:
         """Adds an update that was still pending (and its bias) to the residual stream x, and returns x in

@@ -158,6 +158,12 @@ class GQAttention(Mixer):
     def kernel_groups(self):
         return {"head_prep", "attention_plain", "gemm_plain"} | ({"rowwise"} if self.gate_name is not None else set())
 
+    def short_context(self, rt, n_seqs):
+        rot = self.pe.rotation() if self.pe is not None else None
+        if not self.plain_heads or self.kv_shared or (rot is not None and getattr(self.pe, "layout", "halves") == "pairs"):
+            return 0
+        return rt.short_context(n_seqs, self.hd, rot[2] if rot is not None else 0, self.n_q, self.n_kv)
+
     def notes(self, rt):
         import torch
         if rt.dtype != torch.bfloat16:

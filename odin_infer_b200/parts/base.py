@@ -94,6 +94,11 @@ class Part:
         """Kernel libraries this part launches (compiled before the first step)."""
         return set()
 
+    def short_context(self, rt, n_seqs: int) -> int:
+        """Up to how many keys a decode step of n_seqs sequences launches other kernels here than with more (0: the same ones):
+        such steps have graphs of their own."""
+        return 0
+
     def notes(self, rt) -> list[str]:
         """What a user should know at load about how this part will run with its sizes (a size that
         a fast kernel does not take and what runs instead); printed once, never an error."""

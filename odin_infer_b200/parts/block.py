@@ -74,6 +74,9 @@ class PreNormBlock(Block):
     def notes(self, rt):
         return [n for p in self._parts() for n in p.notes(rt)]
 
+    def short_context(self, rt, n_seqs):
+        return max(p.short_context(rt, n_seqs) for p in self._parts())
+
     @property
     def graph_safe(self):
         return all(p.graph_safe for p in self._parts())

@@ -290,6 +290,9 @@ class SideBySide(Mixer):
     def kernel_groups(self):
         return {"rowwise"}.union(*(m.kernel_groups() for m in self._both()))
 
+    def short_context(self, rt, n_seqs):
+        return max(m.short_context(rt, n_seqs) for m in self._both())
+
     def notes(self, rt):
         return [n for m in self._both() for n in m.notes(rt)]
 

@@ -51,3 +51,42 @@ def test_contexts_of_the_32_bit_path_are_one_class():
     lengths = (1, 511, 512, 513, 5000)
     assert len({Runtime("cpu", torch.float32).context_class(n) for n in lengths}) == 1
     assert [Runtime("cpu", torch.bfloat16).context_class(n) for n in lengths] == [context_class_of(n) for n in lengths]
+
+
+def _model(raw):
+    from odin_infer_b200.config import config_from_dict
+    from odin_infer_b200.config.registry import lookup_architecture
+    from odin_infer_b200.engine.model import DecoderModel
+    model = DecoderModel(lookup_architecture(raw.get("architectures", [raw.get("architecture")])[0]).build_spec(config_from_dict(raw)))
+    for pe in model.position_encodings.values():
+        pe.cos = pe.sin = None   # (tables of a loaded model)
+    return model
+
+
+def _qwen3(heads, kv, head_dim):
+    return dict(architectures=["Qwen3ForCausalLM"], hidden_size=256, intermediate_size=256, num_hidden_layers=2, num_attention_heads=heads,
+                num_key_value_heads=kv, head_dim=head_dim, vocab_size=256, rope_theta=1e4, rms_norm_eps=1e-6, tie_word_embeddings=True)
+
+
+def test_graphs_of_short_contexts_only_where_their_kernel_runs(monkeypatch):
+    """A decode step has a graph of its own for short contexts exactly where a layer's attention launches another kernel for them."""
+    import torch
+    from odin_infer_b200.engine.runtime import Runtime
+    from odin_infer_b200.parts.base import Mixer
+    from odin_infer_b200.parts.state_space import SideBySide
+    rt, f32 = Runtime("cpu", torch.bfloat16), Runtime("cpu", torch.float32)
+    for heads, kv, hd in ((16, 8, 128), (8, 8, 64), (4, 2, 64)):
+        assert _model(_qwen3(heads, kv, hd)).short_context(rt, 1) == 128
+        assert _model(_qwen3(heads, kv, hd)).short_context(f32, 1) == 0
+    for heads, kv, hd in ((4, 2, 32), (4, 2, 256), (34, 2, 64)):   # no tensor-core decode attention
+        assert _model(_qwen3(heads, kv, hd)).short_context(rt, 1) == 0
+    side = SideBySide.__new__(SideBySide)   # attention beside another mixer in one layer
+    side.left, side.right = _model(_qwen3(16, 8, 128)).layers[0].mixer, Mixer()
+    assert side.short_context(rt, 1) == 128
+    for n_seqs in (1, 64, 256):
+        assert _model(_qwen3(16, 8, 128)).short_context(rt, n_seqs) == 128   # one key split, whatever the batch
+    monkeypatch.setenv("ODIN_DECODE_SPLITS", "2")
+    assert _model(_qwen3(16, 8, 128)).short_context(rt, 1) == 0
+    monkeypatch.delenv("ODIN_DECODE_SPLITS")
+    monkeypatch.setenv("ODIN_FUSED_ATTENTION", "0")
+    assert _model(_qwen3(16, 8, 128)).short_context(rt, 1) == 0

@@ -156,9 +156,8 @@ __device__ __forceinline__ uint32_t q_off(int row, int col) {  // a [16 x HD] ti
     return (uint32_t)(sub * 2048 + row * 128 + ((chunk ^ (row & 7)) << 4));
 }
 
-// Kernels of short contexts (TOG): up to this many pages, of up to this many query heads, are shared by the four warps (see
+// Kernels of short contexts (TOG): a sequence's only page, of up to this many query heads, is shared by the four warps (see
 // attend_together).
-constexpr int TOGETHER_PAGES = 1;
 constexpr int TOGETHER_HEADS = 8;
 constexpr int TOGETHER_ROW = attn::PAGE_T + 8;   // a head's scores of a page (floats), padded against bank conflicts
 
@@ -175,7 +174,7 @@ struct DecodeTcSmem {
     static_assert(BT_KEEP == 128, "token_by_length uses the page numbers' place and the word behind it");
     static_assert(4 * 16 * OS * 4 <= SLOTS * SLOT, "the merge buffer reuses the page slots");
     static_assert(SLOTS <= 7, "barriers and the flag share 64 bytes");
-    static_assert(SLOTS > TOGETHER_PAGES, "pages that the warps share are all there at once, and their scores in a slot behind them");
+    static_assert(SLOTS > 1, "the scores of a page that the warps share meet in the slot behind it");
     static_assert(2 * HD * 2 <= 4 * 16 * 2 * 4, "the newest key and value wait where the warps' maxima and sums meet later");
 };
 
@@ -262,36 +261,31 @@ __device__ __forceinline__ void attend_page(const uint32_t sK_u, const uint32_t 
     }
 }
 
-// Up to TOGETHER_PAGES pages (n_here, all landed, in the slots 0, 1, ..), at most TOGETHER_HEADS query heads: the four warps
-// share every page instead of taking one each.  A warp computes the scores of sixteen of a page's keys and, when they have
+// A sequence's only page (landed, in slot 0), at most TOGETHER_HEADS query heads, one key split, neither sink nor cap (the
+// fused entry has none): the four warps share the page.  A warp computes the scores of sixteen of its keys and, when they have
 // met in shared memory, the sums over a quarter of the head's columns; the softmax between is every warp's own.  (A page
-// alone in a warp is 128 MMAs in a row, and the merge of the warps two more meetings.)  Every page keeps a maximum, a sum
-// and columns of its own and they are merged in their order, as the warps' are: each number is the same sum in the same
-// order, so the bits are those of pages that a warp has alone.  Writes the result, or this split's partial. 
+// alone in a warp is 128 MMAs in a row, and the merge of the warps two more meetings.)  Each number is the same sum in the
+// same order as there, so the bits are the same.
 template <int HD, int SLOTS, int BAR>
-__device__ __forceinline__ void attend_together(const DecodeTcParams& p, uint8_t* smem, const int n_here, const int key_a, const int t_lo,
-                                             const int t_hi, const int t, const int h0, const int g, float* my_acc, float* my_ml,
-                                             const int tid) {
+__device__ __forceinline__ void attend_together(const DecodeTcParams& p, uint8_t* smem, const int key_p, const int t_lo, const int t_hi,
+                                                const int t, const int h0, const int g, const int tid) {
     using namespace attn;
     using L = DecodeTcSmem<HD, SLOTS>;
     constexpr int KB = HD / 16, NB_W = HD / 32;   // blocks of eight columns of a warp
     const int warp = tid >> 5, lane = tid & 31, row = lane >> 2, col = (lane & 3) * 2;
-    float* s_s = reinterpret_cast<float*>(smem + n_here * L::SLOT);   // the scores meet in a slot without a page
+    float* s_s = reinterpret_cast<float*>(smem + L::SLOT);
     uint32_t qa[KB][4];
     const uint32_t sQ_u = tc::smem_u32(smem + SLOTS * L::SLOT);
 #pragma unroll
     for (int kb = 0; kb < KB; ++kb) ldmatrix_x4(qa[kb], sQ_u + q_off(lane & 15, kb * 16 + (lane >> 4) * 8));
-#pragma unroll
-    for (int i = 0; i < TOGETHER_PAGES; ++i) {
-        if (i >= n_here) break;
-        const int key_p = key_a + i * PAGE_T;   // the page's first key
+    const uint32_t sK_u = tc::smem_u32(smem), sV_u = sK_u + L::TILE;   // key_p: the page's first key
+    {
         float s[2][4];
 #pragma unroll
         for (int nb = 0; nb < 2; ++nb)
 #pragma unroll
             for (int j = 0; j < 4; ++j) s[nb][j] = 0.f;
         if (key_p + warp * 16 < t_hi) {
-            const uint32_t sK_u = tc::smem_u32(smem + i * L::SLOT);
 #pragma unroll
             for (int kb = 0; kb < KB; ++kb) {
                 uint32_t b[4];
@@ -305,100 +299,58 @@ __device__ __forceinline__ void attend_together(const DecodeTcParams& p, uint8_t
 #pragma unroll
             for (int j = 0; j < 2; ++j) {   // (rows 8 and up hold no head)
                 const int tk = key_p + warp * 16 + nb * 8 + col + j;
-                float v = s[nb][j] * p.scale_log2;
-                if (p.cap_log2 > 0.f) v = softcap_log2(v, p.cap_log2);
-                if (tk < t_lo || tk >= t_hi) v = -CUDART_INF_F;
-                s[nb][j] = v;
+                const float v = s[nb][j] * p.scale_log2;
+                s[nb][j] = (tk < t_lo || tk >= t_hi) ? -CUDART_INF_F : v;
             }
-            if (row < g) *reinterpret_cast<float2*>(s_s + (i * g + row) * TOGETHER_ROW + warp * 16 + nb * 8 + col) = make_float2(s[nb][0], s[nb][1]);
+            if (row < g) *reinterpret_cast<float2*>(s_s + row * TOGETHER_ROW + warp * 16 + nb * 8 + col) = make_float2(s[nb][0], s[nb][1]);
         }
     }
     group_sync<BAR>();
-    float o[TOGETHER_PAGES][NB_W][2], m[TOGETHER_PAGES], l[TOGETHER_PAGES];
+    float s[8][2], mx = -CUDART_INF_F, l = 0.f;
 #pragma unroll
-    for (int i = 0; i < TOGETHER_PAGES; ++i) {
-        m[i] = NEG_BIG;
-        l[i] = 0.f;
-#pragma unroll
-        for (int n = 0; n < NB_W; ++n) o[i][n][0] = o[i][n][1] = 0.f;
-        if (i >= n_here) continue;
-        float s[8][2], mx = -CUDART_INF_F;
-#pragma unroll
-        for (int nb = 0; nb < 8; ++nb) {
-            const float2 v = *reinterpret_cast<const float2*>(s_s + (i * g + min(row, g - 1)) * TOGETHER_ROW + nb * 8 + col);
-            s[nb][0] = v.x; s[nb][1] = v.y;
-            mx = fmaxf(mx, fmaxf(v.x, v.y));
-        }
-        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
-        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
-        const float m_use = (mx == -CUDART_INF_F) ? 0.f : mx;
-#pragma unroll
-        for (int nb = 0; nb < 8; ++nb)
-#pragma unroll
-            for (int j = 0; j < 2; ++j) {
-                s[nb][j] = exp2f(s[nb][j] - m_use);
-                l[i] += s[nb][j];
-            }
-        m[i] = fmaxf(mx, NEG_BIG);
-        const int n_ks = min(4, (t_hi - (key_a + i * PAGE_T) + 15) / 16);
-        const uint32_t sV_u = tc::smem_u32(smem + i * L::SLOT + L::TILE);
-        float acc[NB_W][4];
-#pragma unroll
-        for (int n = 0; n < NB_W; ++n)
-#pragma unroll
-            for (int j = 0; j < 4; ++j) acc[n][j] = 0.f;
-#pragma unroll
-        for (int ks = 0; ks < 4; ++ks) {
-            if (ks >= n_ks) break;
-            const uint32_t pf[4] = {pack_bf16(s[2 * ks][0], s[2 * ks][1]), 0u, pack_bf16(s[2 * ks + 1][0], s[2 * ks + 1][1]), 0u};
-#pragma unroll
-            for (int n2 = 0; n2 < NB_W / 2; ++n2) {
-                uint32_t b[4];
-                ldmatrix_x4_trans(b, sV_u + tile_off(ks * 16 + (lane & 7) + (((lane >> 3) & 1) << 3), warp * (HD / 4) + n2 * 16 + (lane >> 4) * 8));
-                mma_bf16(acc[2 * n2], pf, b[0], b[1]);
-                mma_bf16(acc[2 * n2 + 1], pf, b[2], b[3]);
-            }
-        }
-#pragma unroll
-        for (int n = 0; n < NB_W; ++n) { o[i][n][0] = acc[n][0]; o[i][n][1] = acc[n][1]; }
-        l[i] += __shfl_xor_sync(0xffffffffu, l[i], 1);
-        l[i] += __shfl_xor_sync(0xffffffffu, l[i], 2);
+    for (int nb = 0; nb < 8; ++nb) {
+        const float2 v = *reinterpret_cast<const float2*>(s_s + min(row, g - 1) * TOGETHER_ROW + nb * 8 + col);
+        s[nb][0] = v.x; s[nb][1] = v.y;
+        mx = fmaxf(mx, fmaxf(v.x, v.y));
     }
-    odin_trace_mark(3);  // every page is multiplied
-    float mm = NEG_BIG, ll = 0.f, a[NB_W][2];
+    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+    const float m_use = (mx == -CUDART_INF_F) ? 0.f : mx;
 #pragma unroll
-    for (int i = 0; i < TOGETHER_PAGES; ++i) mm = fmaxf(mm, m[i]);
+    for (int nb = 0; nb < 8; ++nb)
 #pragma unroll
-    for (int n = 0; n < NB_W; ++n) a[n][0] = a[n][1] = 0.f;
+        for (int j = 0; j < 2; ++j) {
+            s[nb][j] = exp2f(s[nb][j] - m_use);
+            l += s[nb][j];
+        }
+    const int n_ks = min(4, (t_hi - key_p + 15) / 16);
+    float acc[NB_W][4];
 #pragma unroll
-    for (int i = 0; i < TOGETHER_PAGES; ++i) {
-        const float c = exp2f(m[i] - mm);
+    for (int n = 0; n < NB_W; ++n)
 #pragma unroll
-        for (int n = 0; n < NB_W; ++n) { a[n][0] += o[i][n][0] * c; a[n][1] += o[i][n][1] * c; }
-        ll += l[i] * c;
+        for (int j = 0; j < 4; ++j) acc[n][j] = 0.f;
+#pragma unroll
+    for (int ks = 0; ks < 4; ++ks) {
+        if (ks >= n_ks) break;
+        const uint32_t pf[4] = {pack_bf16(s[2 * ks][0], s[2 * ks][1]), 0u, pack_bf16(s[2 * ks + 1][0], s[2 * ks + 1][1]), 0u};
+#pragma unroll
+        for (int n2 = 0; n2 < NB_W / 2; ++n2) {
+            uint32_t b[4];
+            ldmatrix_x4_trans(b, sV_u + tile_off(ks * 16 + (lane & 7) + (((lane >> 3) & 1) << 3), warp * (HD / 4) + n2 * 16 + (lane >> 4) * 8));
+            mma_bf16(acc[2 * n2], pf, b[0], b[1]);
+            mma_bf16(acc[2 * n2 + 1], pf, b[2], b[3]);
+        }
     }
+    l += __shfl_xor_sync(0xffffffffu, l, 1);
+    l += __shfl_xor_sync(0xffffffffu, l, 2);
+    odin_trace_mark(3);  // the page is multiplied
     if (row >= g) return;
     const int d0 = warp * (HD / 4) + col;
-    if (p.n_split == 1) {
-        float c = 1.f;
-        if (p.sink != nullptr) {   // (as add_sink)
-            const float sk = p.sink[h0 + row] * 1.4426950408889634f, m2 = fmaxf(mm, sk);
-            c = exp2f(mm - m2);
-            ll = ll * c + exp2f(sk - m2);
-        }
-        const float inv = ll > 0.f ? 1.0f / ll : 0.f;
+    const float inv = l > 0.f ? 1.0f / l : 0.f;
 #pragma unroll
-        for (int n = 0; n < NB_W; ++n) {
-            if (p.sink != nullptr) { a[n][0] *= c; a[n][1] *= c; }
-            *reinterpret_cast<uint32_t*>(p.out + (size_t)t * p.out_stride + (size_t)(h0 + row) * HD + d0 + n * 8) =
-                pack_bf16(a[n][0] * inv, a[n][1] * inv);
-        }
-    } else {
-#pragma unroll
-        for (int n = 0; n < NB_W; ++n)
-            *reinterpret_cast<float2*>(my_acc + (size_t)row * p.n_split * HD + d0 + n * 8) = make_float2(a[n][0], a[n][1]);
-        if (warp == 0 && (lane & 3) == 0) { my_ml[(size_t)row * p.n_split * 2] = mm; my_ml[(size_t)row * p.n_split * 2 + 1] = ll; }
-    }
+    for (int n = 0; n < NB_W; ++n)
+        *reinterpret_cast<uint32_t*>(p.out + (size_t)t * p.out_stride + (size_t)(h0 + row) * HD + d0 + n * 8) =
+            pack_bf16(acc[n][0] * inv, acc[n][1] * inv);
 }
 
 // PREP 0: q is given and the cache is complete.  PREP 1 (32-bit parts) and 2 (bfloat16): the
@@ -411,12 +363,14 @@ __device__ __forceinline__ void attend_together(const DecodeTcParams& p, uint8_t
 // bytes, 1024-byte aligned.  (split, kvh, t): which piece of the work.  wait_before(): called by all 128
 // threads together, once, where the body first needs what ran before it (the stand-alone kernel waits for
 // the kernel before it there); tables, weights and the cache's older pages are read ahead of it.
-// TOG: for short contexts in one split: pages that the warps share (attend_together), and heads prepared two at a time.
+// TOG (with PREP, in one split): for short contexts: a sequence's only page is shared by the warps (attend_together), and heads
+// are prepared two at a time, which is all that changes for sequences of more pages.
 template <int HD, int SLOTS, int PREP, bool TOG, int BAR, typename WaitFn>
 __device__ __forceinline__ void attn_decode_tc_body(const CUtensorMap& map_k, const CUtensorMap& map_v,
                                                     const DecodeTcParams& p, uint8_t* smem, const int tid,
                                                     const int split, const int kvh, const int t, WaitFn&& wait_before) {
     using namespace attn;
+    static_assert(!TOG || PREP != 0, "a page is shared where the heads are prepared");
     using TI = typename std::conditional<PREP == 2, bf16, float>::type;
     constexpr int VEC = HD / 32;
     using L = DecodeTcSmem<HD, SLOTS>;
@@ -570,26 +524,21 @@ __device__ __forceinline__ void attn_decode_tc_body(const CUtensorMap& map_k, co
         __syncwarp();
     };
     if constexpr (TOG) {
-        if (n_here <= TOGETHER_PAGES && g <= TOGETHER_HEADS) {
-            bool ok = true;
-            for (int i = 0; i < n_here; ++i) ok = ok && tc::mbar_wait(&full[i], 0, abort_flag);
-            if (has_last && ok) {
-                uint8_t *sK = smem + (p_last - pa) * SLOT, *sV = sK + TILE;
-                if (PREP != 0 && warp == 0) put_newest(sK, sV, s_pages[p_last - pa]);
+        if (n_here == 1 && g <= TOGETHER_HEADS) {   // the newest page, in slot 0
+            if (tc::mbar_wait(&full[0], 0, abort_flag)) {
+                if (warp == 0) put_newest(smem, smem + TILE, s_pages[0]);
                 // value rows past the sequence's end that are multiplied may hold a stale Inf or NaN, and 0 x NaN is NaN
                 const int rrow = pos % PAGE_T, rows = (rrow / 16 + 1) * 16;
                 for (int idx = tid; idx < (rows - (rrow + 1)) * (HD / 8); idx += 128)
-                    *reinterpret_cast<uint4*>(sV + tile_off(rrow + 1 + idx / (HD / 8), (idx % (HD / 8)) * 8)) = make_uint4(0, 0, 0, 0);
+                    *reinterpret_cast<uint4*>(smem + TILE + tile_off(rrow + 1 + idx / (HD / 8), (idx % (HD / 8)) * 8)) = make_uint4(0, 0, 0, 0);
             }
             group_sync<BAR>();
             if (*abort_flag) {
                 if (tid == 0 && p.error != nullptr) atomicExch(p.error, 1);
                 return;
             }
-            attend_together<HD, SLOTS, BAR>(p, smem, n_here, pa * PAGE_T, t_lo, t_hi, t, h0, g, my_acc, my_ml, tid);
+            attend_together<HD, SLOTS, BAR>(p, smem, pa * PAGE_T, t_lo, t_hi, t, h0, g, tid);
             odin_trace_mark(4);
-            if (p.n_split > 1) split_arrive_and_combine<HD, BAR>(p, t, kvh, g, h0, s_last, tid);
-            odin_trace_mark(5);
             return;
         }
     }

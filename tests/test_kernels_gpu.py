@@ -555,6 +555,36 @@ def test_experts_of_few_tokens_have_the_grouped_products_bits(T, E, per, d, ff, 
     ops.moe_tc_check()
 
 
+@pytest.mark.parametrize("T,per,d", [(33, 2, 64), (32, 9, 64), (29, 9, 64), (32, 2, 4096)])
+def test_experts_of_few_tokens_refused(T, per, d):
+    """More than 32 tokens, more than 256 choices, rows too wide for the ring beside 32 of them: nothing is launched, and the runtime
+    gives the grouped products' result."""
+    from odin_infer_b200.csrc import ops
+    from odin_infer_b200.engine import runtime
+    E, ff = 6, 64
+    torch.manual_seed(T + per)
+    h = torch.randn(T, d, device=DEV).bfloat16()
+    w1 = (torch.randn(E, 2 * ff, d, device=DEV) / math.sqrt(d)).bfloat16()
+    w2 = (torch.randn(E, d, ff, device=DEV) / math.sqrt(ff)).bfloat16()
+    ids, wts = torch.randint(-1, E, (T, per), device=DEV, dtype=torch.int32), torch.rand(T, per, device=DEV)
+    a, c = torch.full((T * per, ff), 5.0, device=DEV).bfloat16(), torch.full((T * per, d), 5.0, device=DEV)
+    launched = ops.launch_count()
+    assert not ops.moe_few(h, w1, w2, ids, "silu", a, c)
+    assert ops.launch_count() == launched and (a == 5.0).all() and (c == 5.0).all()
+    got = runtime.Runtime(DEV, torch.bfloat16).experts(h, w1, w2, ids, wts, "silu")
+    assert got.shape == (T, d)
+    ref = torch.zeros(T, d, dtype=torch.float64, device=DEV)
+    for k in range(per):
+        e = ids[:, k].clamp_min(0).long()
+        z = torch.einsum("td,tfd->tf", h.double(), w1.double()[e])
+        act = (torch.nn.functional.silu(z[:, :ff]) * z[:, ff:]).bfloat16().double()
+        ref += torch.where(ids[:, k:k + 1] >= 0, wts[:, k:k + 1].double() * torch.einsum("tf,tdf->td", act, w2.double()[e]), 0.0)
+    # both sides round the activations to bfloat16 (half a unit: 2^-9 of a value), and a sum in another order turns a few of these
+    # roundings the other way: less than 2^-8 of the whole
+    assert (got.double() - ref).norm() <= 4e-3 * ref.norm()
+    ops.moe_tc_check()
+
+
 def test_experts_of_few_tokens_from_two_threads():
     """Two engines' threads on one stream, with 8 and 16 tokens: the same kernels with different shared memory."""
     import threading
@@ -642,15 +672,21 @@ def test_decode_attention_of_short_contexts_has_the_bits_of_any(geom, parts, win
     norm = (1 + 0.1 * torch.randn(hd, device=DEV)).bfloat16()
     ang = torch.randn(700, hd // 2, device=DEV)
     cos, sin = torch.cos(ang).contiguous(), torch.sin(ang).contiguous()
-    for n_split in (1, 3):
+    for n_split in (1, 3):   # (with three splits the kernel of every context runs: head preparation and attention apart are the other side)
         scratch = torch.empty(ops.attention_decode_scratch(T, n_q, hd, n_split), device=DEV)
         got = []
-        for short in (False, True):
+        for form in ("every", "short", "apart"):
             kc, vc, out = k_cache.clone(), v_cache.clone(), torch.full((T, n_q * hd), 7.0, device=DEV, dtype=torch.bfloat16)
-            assert ops.attention_decode_fused(qkv, out, n_q, n_kv, hd, norm, norm, 1e-6, cos, sin, hd, kc, vc, tok_pos, tok_seq, bt,
-                                              window, scratch, n_split, short=short)
+            if form == "apart":
+                q = torch.zeros(T, n_q * hd, device=DEV, dtype=torch.bfloat16)
+                ops.head_prep(qkv, n_q, n_kv, hd, norm, norm, 1e-6, cos, sin, hd, tok_pos, tok_seq, bt, kc, vc, q_out=q)
+                ops.attention_decode(q, out, n_q, n_kv, hd, kc, vc, tok_pos, tok_seq, bt, window, scratch, n_split)
+            else:
+                assert ops.attention_decode_fused(qkv, out, n_q, n_kv, hd, norm, norm, 1e-6, cos, sin, hd, kc, vc, tok_pos, tok_seq, bt,
+                                                  window, scratch, n_split, short=form == "short")
             got.append([out] + [torch.nan_to_num(t.float(), nan=-1.0) for t in (kc, vc)])
-        assert got[0][0].isfinite().all() and all(torch.equal(a, b) for a, b in zip(*got))
+        assert got[0][0].isfinite().all()
+        assert all(torch.equal(a, b) for other in got[1:] for a, b in zip(got[0], other))
     ops.attention_decode_check()
 
 

@@ -182,36 +182,42 @@ mix_streams_fast_kernel(StreamArgs a, TO* __restrict__ out) {
 #pragma unroll
         for (int i = 0; i < NV; ++i) load_streams(i, X[EARLY ? i : 0]);
     }
+    // One group of four a thread (decoding): the first nine parts of one term go out together, or four at a time of two terms:
+    // 64 to 77 registers a thread.  (Six of two terms took up to 119, and a block of 512 threads left no room on its SM for the
+    // next product's.  What is not here: three of two and eight of one in 64 registers, up to 30 % slower at 128 rows of one term.)
+    constexpr int B = NV != 1 ? 1 : NT == 2 ? 4 : 9;
+    float4 early[NT > 0 ? NT : 1][B];
+    const int own = threadIdx.x * 4;
+    auto load_parts = [&](int s0) {
+#pragma unroll
+        for (int n = 0; n < NT; ++n)
+#pragma unroll
+            for (int u = 0; u < B; ++u)
+                if (s0 + u < a.terms.t[n].n_split)
+                    early[n][u] = ld4((const float*)a.terms.t[n].p + (size_t)(s0 + u) * a.terms.t[n].split_stride + (size_t)r * d + own);
+    };
+    auto add_parts = [&](int n, int s0) {
+#pragma unroll
+        for (int u = 0; u < B; ++u)
+            if (s0 + u < a.terms.t[n].n_split) { t[n][0].x += early[n][u].x; t[n][0].y += early[n][u].y; t[n][0].z += early[n][u].z; t[n][0].w += early[n][u].w; }
+    };
+    if (NV == 1 && NT == 1 && own < d) load_parts(0);
 #pragma unroll
     for (int n = 0; n < NT; ++n)
 #pragma unroll
         for (int i = 0; i < NV; ++i) t[n][i] = make_float4(0.f, 0.f, 0.f, 0.f);
-    // One group of four a thread (decoding): the first nine parts of one term go out together, or four at a time of two terms:
-    // 64 to 77 registers a thread.  (Six of two terms took up to 119, and a block of 512 threads left no room on its SM for the
-    // next product's; three of two and eight of one, in 64 registers, were up to 30 % slower at 128 rows of one term.)
-    constexpr int B = NT == 2 ? 4 : 9;
-    const int own = threadIdx.x * 4;
-    if (NT > 0 && NV == 1 && own < d) {
-        int most = a.terms.t[0].n_split;
-        if (NT > 1) most = max(most, a.terms.t[NT - 1].n_split);
-        for (int s0 = 0; s0 < (NT == 2 ? most : 1); s0 += B) {
-            float4 part[NT > 0 ? NT : 1][B];
+    if (NV == 1 && NT == 2 && own < d) {
+        const int most = max(a.terms.t[0].n_split, a.terms.t[NT - 1].n_split);
+        for (int s0 = 0; s0 < most; s0 += B) {
+            load_parts(s0);
 #pragma unroll
-            for (int n = 0; n < NT; ++n)
-#pragma unroll
-                for (int u = 0; u < B; ++u)
-                    if (s0 + u < a.terms.t[n].n_split)
-                        part[n][u] = ld4((const float*)a.terms.t[n].p + (size_t)(s0 + u) * a.terms.t[n].split_stride + (size_t)r * d + own);
-#pragma unroll
-            for (int n = 0; n < NT; ++n)
-#pragma unroll
-                for (int u = 0; u < B; ++u)
-                    if (s0 + u < a.terms.t[n].n_split) { t[n][0].x += part[n][u].x; t[n][0].y += part[n][u].y; t[n][0].z += part[n][u].z; t[n][0].w += part[n][u].w; }
+            for (int n = 0; n < NT; ++n) add_parts(n, s0);
         }
     }
 #pragma unroll
     for (int n = 0; n < NT; ++n) {
         const CombineTerm& tm = a.terms.t[n];
+        if (NV == 1 && NT == 1 && own < d) add_parts(n, 0);
         for (int sp = NV != 1 ? 0 : NT == 1 ? B : tm.n_split; sp < tm.n_split; ++sp) {
 #pragma unroll
             for (int i = 0; i < NV; ++i) {

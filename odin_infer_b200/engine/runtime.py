@@ -67,16 +67,14 @@ LIGHT_STAGES = int(os.environ.get("ODIN_GEMM_LIGHT_STAGES", "5"))
 STAGED_BLOCKS = int(os.environ.get("ODIN_GEMM_STAGED", "15"))
 
 
-def short_context_of(n_q: int, n_kv: int) -> int:
-    """Up to how many keys decode attention's kernel of short contexts is the faster one (with head preparation, one key split).
-
-    Up to 64 a sequence's only page is shared by a block's warps; a step at 20 to 60 keys with it and without, on the 1.7B size
-    (two query heads per kv head): 0.96 and 1.01 ms for one sequence, 1.00 and 1.06 for 8, 1.72 and 1.84 for 64, 2.47 and 2.70 for
-    128; on the 8B size (four): 2.66 and 2.69, 2.81 and 2.85, 4.07 and 4.17, 5.41 and 5.63.  From 65 to 128 a warp takes a page alone
-    and only the heads are prepared two at a time: with two heads per kv head 0.997 and 1.002, 1.026 and 1.059, 1.84 and 1.89, 2.76
-    and 2.99 ms; with four it is the slower one for one to 32 sequences (2.711 and 2.681 for one, 2.896 and 2.877 for 8), so the line
-    lies at a page there.  Beyond, the kernel of every context: in one kernel with this one's code it was 2 to 5 % slower."""
-    return 128 if n_q <= 2 * n_kv else 64
+# Up to this many keys a decode step's attention runs the kernel of short contexts (with head preparation, one key split): a
+# sequence's only page is shared by a block's warps, of two pages a warp takes each, and heads are prepared two at a time.  A
+# step with it and without (ms), on the 1.7B size at 20 to 34 keys: 1 sequence 0.920 and 1.006, 8: 0.971 and 1.048, 64: 1.68 and 1.83,
+# 128: 2.39 and 2.68; at 70 to 84: 0.961 and 0.995, 1.015 and 1.049, 1.81 and 1.88, 2.70 and 2.88; on the 8B size at 20 to 34: 2.667 and
+# 2.703, 2.805 and 2.846, 4.00 and 4.15, 5.35 and 5.41; at 70 to 84: 2.677 and 2.690, 2.852 and 2.873, 4.69 and 4.79, 6.00 and 6.09 (two of
+# twenty pairs, at 32 and 64 sequences, lay 0.3 and 0.7 % the other way).  Beyond, the kernel of every context: in one kernel with
+# this one's code it was 2 to 5 % slower, and this one at 180 to 210 keys 2 %.
+SHORT_CONTEXT = 128
 
 
 def context_class_of(longest: int, page: int = 64) -> int:
@@ -334,8 +332,7 @@ class Runtime:
         """Up to how many keys a step of n_seqs sequences runs decode attention's kernel of short contexts (0: never)."""
         if not self.heads_prepared_in_attention(head_dim, rotary_dim, n_q, n_kv):
             return 0
-        keys = short_context_of(n_q, n_kv)
-        return keys if decode_key_splits(n_seqs, n_kv, keys, n_sms=self.n_sms) == 1 else 0
+        return SHORT_CONTEXT if decode_key_splits(n_seqs, n_kv, SHORT_CONTEXT, n_sms=self.n_sms) == 1 else 0
 
     def settle(self, x: torch.Tensor, delta, bias) -> torch.Tensor:
         """Adds an update that was still pending (and its bias) to the residual stream x, and returns x in

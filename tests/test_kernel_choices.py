@@ -90,13 +90,3 @@ def test_graphs_of_short_contexts_only_where_their_kernel_runs(monkeypatch):
     monkeypatch.delenv("ODIN_DECODE_SPLITS")
     monkeypatch.setenv("ODIN_FUSED_ATTENTION", "0")
     assert _model(_qwen3(16, 8, 128)).short_context(rt, 1) == 0
-
-
-def test_short_contexts_by_the_heads_that_share_a_key_head():
-    """Up to 128 keys with one or two query heads per kv head, up to a page with more (measured on both sides)."""
-    import torch
-    from odin_infer_b200.engine.runtime import Runtime
-    rt = Runtime("cpu", torch.bfloat16)
-    for heads, kv, keys in ((16, 8, 128), (8, 8, 128), (32, 8, 64), (24, 8, 64), (32, 2, 64)):
-        assert rt.short_context(1, 128, 128, heads, kv) == keys
-        assert _model(_qwen3(heads, kv, 128)).short_context(rt, 1) == keys

@@ -157,6 +157,9 @@ __device__ __forceinline__ void pdl_wait() {
 
 #include <cstdlib>
 #include <cstring>
+#include <map>
+#include <mutex>
+#include <utility>
 
 static inline bool odin_pdl_enabled() {
     static int v = -1;
@@ -165,6 +168,24 @@ static inline bool odin_pdl_enabled() {
         v = (e != nullptr && e[0] == '0') ? 0 : 1;
     }
     return v != 0;
+}
+
+// Lets a kernel be launched with `bytes` of dynamic shared memory.  The limit is the function's on the device, for all threads of
+// the process: it only ever grows, so that another thread's smaller launch cannot lower it between this call and the launch
+// behind it.
+template <typename... KArgs>
+static inline cudaError_t odin_allow_smem(void (*kernel)(KArgs...), size_t bytes) {
+    static std::mutex mu;
+    static std::map<std::pair<const void*, int>, size_t> allowed;
+    int device = 0;
+    cudaError_t e = cudaGetDevice(&device);
+    if (e != cudaSuccess) return e;
+    std::lock_guard<std::mutex> guard(mu);
+    size_t& most = allowed[{(const void*)kernel, device}];
+    if (bytes <= most) return cudaSuccess;
+    e = cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    if (e == cudaSuccess) most = bytes;
+    return e;
 }
 
 template <typename... KArgs, typename... Args>

@@ -310,7 +310,7 @@ extern "C" int odin_decay_blocks(const float* q, long long q_stride, const float
     const size_t smem = sizeof(float) * (size_t)(DB_HALF * ld + DB_HALF * (ld > 64 * nj ? ld : 64 * nj) + DB_HALF * DB_P + DB_TOK + 1);
     auto kern = nj == 2 ? decay_out_kernel<2> : decay_out_kernel<1>;
     if (smem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaError_t e = odin_allow_smem(kern, smem);
         if (e != cudaSuccess) return (int)e;
     }
     odin_launch(kern, dim3(items * 2, H, (dv + 64 * nj - 1) / (64 * nj)), dim3(256), smem, s, p);

@@ -675,7 +675,7 @@ template <typename... A>
 static int set_smem(void (*kern)(A...), size_t bytes) {
     if (bytes > 227 * 1024) return ODIN_ERR_UNSUPPORTED;
     if (bytes <= 48 * 1024) return 0;
-    return (int)cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    return (int)odin_allow_smem(kern, bytes);
 }
 
 // Floats of scratch that the chunked form needs for a step of T rows.

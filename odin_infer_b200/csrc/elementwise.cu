@@ -433,7 +433,7 @@ static int launch_add_rmsnorm(float* x, const void* delta, int n_split, size_t s
         const int threads = d >= 2048 ? 512 : (d >= 1024 ? 256 : 128);
         auto kern = add_rmsnorm_kernel<TD, TO, true, 512>;
         if (smem > 48 * 1024) {
-            cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            cudaError_t e = odin_allow_smem(kern, smem);
             if (e != cudaSuccess) return (int)e;
         }
         odin_launch(kern, dim3(n_rows), dim3(threads), smem, s, x, (const TD*)delta, n_split, split_stride, w, eps,
@@ -441,8 +441,7 @@ static int launch_add_rmsnorm(float* x, const void* delta, int n_split, size_t s
     } else {
         const int threads = d >= 2048 ? 512 : (d >= 512 ? 256 : 128);
         if (smem > 48 * 1024) {
-            cudaError_t e = cudaFuncSetAttribute(add_rmsnorm_kernel<TD, TO, false>,
-                                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            cudaError_t e = odin_allow_smem(add_rmsnorm_kernel<TD, TO, false>, smem);
             if (e != cudaSuccess) return (int)e;
         }
         odin_launch(add_rmsnorm_kernel<TD, TO, false>, dim3(n_rows), dim3(threads), smem, s, x, (const TD*)delta, n_split,

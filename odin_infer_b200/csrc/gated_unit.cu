@@ -140,7 +140,7 @@ extern "C" int odin_gated_unit_step(const void* u, int dtype, const void* w, int
 #define GO(T, TW)                                                                                                    \
     do {                                                                                                             \
         if (smem > 20 * 1024) {                                                                                      \
-            cudaError_t e = cudaFuncSetAttribute(gated_unit_step_kernel<T, TW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
+            cudaError_t e = odin_allow_smem(gated_unit_step_kernel<T, TW>, smem); \
             if (e != cudaSuccess) return (int)e;                                                                     \
         }                                                                                                            \
         odin_launch(gated_unit_step_kernel<T, TW>, grid, dim3(GU_STEP_THREADS), smem, s, (const T*)u, (const TW*)w, bias, log_decay, \

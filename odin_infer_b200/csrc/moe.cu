@@ -272,7 +272,7 @@ extern "C" int odin_moe_router(const void* h, int h_dtype, long long h_stride, c
 #define GO(TH, TW)                                                                                                   \
     do {                                                                                                             \
         if (smem > 48 * 1024)                                                                                        \
-            cudaFuncSetAttribute(moe_router_kernel<TH, TW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
+            odin_allow_smem(moe_router_kernel<TH, TW>, smem); \
         odin_launch(moe_router_kernel<TH, TW>, dim3(T), dim3(threads), smem, s, (const TH*)h, (size_t)h_stride,      \
                     (const TW*)w, bv, E, d, top, always, tok_seq, ids, wts, logits, score, groups, keep,             \
                     route_scale, gate_row, gate_out, n_real, pass_out);                                              \
@@ -327,7 +327,7 @@ extern "C" int odin_moe_gate_up(const void* h, int h_dtype, long long h_stride, 
 #define GO(TH, TW)                                                                                                    \
     do {                                                                                                              \
         if (smem > 48 * 1024)                                                                                         \
-            cudaFuncSetAttribute(moe_gate_up_kernel<TH, TW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
+            odin_allow_smem(moe_gate_up_kernel<TH, TW>, smem); \
         odin_launch(moe_gate_up_kernel<TH, TW>, grid, dim3(MOE_THREADS), smem, s, (const TH*)h, (size_t)h_stride,     \
                     (const TW*)w, ids, in_wts, per, ff, d, act, gated, (TH*)out);                                     \
     } while (0)
@@ -379,7 +379,7 @@ extern "C" int odin_moe_down(const void* a, int a_dtype, const void* w, int w_dt
 #define GO(TA, TW)                                                                                                 \
     do {                                                                                                           \
         if (smem > 48 * 1024)                                                                                      \
-            cudaFuncSetAttribute(moe_down_kernel<TA, TW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
+            odin_allow_smem(moe_down_kernel<TA, TW>, smem); \
         odin_launch(moe_down_kernel<TA, TW>, grid, dim3(MOE_THREADS), smem, s, (const TA*)a, (const TW*)w, ids,    \
                     wts, T, per, ff, d, y);                                                                        \
     } while (0)

@@ -346,14 +346,8 @@ constexpr int few_smem(int stages, int K, int x_rows) { return 1024 /* alignment
 template <int MODE, int TN>
 int launch_few(const CUtensorMap& mw, FewParams p, int smem, cudaStream_t s) {
     auto k = moe_few_kernel<MODE, TN>;
-    // Once, to the most that it can ask for: the limit is the function's, and with each call's own size another thread's smaller
-    // one came between a call's limit and its launch, which then failed.
-    static const cudaError_t configured = [k] {
-        cudaFuncAttributes a;
-        const cudaError_t e = cudaFuncGetAttributes(&a, k);
-        return e != cudaSuccess ? e : cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, MOST_SMEM - (int)a.sharedSizeBytes);
-    }();
-    if (configured != cudaSuccess) return (int)configured;
+    const cudaError_t e = odin_allow_smem(k, (size_t)smem);
+    if (e != cudaSuccess) return (int)e;
     odin_launch(k, dim3(sm_count()), dim3(FEW_THREADS), (size_t)smem, s, mw, p);
     ODIN_LAUNCH_CHECK();
     return 0;

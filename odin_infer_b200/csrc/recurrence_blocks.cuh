@@ -120,7 +120,7 @@ recurrence_carry_out_kernel(RecParams p) {
 static inline int launch_recurrence_carry_out(const RecParams& p, int n_items, cudaStream_t s) {
     const size_t co_smem = (size_t)p.dk * 32 * sizeof(float) + ((p.dk & 3) == 0 ? (size_t)CARRY_OUT_TOK * p.dk * sizeof(float) : 0);
     if (co_smem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(recurrence_carry_out_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)co_smem);
+        cudaError_t e = odin_allow_smem(recurrence_carry_out_kernel, co_smem);
         if (e != cudaSuccess) return (int)e;
     }
     odin_launch(recurrence_carry_out_kernel, dim3(n_items, p.H, (p.dv + 31) / 32), dim3(256), co_smem, s, p);

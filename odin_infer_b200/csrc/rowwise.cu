@@ -176,7 +176,7 @@ static int row_update_launch(float* x, const void* delta, int delta_dtype, int n
     do {                                                                                                         \
         auto kern = vec ? row_update_kernel<TD, TO, true> : row_update_kernel<TD, TO, false>;                    \
         if (smem > 48 * 1024) {                                                                                  \
-            cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);  \
+            cudaError_t e = odin_allow_smem(kern, smem);  \
             if (e != cudaSuccess) return (int)e;                                                                 \
         }                                                                                                        \
         odin_launch(kern, dim3(n_rows), dim3(ROW_THREADS), smem, s, x, (const TD*)delta, n_split,                 \
@@ -274,7 +274,7 @@ extern "C" int odin_normed_add(float* x, const void* y, int y_dtype, int n_split
     do {                                                                                                         \
         auto kern = vec ? normed_add_kernel<TY, true> : normed_add_kernel<TY, false>;                                                                     \
         if (smem > 48 * 1024) {                                                                                  \
-            cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);  \
+            cudaError_t e = odin_allow_smem(kern, smem);  \
             if (e != cudaSuccess) return (int)e;                                                                 \
         }                                                                                                        \
         odin_launch(kern, dim3(n_rows), dim3(ROW_THREADS), smem, s, x, (const TY*)y, n_split, (size_t)split_stride, \
@@ -848,7 +848,7 @@ extern "C" int odin_combine_add(float* x, int n_terms, const void* const* ptrs, 
     do {                                                                                                             \
         auto kern = vec ? combine_add_kernel<TO, true> : combine_add_kernel<TO, false>;                              \
         if (smem > 48 * 1024) {                                                                                      \
-            cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);       \
+            cudaError_t e = odin_allow_smem(kern, smem);       \
             if (e != cudaSuccess) return (int)e;                                                                     \
         }                                                                                                            \
         odin_launch(kern, dim3(n_rows), dim3(ROW_THREADS), smem, s, x, a, post, next, (TO*)out, rows, tok_seq, d);  \

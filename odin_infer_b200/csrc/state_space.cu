@@ -548,7 +548,7 @@ extern "C" int odin_skip_gate_norm(const float* o, const float* x, long long x_s
 #define GO(TZ, TO)                                                                                                      \
     do {                                                                                                                \
         if (smem > 48 * 1024) {                                                                                         \
-            cudaError_t e = cudaFuncSetAttribute(skip_gate_norm_kernel<TZ, TO>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
+            cudaError_t e = odin_allow_smem(skip_gate_norm_kernel<TZ, TO>, smem); \
             if (e != cudaSuccess) return (int)e;                                                                        \
         }                                                                                                               \
         odin_launch(skip_gate_norm_kernel<TZ, TO>, dim3(T, groups), dim3(threads), smem, s, o, x, (size_t)x_stride, Dv, P, (const TZ*)z, \

@@ -357,7 +357,7 @@ extern "C" int odin_mix_streams(float* x, long long stream_stride, int s, int ha
     do {                                                                                                             \
         auto kern = vec ? mix_streams_kernel<TO, true> : mix_streams_kernel<TO, false>;                              \
         if (smem > 48 * 1024) {                                                                                      \
-            cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);       \
+            cudaError_t e = odin_allow_smem(kern, smem);       \
             if (e != cudaSuccess) return (int)e;                                                                     \
         }                                                                                                            \
         odin_launch(kern, dim3(n_rows), dim3(STREAM_THREADS), smem, st, a, (TO*)out);                                \

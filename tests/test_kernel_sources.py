@@ -75,3 +75,15 @@ def test_no_wait_for_either_phase(source):
         text = _without_comments(f.read())
     for bar in re.findall(r"try_wait\(([^;]*?), [01]\) \|\|", text):
         assert f"try_wait({bar}, 0) || tc::mbar_try_wait({bar}, 1)" not in text, (source, bar)
+
+
+@pytest.mark.parametrize("source", SOURCES)
+def test_shared_memory_limits_only_grow(source):
+    """A kernel's limit belongs to all threads: with sizes of single calls it is set where it cannot be lowered (odin_allow_smem)."""
+    with open(os.path.join(CSRC, source)) as f:
+        text = _without_comments(f.read())
+    if source == "common.cuh":
+        text = text.replace(_block(text, text.index("{", text.index("odin_allow_smem"))), "")
+    for size in re.findall(r"cudaFuncAttributeMaxDynamicSharedMemorySize,\s*([^;]*)\)", text):
+        assert not re.search(r"\(int\)\s*(smem|bytes|co_smem)\b", size), (source, size)
+

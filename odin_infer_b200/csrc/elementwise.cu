@@ -253,13 +253,13 @@ add_rmsnorm_kernel(float* __restrict__ x, const TD* delta, int n_split, size_t s
 
 // The variant for a few wide rows (decoding): NV groups of four per thread, kept in registers (no staging in shared
 // memory), the loads of PARTS parts of a group issued together; the same order of additions as the kernel above with as
-// many threads, so the same bits.  1,024 threads from 4,096 columns on, 512 below: there a product's update comes in eight
-// or nine parts, and with two of them in flight a row's loads were five trips to L2 (a request of one 37-token question and
-// 24 tokens on the 1.7B size 28.06 ms, with nine in flight 26.34; back to back 8 rows of nine parts 2.64 and 2.07 us, 128 rows
-// 4.02 and 2.97, of 4,092 columns 6.66 and 5.07).  Its registers are capped so that a block leaves more than a third of an SM's
-// registers free: the product that follows starts its CTAs while this kernel runs, to fetch weights, and on the
-// SMs that hold a row it could not (with 64 registers a thread the block took them all; those CTAs then started 4
-// to 7 us after the others and the whole product ended that much later).
+// many threads, so the same bits.  1,024 threads from 4,096 columns on, 512 below.  A row of 2,048 columns is one group a thread:
+// there nine parts are in flight, as many as a product's update comes in; with two a row's loads were five trips to L2 (a request
+// of one 37-token question and 24 tokens on the 1.7B size 28.06 ms, with nine 26.34; back to back 8 rows of nine parts 2.9 and
+// 2.45 us, 128 rows 3.8 and 3.1).  Wider rows are two groups of four parts each (2,560 columns, 8 rows of nine parts 4.4 and 3.7 us).
+// Its registers are capped so that a block leaves more than a third of an SM's registers free: the product that follows starts
+// its CTAs while this kernel runs, to fetch weights, and on the SMs that hold a row it could not (with 64 registers a thread a
+// block of 1,024 took them all; those CTAs then started 4 to 7 us after the others and the whole product ended that much later).
 template <typename TD, typename TO, int NV, int THREADS, int PARTS>
 __global__ void __maxnreg__(THREADS == 512 ? 64 : NV == 1 ? 40 : 48)
 add_rmsnorm_wide_kernel(float* __restrict__ x, const TD* delta, int n_split, size_t split_stride, VecRef w,

@@ -199,7 +199,8 @@ struct GCfg {
 // A tile of 128 places of an expert with a handful of rows is nearly all padding.  Up to FEW rows their box alone is copied
 // (2 KB instead of 16 a stage beside 32 KB of weights) and the other rows of the stage hold whatever was there: a row of the
 // product depends on its own row of A alone, and nobody reads what belongs to padding.  24 steps of 8 sequences with 7 layers
-// of 32 experts, 4 a token: 29.2 -> 26.5 ms a request.
+// of 32 experts, 4 a token: 29.2 -> 26.5 ms a request, measured before up to 32 tokens had kernels of their own (moe_few_tc.cu);
+// what reaches this now are more tokens, or rows and choices that those refuse.
 constexpr int FEW = 16;
 
 // PER_ELEMENT: a product per head whose outputs have a gate each (the plain form)

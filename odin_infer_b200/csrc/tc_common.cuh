@@ -77,7 +77,9 @@ __device__ __forceinline__ bool elect_one() {
 // tries.  How long one try_wait suspends is up to the hardware (about 4 us on an idle SM, far
 // less on a busy one), so a limit on the number of tries alone would mean anything between a
 // fraction of a second and a quarter of a minute; legitimate waits of these kernels are
-// microseconds (no role spins across a kernel boundary: each calls pdl_wait() first).
+// microseconds: what comes from the kernel before is waited for by pdl_wait() (in the second product of few
+// tokens' experts by the warps that bring the rows; the loads and the MMA wait behind them for as long as the
+// first product runs, tens of microseconds).
 #define TC_WAIT_SECONDS 4ull
 
 __device__ __forceinline__ unsigned long long global_ns() {

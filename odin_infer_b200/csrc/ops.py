@@ -49,15 +49,19 @@ def _stream() -> c_void_p:
 
 
 _streams: dict = {}
+MOST_STREAMS = 256
 
 
 def current_stream() -> torch.cuda.Stream:
-    """`torch.cuda.current_stream()` from a table of the streams seen so far (a handful: torch's streams are a fixed pool)."""
+    """`torch.cuda.current_stream()` from a table of the streams seen so far (a handful: torch's streams are a fixed pool; a
+    program's own can be any number, so the table starts anew at MOST_STREAMS)."""
     if _current_raw_stream is None:
         return torch.cuda.current_stream()
     key = torch._C._cuda_getCurrentStream(torch.cuda.current_device())
     s = _streams.get(key)
     if s is None:
+        if len(_streams) >= MOST_STREAMS:
+            _streams.clear()
         s = _streams[key] = torch.cuda.current_stream()
     return s
 

@@ -90,3 +90,18 @@ def test_graphs_of_short_contexts_only_where_their_kernel_runs(monkeypatch):
     monkeypatch.delenv("ODIN_DECODE_SPLITS")
     monkeypatch.setenv("ODIN_FUSED_ATTENTION", "0")
     assert _model(_qwen3(16, 8, 128)).short_context(rt, 1) == 0
+
+
+def test_the_table_of_streams_is_bounded(monkeypatch):
+    """A program that makes streams without end gets the right one each time, and the table does not grow with them."""
+    import torch
+    from odin_infer_b200.csrc import ops
+    now = [0]
+    monkeypatch.setattr(ops, "_streams", {})
+    monkeypatch.setattr(ops, "_current_raw_stream", lambda device: now[0])
+    monkeypatch.setattr(torch.cuda, "current_device", lambda: 0)
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda: ("stream", now[0]))
+    monkeypatch.setattr(torch._C, "_cuda_getCurrentStream", lambda device: (now[0], device, 1), raising=False)
+    for now[0] in [*range(1000), *range(1000)]:
+        assert ops.current_stream() == ("stream", now[0])
+        assert len(ops._streams) <= 256
